@@ -2,308 +2,310 @@
 // averaged in z, subgrid.f90:261-414 sgs_dynamic_Smagorinsky) and LES = 3
 // (pointwise coefficient, subgrid.f90:420-583 _noaverage).
 //
-// The model runs in FP64 in both precisions, on dense (nxg,nyg,nzg) work
-// arrays indexed 1-based like the source's module arrays (i fastest); the
-// velocity-shaped ones use the U (nx,nyg), V (nxg,ny), W (nxg,nyg) plane
-// shapes.  Every step of the source is one kernel (one thread per point) in
-// the source's order, with the source's evaluation order in each expression (the file is
-// compiled with -fmad=false):
-//   interpolate_x/y/z (interpolation.f90:24-114) to cell centres;
-//   the x helpers apply_Neumann_bc_x / apply_periodic_bc_x
-//   (boundary_conditions.f90:295-344) and apply_periodic_bc_z (:732-760) on
-//   one process, where update_ghost_interior_planes is empty;
-//   filter_xzy (subgrid.f90:140-184, fil_size = 2);
-//   compute_Sij (subgrid.f90:672-730), with the in-place corner averages
-//   taken from a separate array of edge values (the source's loop order
-//   reads only not-yet-averaged neighbours, so the values are the same);
-//   the Lij, Mij contractions, the z average (LES = 2), clipping and
-//   Neumann y (Dirichlet_nu_t = 0).
-// The result goes to nu_t in the box layout as T.  Every index a kernel
-// touches lies in 1..nxg x 1..nyg x 1..nzg of its array's own shape.
+// The model runs in FP64 in both precisions.  The source makes some sixty
+// whole-array passes (interpolations, 24 filters, 34 ghost fills, two rates of
+// strain, contractions); here they are four kernels and, for LES = 2, a fifth:
+//   k_dyn_strain   |S| and |S| Sij of U, V, W;
+//   k_dyn_filter   filtered face velocities hat(U), hat(V), hat(W);
+//   k_dyn_strain   4 |hat(S)| hat(Sij) of those;
+//   k_dyn_contract the 15 filters of Lij and Mij (hat(ui uj), hat(ui),
+//                  hat(|S| Sij)), the contractions Mij Lij and Mij Mij and, for
+//                  LES = 3, nu_t with its clipping and ghosts;
+//   k_dyn_zavg     LES = 2: the z averages, nu_t, clipping and ghosts.
+// Ghost entries (apply_Neumann_bc_x / apply_periodic_bc_x,
+// boundary_conditions.f90:295-344; apply_periodic_bc_z, :732-760; one process)
+// are never stored: a reader takes the interior entry that the source's copies
+// would have left there, by index (XMap, zmap).
+// The filter of filter_xzy (subgrid.f90:140-184, fil_size = 2) is the product
+// of (1,4,1)/6 along x, y and z (one-sided 2/3, 1/3 at the first and last row
+// of its y section), applied as three sums.
+//
+// Work arrays are dense (nxg,nyg) planes, i fastest, Fortran indices.
 #include "kernels.cuh"
+#include "strain.cuh"
 
 namespace blgpu {
 namespace {
 
-enum { W_U, W_V, W_W, W_T0, W_T1, W_T2, W_S, W_UF, W_VF, W_WF, W_TB, W_L, W_G = W_L + 6, W_M = W_G + 6,
-       W_COUNT = W_M + 6 };
+// |S|; |S| Sij; 4 |hat S| hat Sij; hat(U), hat(V), hat(W) and, once those are
+// used, Mij Lij and Mij Mij of LES = 2 in the first two of them
+enum { W_S, W_SS, W_M = W_SS + 6, W_F = W_M + 6, W_COUNT = W_F + 3 };
 
 struct P6 {
   double *p[6];
 };
-
-// index range i0..i0+ni-1, j0.., k0..: one thread per point, i along
-// blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z
-// (nj, nk <= 65535, checked at blgpu_create)
-struct Rng {
-  int i0, ni, j0, nj, k0, nk;
+struct P3 {
+  double *p[3];
 };
 
-__device__ __forceinline__ long long dix(int i, int j, int k, int d1, int d2) {
-  return ((long long)(k - 1) * d2 + (j - 1)) * (long long)d1 + (i - 1);
+__device__ __forceinline__ long long dix(int i, int j, int k, const Geo &g) {
+  return ((long long)(k - 1) * g.nyg + (j - 1)) * (long long)g.nxg + (i - 1);
 }
 
-#define FOR_RNG(R)                                                                                 \
-  if (const int i = (R).i0 + (int)(blockIdx.x * blockDim.x + threadIdx.x), j = (R).j0 + (int)blockIdx.y, \
-      k = (R).k0 + (int)blockIdx.z;                                                                      \
-      i < (R).i0 + (R).ni)
+// the column whose entry the source's x ghost fill leaves at column i of an
+// array of n1 columns: Neumann, periodic for a face array (n1 = nx, id 1) or
+// periodic for a centre array (n1 = nxg, id 2)
+__device__ __forceinline__ int xmap(int i, int n1, int periodic, bool face) {
+  if (!periodic) return i <= 1 ? 2 : i >= n1 ? n1 - 1 : i;
+  if (face) return i <= 1 ? n1 - 1 : i >= n1 ? 2 : i;
+  return i <= 1 ? n1 - 2 : i >= n1 ? 3 : i == n1 - 1 ? 2 : i;
+}
+// the plane left at plane k by apply_periodic_bc_z: centre arrays (n3 = nzg
+// planes, two copies above) and W faces (n3 = nz)
+__device__ __forceinline__ int zmap(int k, int nzg) { return k <= 1 ? nzg - 2 : k == nzg - 1 ? 2 : k >= nzg ? 3 : k; }
+__device__ __forceinline__ int zmap_w(int k, int nz) { return k <= 1 ? nz - 1 : k >= nz ? 2 : k; }
+
+// velocities of the box around (i,j), as FP64
+template <typename T> struct LdBox {
+  const T *U, *V, *W;
+  long long c, px, pl;  // c: box index of (i-1, j, k = 0)
+  __device__ LdBox(const Geo &g, const T *u, const T *v, const T *w, int i, int j, int)
+      : U(u), V(v), W(w), c(bidx(g, i - 1, j, 0)), px(g.px), pl(g.plane) {}
+  __device__ __forceinline__ double at(const T *a, int s, int dj, int k) const {
+    return (double)__ldg(a + c + s + dj * px + k * pl);
+  }
+  __device__ __forceinline__ double u(int s, int dj, int k) const { return at(U, s, dj, k); }
+  __device__ __forceinline__ double v(int s, int dj, int k) const { return at(V, s, dj, k); }
+  __device__ __forceinline__ double w(int s, int dj, int k) const { return at(W, s, dj, k); }
+};
+
+// the filtered velocities around (i,j), ghosts by index
+struct LdHat {
+  const double *U, *V, *W;
+  int xu[2], xc[3], j, nxg, nz, nzg;
+  long long pl;
+  __device__ LdHat(const Geo &g, const double *u, const double *v, const double *w, int i, int j_, int periodic)
+      : U(u), V(v), W(w), j(j_), nxg(g.nxg), nz(g.nz), nzg(g.nzg), pl((long long)g.nxg * g.nyg) {
+    for (int s = 0; s < 2; ++s) xu[s] = xmap(i - 1 + s, g.nx, periodic, true) - 1;
+    for (int s = 0; s < 3; ++s) xc[s] = xmap(i - 1 + s, g.nxg, periodic, false) - 1;
+  }
+  __device__ __forceinline__ double u(int s, int dj, int k) const {
+    return __ldg(U + (zmap(k, nzg) - 1) * pl + (j + dj - 1) * nxg + xu[s]);
+  }
+  __device__ __forceinline__ double v(int s, int dj, int k) const {
+    return __ldg(V + (zmap(k, nzg) - 1) * pl + (j + dj - 1) * nxg + xc[s]);
+  }
+  __device__ __forceinline__ double w(int s, int dj, int k) const {
+    return __ldg(W + (zmap_w(k, nz) - 1) * pl + (j + dj - 1) * nxg + xc[s]);
+  }
+};
+
+// scale |S| Sij of every cell (i = 2..nxg-1, j = 2..nyg-1, k = 2..nzg-1) and,
+// unless null, |S|
+template <typename T, typename LD>
+__global__ void __launch_bounds__(128) k_dyn_strain(Geo g, const T *__restrict__ U, const T *__restrict__ V,
+                                                    const T *__restrict__ W, int periodic, double scale, P6 out,
+                                                    double *__restrict__ S, int kchunk) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2, j = blockIdx.y * blockDim.y + threadIdx.y + 2;
+  if (i > g.nxg - 1 || j > g.nyg - 1) return;
+  const int k0 = 2 + blockIdx.z * kchunk, k1 = min(k0 + kchunk - 1, g.nzg - 1);
+  const LD ld(g, U, V, W, i, j, periodic);
+  StrainColumn<double, LD> col(ld, g.ax.F, g.ax.rF, g.ax.C, g.ax.rC, g.ay.F, g.ay.rF, g.ay.C, g.ay.rC, g.az.F, g.az.rF,
+                               g.az.C, g.az.rC, i, j);
+  col.start(k0);
+  for (int k = k0; k <= k1; ++k) {
+    double s[6];
+    const double n = col.cell(k, s);
+    const long long c = dix(i, j, k, g);
+    const double f = scale * n;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) out.p[m][c] = f * s[m];
+    if (S) S[c] = n;
+  }
+}
+
+constexpr double F1 = 1.0 / 6.0, F2 = 2.0 / 3.0;
+
+// y weights of row j of the section ja..jb, and the rows they belong to
+struct YW {
+  double a, b, c;
+  int jm, jp;
+  __device__ YW(int j, int ja, int jb)
+      : a(j == ja ? 0.0 : j == jb ? 1.0 / 3.0 : F1), b(F2), c(j == ja ? 1.0 / 3.0 : j == jb ? 0.0 : F1),
+        jm(j == ja ? j : j - 1), jp(j == jb ? j : j + 1) {}
+  __device__ __forceinline__ double operator()(double m, double o, double p) const {
+    return __fma_rn(c, p, __fma_rn(a, m, b * o));
+  }
+};
+__device__ __forceinline__ double f141(double m, double o, double p) { return __fma_rn(F1, m + p, F2 * o); }
+
+// hat(U), hat(V), hat(W) on the interior of their own x and z ranges and all
+// rows; blockIdx.z = 3 chunk + component
+template <typename T>
+__global__ void __launch_bounds__(256) k_dyn_filter(Geo g, const T *__restrict__ U, const T *__restrict__ V,
+                                                    const T *__restrict__ W, P3 out, int kchunk) {
+  const int q = blockIdx.z % 3;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2, j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const int n1 = q == 0 ? g.nx : g.nxg, n2 = q == 1 ? g.ny : g.nyg, n3 = q == 2 ? g.nz : g.nzg;
+  const int k0 = 2 + (blockIdx.z / 3) * kchunk, k1 = min(k0 + kchunk - 1, n3 - 1);
+  if (i > n1 - 1 || j > n2 || k0 > k1) return;
+  const T *__restrict__ a = q == 0 ? U : q == 1 ? V : W;
+  const YW y(j, 1, n2);
+  const long long om = bidx(g, i, y.jm, 0), oo = bidx(g, i, j, 0), op = bidx(g, i, y.jp, 0);
+  auto plane = [&](int k) {  // the x and y sums of plane k
+    const T *p = a + k * g.plane;
+    double v[3];
+#pragma unroll
+    for (int s = 0; s < 3; ++s)
+      v[s] = y((double)__ldg(p + om + s - 1), (double)__ldg(p + oo + s - 1), (double)__ldg(p + op + s - 1));
+    return f141(v[0], v[1], v[2]);
+  };
+  double lo = plane(k0 - 1), mid = plane(k0);
+  double *__restrict__ o = q == 0 ? out.p[0] : q == 1 ? out.p[1] : out.p[2];
+  for (int k = k0; k <= k1; ++k) {
+    const double hi = plane(k + 1);
+    o[dix(i, j, k, g)] = f141(lo, mid, hi);
+    lo = mid;
+    mid = hi;
+  }
+}
+
+// nu_t(i,j,k) into the box: clipped, its Neumann rows (j = 1, nyg), and for
+// LES = 3 the periodic x and z ghosts that take their value from it; an entry
+// that the source's ghost copies overwrite is not written
+template <typename T>
+__device__ __forceinline__ void put_rows(const Geo &g, T *__restrict__ nut, int i, int j, int k, double v) {
+  const T t = (T)(v > 0.0 ? v : 0.0);
+  nut[bidx(g, i, j, k)] = t;
+  if (j == 2) nut[bidx(g, i, 1, k)] = t;
+  if (j == g.nyg - 1) nut[bidx(g, i, g.nyg, k)] = t;
+}
+template <typename T>
+__device__ __forceinline__ void put_periodic(const Geo &g, T *__restrict__ nut, int i, int j, int k, double v) {
+  const int gi = i == g.nxg - 2 ? 1 : i == 2 ? g.nxg - 1 : i == 3 ? g.nxg : 0;
+  const int gk = k == g.nzg - 2 ? 1 : k == 2 ? g.nzg - 1 : k == 3 ? g.nzg : 0;
+  if (i == g.nxg - 1 || k == g.nzg - 1) return;
+  put_rows(g, nut, i, j, k, v);
+  if (gi) put_rows(g, nut, gi, j, k, v);
+  if (gk) put_rows(g, nut, i, j, gk, v);
+  if (gi && gk) put_rows(g, nut, gi, j, gk, v);
+}
+
+// Lij, Mij and their contractions.  A warp owns 32 columns of one row j and
+// gives its 30 inner ones; it walks up k.  Per plane a lane forms the y sums
+// of the 15 filtered quantities at its own column (the centre velocities are
+// averaged from the box there), the x sums take the two neighbours' by
+// shuffles, and the z sums two planes carried in registers.  LES = 3 stores
+// nu_t, LES = 2 Mij Lij and Mij Mij.
+constexpr int DC_ROWS = 4;
 
 template <typename T>
-__global__ void k_gather(Geo g, Rng R, const T *__restrict__ U, const T *__restrict__ V, const T *__restrict__ W,
-                         double *__restrict__ Ud, double *__restrict__ Vd, double *__restrict__ Wd) {
-  FOR_RNG(R) {
-    const long long b = bidx(g, i, j, k);
-    if (i <= g.nx) Ud[dix(i, j, k, g.nx, g.nyg)] = (double)U[b];
-    if (j <= g.ny) Vd[dix(i, j, k, g.nxg, g.ny)] = (double)V[b];
-    if (k <= g.nz) Wd[dix(i, j, k, g.nxg, g.nyg)] = (double)W[b];
-  }
-}
-
-// faces to centres: term(2:nx), term_1(:,2:ny), term_2(:,:,2:nz), term_2(nzg) = 0
-__global__ void k_interp(Geo g, Rng R, const double *__restrict__ Ud, const double *__restrict__ Vd,
-                         const double *__restrict__ Wd, double *__restrict__ t0, double *__restrict__ t1,
-                         double *__restrict__ t2) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    if (i >= 2 && i <= g.nx) t0[c] = 0.5 * (Ud[dix(i - 1, j, k, g.nx, g.nyg)] + Ud[dix(i, j, k, g.nx, g.nyg)]);
-    if (j >= 2 && j <= g.ny) t1[c] = 0.5 * (Vd[dix(i, j - 1, k, g.nxg, g.ny)] + Vd[dix(i, j, k, g.nxg, g.ny)]);
-    if (k >= 2 && k <= g.nz) t2[c] = 0.5 * (Wd[dix(i, j, k - 1, g.nxg, g.nyg)] + Wd[dix(i, j, k, g.nxg, g.nyg)]);
-    if (k == g.nzg) t2[c] = 0.0;
-  }
-}
-
-// x ghosts of every row (j,k) of a dense array with first dimension d1
-__global__ void k_bc_x(long long rows, double *__restrict__ a, int d1, int id, int periodic, int nx, int nxg) {
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < rows; q += (long long)gridDim.x * blockDim.x) {
-    double *r = a + q * d1;
-    if (!periodic) {
-      if (id == 1) { r[0] = r[1]; r[nx - 1] = r[nx - 2]; }
-      else { r[0] = r[1]; r[nxg - 1] = r[nxg - 2]; }
-    } else {
-      if (id == 1) { r[0] = r[nx - 2]; r[nx - 1] = r[1]; }
-      else { r[0] = r[nxg - 3]; r[nxg - 2] = r[1]; r[nxg - 1] = r[2]; }
+__global__ void __launch_bounds__(32 * DC_ROWS, 3)
+    k_dyn_contract(Geo g, const T *__restrict__ U, const T *__restrict__ V, const T *__restrict__ W, P6 SS, P6 M0,
+                   const double *__restrict__ S, int model, double *__restrict__ ml_out, double *__restrict__ mm_out,
+                   T *__restrict__ nut, int kchunk) {
+  const int lane = threadIdx.x, i = 1 + blockIdx.x * 30 + lane, j = blockIdx.y * DC_ROWS + threadIdx.y + 2;
+  const int k0 = 2 + blockIdx.z * kchunk, k1 = min(k0 + kchunk - 1, g.nzg - 1);
+  if (j > g.nyg - 1) return;  // whole warps
+  const int periodic = model == 3;
+  const int ic = min(i, g.nxg);                       // lanes past the last column repeat it
+  const int im = xmap(ic, g.nxg, periodic, false);
+  const bool moved = im != ic;
+  const YW y(j, 2, g.nyg - 1);
+  const int rows[3] = {y.jm, j, y.jp};
+  auto U_ = [&](int x, int r, int k) { return (double)__ldg(U + bidx(g, x, r, k)); };
+  auto V_ = [&](int x, int r, int k) { return (double)__ldg(V + bidx(g, x, r, k)); };
+  auto W_ = [&](int x, int r, int k) { return (double)__ldg(W + bidx(g, x, r, k)); };
+  const bool out = lane >= 1 && lane <= 30 && i <= g.nxg - 1;
+  double lo[15], mid[15];
+#pragma unroll
+  for (int q = 0; q < 15; ++q) lo[q] = mid[q] = 0.0;
+  for (int kk = k0 - 1; kk <= k1 + 1; ++kk) {
+    const int km = zmap(kk, g.nzg);
+    double v[15];
+    {
+      double a[3], b[3], c[3];  // centre velocities at (im, rows, km): the products' entries
+      double vb = V_(im, rows[0] - 1, km);
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        a[r] = 0.5 * (U_(im - 1, rows[r], km) + U_(im, rows[r], km));
+        const double vt = V_(im, rows[r], km);
+        // rows ja and jb repeat a row with a zero weight
+        b[r] = 0.5 * ((r > 0 && rows[r] == rows[r - 1] ? V_(im, rows[r] - 1, km) : vb) + vt);
+        vb = vt;
+        c[r] = 0.5 * (W_(im, rows[r], km - 1) + W_(im, rows[r], km));
+      }
+      v[0] = y(a[0] * a[0], a[1] * a[1], a[2] * a[2]);
+      v[1] = y(b[0] * b[0], b[1] * b[1], b[2] * b[2]);
+      v[2] = y(c[0] * c[0], c[1] * c[1], c[2] * c[2]);
+      v[3] = y(a[0] * b[0], a[1] * b[1], a[2] * b[2]);
+      v[4] = y(a[0] * c[0], a[1] * c[1], a[2] * c[2]);
+      v[5] = y(b[0] * c[0], b[1] * c[1], b[2] * c[2]);
+      // the velocities alone: u with x ghosts only, v with none, w with z ghosts only
+      if (kk != km) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) a[r] = 0.5 * (U_(im - 1, rows[r], kk) + U_(im, rows[r], kk));
+      }
+      if (kk != km || moved) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          b[r] = 0.5 * (V_(ic, rows[r] - 1, kk) + V_(ic, rows[r], kk));
+          c[r] = 0.5 * (W_(ic, rows[r], km - 1) + W_(ic, rows[r], km));
+        }
+      }
+      v[6] = y(a[0], a[1], a[2]);
+      v[7] = y(b[0], b[1], b[2]);
+      v[8] = y(c[0], c[1], c[2]);
     }
-  }
-}
-
-// z ghost planes (planes of pl = d1*d2 entries)
-__global__ void k_bc_z(long long pl, double *__restrict__ a, int id, int nz, int nzg) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < pl; p += (long long)gridDim.x * blockDim.x) {
-    if (id == 3) {
-      a[p] = a[(nz - 2) * pl + p];
-      a[(nz - 1) * pl + p] = a[pl + p];
-    } else {
-      a[p] = a[(nzg - 3) * pl + p];
-      a[(nzg - 2) * pl + p] = a[pl + p];
-      a[(nzg - 1) * pl + p] = a[2 * pl + p];
-    }
-  }
-}
-
-__global__ void k_prod(Geo g, Rng R, double *__restrict__ tb, const double *__restrict__ pa,
-                       const double *__restrict__ pb) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    tb[c] = pa[c] * pb[c];
-  }
-}
-
-// filter_xzy of the section a(1:n1, ja:jb, 1:n3) of a dense (d1,d2,*) array
-// into o(i,j,k), i = 2..n1-1, j = ja..jb, k = 2..n3-1 (output dims e1,e2);
-// the range R carries those output indices.  A block of FK_I threads takes
-// FK_I outputs along i at one j and marches over FK_K planes in k: the
-// y-combined values of input columns i-1..i+FK_I of plane kk go to a ring of
-// three shared rows, and each output sums its 3 x 3 (x,z) neighbourhood from
-// the ring in the source's order (x outer, z inner).
-constexpr int FK_I = 128, FK_K = 16;
-
-__global__ void __launch_bounds__(FK_I) k_filter(Rng R, const double *__restrict__ a, int d1, int d2, int ja,
-                                                 int jb, double *__restrict__ o, int e1, int e2) {
-  const double fil[3][3] = {{1.0 / 36.0, 1.0 / 9.0, 1.0 / 36.0},
-                            {1.0 / 9.0, 4.0 / 9.0, 1.0 / 9.0},
-                            {1.0 / 36.0, 1.0 / 9.0, 1.0 / 36.0}};
-  __shared__ double ys[3][FK_I + 2];
-  const int t = threadIdx.x;
-  const int ib = R.i0 + (int)blockIdx.x * FK_I;  // first output i of the block
-  const int i = ib + t, ilast = R.i0 + R.ni - 1;
-  const int j = R.j0 + (int)blockIdx.y;
-  const int kb = R.k0 + (int)blockIdx.z * FK_K;
-  const int ke = min(kb + FK_K - 1, R.k0 + R.nk - 1);
-  for (int kk = kb - 1; kk <= ke + 1; ++kk) {
-    double *row = ys[(kk - kb + 1) % 3];
-    for (int x = t; x < FK_I + 2; x += FK_I) {
-      const int ii = ib - 1 + x;
-      if (ii <= ilast + 1) {
-        double y;
-        if (j == ja)
-          y = 2.0 / 3.0 * a[dix(ii, j, kk, d1, d2)] + 1.0 / 3.0 * a[dix(ii, j + 1, kk, d1, d2)];
-        else if (j == jb)
-          y = 1.0 / 3.0 * a[dix(ii, j - 1, kk, d1, d2)] + 2.0 / 3.0 * a[dix(ii, j, kk, d1, d2)];
-        else
-          y = 1.0 / 6.0 * a[dix(ii, j - 1, kk, d1, d2)] + 2.0 / 3.0 * a[dix(ii, j, kk, d1, d2)] +
-              1.0 / 6.0 * a[dix(ii, j + 1, kk, d1, d2)];
-        row[x] = y;
+    const long long om = dix(im, rows[0], km, g), oo = dix(im, j, km, g), op = dix(im, rows[2], km, g);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v[9 + m] = y(__ldg(SS.p[m] + om), __ldg(SS.p[m] + oo), __ldg(SS.p[m] + op));
+#pragma unroll
+    for (int q = 0; q < 15; ++q)
+      v[q] = f141(__shfl_up_sync(0xffffffffu, v[q], 1), v[q], __shfl_down_sync(0xffffffffu, v[q], 1));
+    const int k = kk - 1;
+    if (kk >= k0 + 1 && out) {
+      double f[15];
+#pragma unroll
+      for (int q = 0; q < 15; ++q) f[q] = f141(lo[q], mid[q], v[q]);
+      const long long c = dix(i, j, k, g);
+      const double L[6] = {f[0] - f[6] * f[6], f[1] - f[7] * f[7], f[2] - f[8] * f[8],
+                           f[3] - f[6] * f[7], f[4] - f[6] * f[8], f[5] - f[7] * f[8]};
+      double ml = 0.0, mm = 0.0;
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        const double M = M0.p[m][c] - f[9 + m], t = m < 3 ? M : 2.0 * M;
+        ml = __fma_rn(t, L[m], ml);
+        mm = __fma_rn(t, M, mm);
+      }
+      if (model == 2) {
+        ml_out[c] = ml;
+        mm_out[c] = mm;
+      } else {
+        put_periodic(g, nut, i, j, k, -0.5 * (ml / mm) * S[c]);
       }
     }
-    __syncthreads();
-    if (kk >= kb + 1 && i <= ilast) {  // output plane k = kk-1 from planes kk-2, kk-1, kk
-      const int k = kk - 1;
-      double s = 0.0;
-      for (int di = -1; di <= 1; ++di)
-        for (int dk = -1; dk <= 1; ++dk) s = s + ys[(k + dk - kb + 1) % 3][t + 1 + di] * fil[di + 1][dk + 1];
-      o[dix(i, j, k, e1, e2)] = s;
-    }
-    __syncthreads();
-  }
-}
-
-// Lij = hat(ui uj) - hat(ui) hat(uj)
-__global__ void k_leonard(Geo g, Rng R, P6 L, P6 G) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    const double u = G.p[0][c], v = G.p[1][c], w = G.p[2][c];
-    L.p[0][c] = L.p[0][c] - u * u;
-    L.p[1][c] = L.p[1][c] - v * v;
-    L.p[2][c] = L.p[2][c] - w * w;
-    L.p[3][c] = L.p[3][c] - u * v;
-    L.p[4][c] = L.p[4][c] - u * w;
-    L.p[5][c] = L.p[5][c] - v * w;
-  }
-}
-
-struct DV {
-  const double *U, *V, *W;
-  int nx, ny, nxg, nyg;
-  __device__ double u(int i, int j, int k) const { return U[dix(i, j, k, nx, nyg)]; }
-  __device__ double v(int i, int j, int k) const { return V[dix(i, j, k, nxg, ny)]; }
-  __device__ double w(int i, int j, int k) const { return W[dix(i, j, k, nxg, nyg)]; }
-};
-
-// the edge rates of strain of compute_Sij before its corner averages
-__device__ __forceinline__ double e4(const Geo &g, const DV &d, int i, int j, int k) {
-  return 0.5 * ((d.u(i - 1, j, k) - d.u(i - 1, j - 1, k)) / (g.yg[j] - g.yg[j - 1]) +
-                (d.v(i, j - 1, k) - d.v(i - 1, j - 1, k)) / (g.xg[i] - g.xg[i - 1]));
-}
-__device__ __forceinline__ double e5(const Geo &g, const DV &d, int i, int j, int k) {
-  return 0.5 * ((d.u(i - 1, j, k) - d.u(i - 1, j, k - 1)) / (g.zg[k] - g.zg[k - 1]) +
-                (d.w(i, j, k - 1) - d.w(i - 1, j, k - 1)) / (g.xg[i] - g.xg[i - 1]));
-}
-__device__ __forceinline__ double e6(const Geo &g, const DV &d, int i, int j, int k) {
-  return 0.5 * ((d.v(i, j - 1, k) - d.v(i, j - 1, k - 1)) / (g.zg[k] - g.zg[k - 1]) +
-                (d.w(i, j, k - 1) - d.w(i, j - 1, k - 1)) / (g.yg[j] - g.yg[j - 1]));
-}
-
-// compute_Sij's edge values at i = 2..nxg, j = 2..nyg, k = 2..nzg (dense (nxg,nyg) planes)
-__global__ void k_edges(Geo g, Rng R, DV d, double *__restrict__ E4, double *__restrict__ E5,
-                        double *__restrict__ E6) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    E4[c] = e4(g, d, i, j, k);
-    E5[c] = e5(g, d, i, j, k);
-    E6[c] = e6(g, d, i, j, k);
-  }
-}
-
-// Sij (cell centres) and |S| of the velocity triple d, the off-diagonal terms
-// as the source's corner averages of the edge values E4..E6
-__global__ void k_sij(Geo g, Rng R, DV d, const double *__restrict__ E4, const double *__restrict__ E5,
-                      const double *__restrict__ E6, P6 G, double *__restrict__ S) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg), sj = g.nxg, sk = (long long)g.nxg * g.nyg;
-    double s[6];
-    s[0] = (d.u(i, j, k) - d.u(i - 1, j, k)) / (g.x[i] - g.x[i - 1]);
-    s[1] = (d.v(i, j, k) - d.v(i, j - 1, k)) / (g.y[j] - g.y[j - 1]);
-    s[2] = (d.w(i, j, k) - d.w(i, j, k - 1)) / (g.z[k] - g.z[k - 1]);
-    s[3] = 0.25 * (E4[c] + E4[c + 1] + E4[c + sj] + E4[c + 1 + sj]);
-    s[4] = 0.25 * (E5[c] + E5[c + 1] + E5[c + sk] + E5[c + 1 + sk]);
-    s[5] = 0.25 * (E6[c] + E6[c + sj] + E6[c + sk] + E6[c + sj + sk]);
-    double q = 0.0;
-    for (int m = 0; m < 6; ++m) {
-      G.p[m][c] = s[m];
-      q = q + (m < 3 ? 2.0 : 4.0) * s[m] * s[m];
-    }
-    S[c] = sqrt(q);
-  }
-}
-
-// Mij = fil_size^2 |hat(S)| hat(Sij), fil_size = 2
-__global__ void k_mij(Geo g, Rng R, P6 M, P6 G, const double *__restrict__ S) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    for (int m = 0; m < 6; ++m) M.p[m][c] = 4.0 * S[c] * G.p[m][c];
-  }
-}
-
-__global__ void k_ssij(Geo g, Rng R, double *__restrict__ t, const double *__restrict__ S,
-                       const double *__restrict__ Gm) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    t[c] = S[c] * Gm[c];
-  }
-}
-
-__global__ void k_msub(Geo g, Rng R, P6 M, P6 G) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    for (int m = 0; m < 6; ++m) M.p[m][c] = M.p[m][c] - G.p[m][c];
-  }
-}
-
-// Mij Lij and Mij Mij; LES = 3 forms nu_t here, LES = 2 keeps both for the z averages
-__global__ void k_contract(Geo g, Rng R, P6 M, P6 L, const double *__restrict__ S, double *__restrict__ nut,
-                           double *__restrict__ ml_out, double *__restrict__ mm_out, int avg) {
-  FOR_RNG(R) {
-    const long long c = dix(i, j, k, g.nxg, g.nyg);
-    double ml = 0.0;
-    for (int m = 0; m < 6; ++m) {
-      if (m < 3) ml = ml + M.p[m][c] * L.p[m][c];
-      else ml = ml + 2.0 * M.p[m][c] * L.p[m][c];
-    }
-    const double m0 = M.p[0][c], m1 = M.p[1][c], m2 = M.p[2][c], m3 = M.p[3][c], m4 = M.p[4][c], m5 = M.p[5][c];
-    const double mm = m0 * m0 + m1 * m1 + m2 * m2 + 2.0 * (m3 * m3 + m4 * m4 + m5 * m5);
-    if (avg) {
-      ml_out[c] = ml;
-      mm_out[c] = mm;
-    } else {
-      nut[c] = -0.5 * (ml / mm) * S[c];
+#pragma unroll
+    for (int q = 0; q < 15; ++q) {
+      lo[q] = mid[q];
+      mid[q] = v[q];
     }
   }
 }
 
-// LES = 2: <Mij Lij> / <Mij Mij> over k = 2..nzg-2, summed in k order
-__global__ void k_zavg(Geo g, Rng R, const double *__restrict__ ml, const double *__restrict__ mm,
-                       const double *__restrict__ S, double *__restrict__ nut) {
-  FOR_RNG(R) {
-    (void)k;
-    double a = 0.0, b = 0.0;
-    for (int kk = 2; kk <= g.nzg - 2; ++kk) a += ml[dix(i, j, kk, g.nxg, g.nyg)];
-    for (int kk = 2; kk <= g.nzg - 2; ++kk) b += mm[dix(i, j, kk, g.nxg, g.nyg)];
-    const double cz = (a / (double)(g.nzg - 3)) / (b / (double)(g.nzg - 3));
-    for (int kk = 2; kk <= g.nzg - 1; ++kk) {
-      const long long c = dix(i, j, kk, g.nxg, g.nyg);
-      nut[c] = -0.5 * cz * S[c];
-    }
-  }
-}
-
-// clipping, Neumann y, box layout
+// LES = 2: <Mij Lij> / <Mij Mij> over k = 2..nzg-2, summed in k order, and
+// nu_t; the x and z ghosts stay zero as in the source
 template <typename T>
-__global__ void k_store(Geo g, Rng R, const double *__restrict__ nd, T *__restrict__ nut) {
-  FOR_RNG(R) {
-    const int jj = j == 1 ? 2 : (j == g.nyg ? g.nyg - 1 : j);
-    const double v = nd[dix(i, jj, k, g.nxg, g.nyg)];
-    nut[bidx(g, i, j, k)] = (T)(v > 0.0 ? v : 0.0);
+__global__ void __launch_bounds__(128) k_dyn_zavg(Geo g, const double *__restrict__ ml, const double *__restrict__ mm,
+                                                  const double *__restrict__ S, T *__restrict__ nut) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 2;
+  if (i > g.nxg) return;
+  const long long pl = (long long)g.nxg * g.nyg, c = dix(i, j, 1, g);
+  if (i == 1 || i == g.nxg) {
+    for (int k = 1; k <= g.nzg; ++k) put_rows(g, nut, i, j, k, 0.0);
+    return;
   }
-}
-
-// grid-stride launches of 256 threads (x / z ghosts), at most 16 blocks per SM of 148
-inline unsigned blocks(long long n) {
-  const long long b = (n + 255) / 256, cap = 148LL * 16;
-  return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
-}
-
-inline Rng rng(int i0, int i1, int j0, int j1, int k0, int k1) {
-  return Rng{i0, i1 - i0 + 1, j0, j1 - j0 + 1, k0, k1 - k0 + 1};
+  double a = 0.0, b = 0.0;
+#pragma unroll 8
+  for (int k = 2; k <= g.nzg - 2; ++k) {
+    a += __ldg(ml + c + (k - 1) * pl);
+    b += __ldg(mm + c + (k - 1) * pl);
+  }
+  const double cz = (a / (double)(g.nzg - 3)) / (b / (double)(g.nzg - 3));
+  put_rows(g, nut, i, j, 1, 0.0);
+#pragma unroll 4
+  for (int k = 2; k <= g.nzg - 1; ++k) put_rows(g, nut, i, j, k, -0.5 * cz * __ldg(S + c + (k - 1) * pl));
+  put_rows(g, nut, i, j, g.nzg, 0.0);
 }
 
 }  // namespace
@@ -315,90 +317,24 @@ size_t dyn_smagorinsky_work_bytes(int nxg, int nyg, int nzg) {
 template <typename T>
 int launch_dyn_smagorinsky(const Geo &g, const T *U, const T *V, const T *W, double *work, int model, T *nut,
                            cudaStream_t st) {
-  const int nx = g.nx, ny = g.ny, nz = g.nz, nxg = g.nxg, nyg = g.nyg, nzg = g.nzg;
-  const size_t n = (size_t)nxg * nyg * nzg;
+  const size_t n = (size_t)g.nxg * g.nyg * g.nzg;
   double *w[W_COUNT];
   for (int q = 0; q < W_COUNT; ++q) w[q] = work + (size_t)q * n;
-  P6 L, G, M;
-  for (int m = 0; m < 6; ++m) { L.p[m] = w[W_L + m]; G.p[m] = w[W_G + m]; M.p[m] = w[W_M + m]; }
-  const int per = model == 3;
-  int launches = 0;
-  auto go = [&](const Rng &R) { ++launches; return dim3((R.ni + 127) / 128, R.nj, R.nk); };
-  auto bcx = [&](double *a, int d1, int d2, int d3, int id, int periodic) {
-    const long long rows = (long long)d2 * d3;
-    ++launches;
-    k_bc_x<<<blocks(rows), 256, 0, st>>>(rows, a, d1, id, periodic, nx, nxg);
-  };
-  auto bcz = [&](double *a, int d1, int d2, int id) {
-    const long long pl = (long long)d1 * d2;
-    ++launches;
-    k_bc_z<<<blocks(pl), 256, 0, st>>>(pl, a, id, nz, nzg);
-  };
-  auto filt = [&](const double *a, int d1, int d2, int n1, int ja, int jb, int n3, double *o, int e1, int e2) {
-    const Rng R = rng(2, n1 - 1, ja, jb, 2, n3 - 1);
-    ++launches;
-    k_filter<<<dim3((R.ni + FK_I - 1) / FK_I, R.nj, (R.nk + FK_K - 1) / FK_K), FK_I, 0, st>>>(R, a, d1, d2, ja, jb, o,
-                                                                                            e1, e2);
-  };
-  const Rng all = rng(1, nxg, 1, nyg, 1, nzg), in = rng(2, nxg - 1, 2, nyg - 1, 2, nzg - 1);
-  double *Ud = w[W_U], *Vd = w[W_V], *Wd = w[W_W], *t0 = w[W_T0], *t1 = w[W_T1], *t2 = w[W_T2], *S = w[W_S];
-  double *Uf = w[W_UF], *Vf = w[W_VF], *Wf = w[W_WF], *tb = w[W_TB];
-  k_gather<T><<<go(all), 128, 0, st>>>(g, all, U, V, W, Ud, Vd, Wd);
-  // Part 1: Leonard term
-  k_interp<<<go(all), 128, 0, st>>>(g, all, Ud, Vd, Wd, t0, t1, t2);
-  bcx(t0, nxg, nyg, nzg, 2, per);
-  bcz(t2, nxg, nyg, 4);
-  const double *pa[6] = {t0, t1, t2, t0, t0, t1}, *pb[6] = {t0, t1, t2, t1, t2, t2};
-  const Rng rp = rng(2, nxg, 2, nyg - 1, 2, nzg);
-  for (int m = 0; m < 6; ++m) {
-    k_prod<<<go(rp), 128, 0, st>>>(g, rp, tb, pa[m], pb[m]);
-    bcx(tb, nxg, nyg, nzg, 2, per);
-    bcz(tb, nxg, nyg, 4);
-    filt(tb, nxg, nyg, nxg, 2, nyg - 1, nzg, L.p[m], nxg, nyg);
-  }
-  filt(t0, nxg, nyg, nxg, 2, nyg - 1, nzg, G.p[0], nxg, nyg);
-  filt(t1, nxg, nyg, nxg, 2, nyg - 1, nzg, G.p[1], nxg, nyg);
-  filt(t2, nxg, nyg, nxg, 2, nyg - 1, nzg, G.p[2], nxg, nyg);
-  k_leonard<<<go(in), 128, 0, st>>>(g, in, L, G);
-  // Part 2: Mij
-  filt(Ud, nx, nyg, nx, 1, nyg, nzg, Uf, nx, nyg);
-  filt(Vd, nxg, ny, nxg, 1, ny, nzg, Vf, nxg, ny);
-  filt(Wd, nxg, nyg, nxg, 1, nyg, nz, Wf, nxg, nyg);
-  bcx(Uf, nx, nyg, nzg, 1, per);
-  bcz(Uf, nx, nyg, 1);
-  bcx(Vf, nxg, ny, nzg, 2, per);
-  bcz(Vf, nxg, ny, 2);
-  bcx(Wf, nxg, nyg, nz, 2, per);
-  bcz(Wf, nxg, nyg, 3);
-  // t0..t2 are free here: they hold the edge values of each compute_Sij
-  const Rng re = rng(2, nxg, 2, nyg, 2, nzg);
-  const DV df{Uf, Vf, Wf, nx, ny, nxg, nyg}, du{Ud, Vd, Wd, nx, ny, nxg, nyg};
-  k_edges<<<go(re), 128, 0, st>>>(g, re, df, t0, t1, t2);
-  k_sij<<<go(in), 128, 0, st>>>(g, in, df, t0, t1, t2, G, S);
-  k_mij<<<go(in), 128, 0, st>>>(g, in, M, G, S);
-  k_edges<<<go(re), 128, 0, st>>>(g, re, du, t0, t1, t2);
-  k_sij<<<go(in), 128, 0, st>>>(g, in, du, t0, t1, t2, G, S);
-  for (int m = 0; m < 6; ++m) {
-    k_ssij<<<go(in), 128, 0, st>>>(g, in, t0, S, G.p[m]);
-    bcx(t0, nxg, nyg, nzg, 2, per);
-    bcz(t0, nxg, nyg, 4);
-    filt(t0, nxg, nyg, nxg, 2, nyg - 1, nzg, G.p[m], nxg, nyg);
-  }
-  k_msub<<<go(in), 128, 0, st>>>(g, in, M, G);
-  // Part 3: nu_t (tb holds it; entries the source leaves at zero stay zero)
-  cudaMemsetAsync(tb, 0, n * sizeof(double), st);
-  ++launches;  // the memset is one stream operation (one graph node) like a kernel
-  if (model == 2) {
-    k_contract<<<go(in), 128, 0, st>>>(g, in, M, L, S, tb, t1, t2, 1);
-    const Rng ij = rng(2, nxg - 1, 2, nyg - 1, 1, 1);
-    k_zavg<<<go(ij), 128, 0, st>>>(g, ij, t1, t2, S, tb);
-  } else {
-    k_contract<<<go(in), 128, 0, st>>>(g, in, M, L, S, tb, nullptr, nullptr, 0);
-    bcx(tb, nxg, nyg, nzg, 4, 1);
-    bcz(tb, nxg, nyg, 4);
-  }
-  k_store<T><<<go(all), 128, 0, st>>>(g, all, tb, nut);
-  return launches;
+  P6 SS, M;
+  for (int m = 0; m < 6; ++m) { SS.p[m] = w[W_SS + m]; M.p[m] = w[W_M + m]; }
+  const P3 F{{w[W_F], w[W_F + 1], w[W_F + 2]}};
+  const int periodic = model == 3, nk = g.nzg - 2, kc = 16;
+  const dim3 sb(32, 4), sg((g.nxg - 2 + 31) / 32, (g.nyg - 2 + 3) / 4, (nk + kc - 1) / kc);
+  k_dyn_strain<T, LdBox<T>><<<sg, sb, 0, st>>>(g, U, V, W, periodic, 1.0, SS, w[W_S], kc);
+  const dim3 fb(32, 8), fg((g.nxg - 2 + 31) / 32, (g.nyg + 7) / 8, 3 * ((nk + kc - 1) / kc));
+  k_dyn_filter<T><<<fg, fb, 0, st>>>(g, U, V, W, F, kc);
+  k_dyn_strain<double, LdHat><<<sg, sb, 0, st>>>(g, w[W_F], w[W_F + 1], w[W_F + 2], periodic, 4.0, M, nullptr, kc);
+  const int cc = 32;
+  const dim3 cb(32, DC_ROWS), cg((g.nxg - 2 + 29) / 30, (g.nyg - 2 + DC_ROWS - 1) / DC_ROWS, (nk + cc - 1) / cc);
+  k_dyn_contract<T><<<cg, cb, 0, st>>>(g, U, V, W, SS, M, w[W_S], model, w[W_F], w[W_F + 1], nut, cc);
+  if (model != 2) return 4;
+  k_dyn_zavg<T><<<dim3((g.nxg + 127) / 128, g.nyg - 2), 128, 0, st>>>(g, w[W_F], w[W_F + 1], w[W_S], nut);
+  return 5;
 }
 
 template int launch_dyn_smagorinsky<double>(const Geo &, const double *, const double *, const double *, double *,

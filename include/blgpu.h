@@ -53,7 +53,7 @@ typedef struct blgpu_config {
   int les_model;      /* LES, nu_t computed on the device before every substep: 0 DNS;
                          1 constant-coefficient Smagorinsky (subgrid.f90:609-730); 2 dynamic
                          Smagorinsky, coefficient averaged in z (subgrid.f90:261-414); 3 dynamic
-                         Smagorinsky, pointwise (subgrid.f90:420-583); 2 and 3 hold 29 FP64
+                         Smagorinsky, pointwise (subgrid.f90:420-583); 2 and 3 hold 16 FP64
                          work arrays of nxg*nyg*nzg.  BLGPU_LES_HOST: eddy viscosity given by
                          blgpu_set_nu_t and held fixed */
   int precision;      /* BLGPU_FP64 | BLGPU_MIXED */

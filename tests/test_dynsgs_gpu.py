@@ -71,3 +71,31 @@ def test_dynamic_les_mixed_close_to_fp64(gpu, model):
     assert rel(a.nu_t(), b.nu_t()) < 1e-3
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("model", [2, 3])
+@pytest.mark.parametrize("grid", [(5, 4, 5), (31, 5, 17), (32, 9, 33), (62, 8, 18), (63, 6, 36)])
+def test_dynamic_nu_t_tile_edges(gpu, model, grid):
+    """Sizes at the edges of the column kernels' tiles: the smallest box, 30
+    outputs of a 32-column warp (nx = 31: 30 interior columns, 32: 31, 62 and
+    63: 61 and 62), 4 rows a block (ny = 5, 9: 4 and 8 interior rows, 6 and 8:
+    a remainder) and z chunks of 16 and 32 planes with one plane more or less;
+    fields that are periodic in no direction, so that every ghost index
+    counts.  The filters' sums run in another order than the oracle's: the
+    cancellation in Lij = hat(ui uj) - hat(ui) hat(uj) with |u| = 1 and
+    fluctuations of 0.05 leaves 2e-16 / 2e-3 = 1e-13 of Lij, some units of
+    which reach the largest nu_t."""
+    c = noisy(*grid, seed=sum(grid), amp=0.05)
+    o = oracle.oracle_for(c)
+    ref = o.dynamic_smagorinsky(model)
+    for prec, tol in ((FP64, 1e-12), (MIXED, None)):
+        s = cases.solver_for(c, precision=prec, les_model=model)
+        nut = s.compute_eddy_viscosity()
+        if tol is None:  # the same FP64 model on velocities rounded to FP32
+            c32 = noisy(*grid, seed=sum(grid), amp=0.05)
+            for q in "UVW":
+                setattr(c32, q, np.asfortranarray(getattr(c32, q).astype(np.float32).astype(np.float64)))
+            ref = oracle.oracle_for(c32).dynamic_smagorinsky(model)
+            tol = 1.2e-7  # nu_t stored in FP32
+        assert np.abs(nut - ref).max() <= tol * np.abs(ref).max()
+        s.close()
