@@ -1020,6 +1020,10 @@ int blgpu_get_grid(blgpu_ctx *ctx, double *x, double *y, double *z) {
 // ---------------------------------------------------------------------------
 // step orchestration (all enqueued on ctx->st; capturable)
 // ---------------------------------------------------------------------------
+template <typename T> static const MetT<T> &met(const blgpu_ctx *ctx) {
+  return *reinterpret_cast<const MetT<T> *>(ctx->fp64 ? (const void *)&ctx->m64 : (const void *)&ctx->m32);
+}
+
 template <typename T>
 static void enq_bc(blgpu_ctx *ctx, int b, int o, int rk_step) {
   T **S = reinterpret_cast<T **>(ctx->S[b]);
@@ -1057,7 +1061,7 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
     r = cufft_path_inverse_x<T>(ctx->cf, ctx->geo, s, ctx->post, (T *)ctx->rhs_p, ctx->st);
     if (r && !ctx->cf_status) ctx->cf_status = r;
     ph_end(ctx, 3);
-    const MetT<T> &m = *reinterpret_cast<const MetT<T> *>(ctx->fp64 ? (const void *)&ctx->m64 : (const void *)&ctx->m32);
+    const MetT<T> &m = met<T>(ctx);
     ph_begin(ctx, PH_PROJECT);
     launch_project<T>(ctx->geo, m, (const T *)ctx->rhs_p, mixed ? ctx->kz0 : nullptr, mixed ? ctx->kz0g : nullptr,
                       S[0], S[1], S[2], (T *)ctx->P, ctx->sc, rk_step == 1 ? 1 : 0, ctx->tiles, ctx->st);
@@ -1101,7 +1105,7 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
   launch_idct<T>(ctx->geo, s, pl, (const T *)ctx->R, (T *)ctx->rhs_p, ctx->tiles.idct_nw, ctx->tiles.xfft,
                  &ctx->sc->err, ctx->st);
   ph_end(ctx, 1);
-  const MetT<T> &m = *reinterpret_cast<const MetT<T> *>(ctx->fp64 ? (const void *)&ctx->m64 : (const void *)&ctx->m32);
+  const MetT<T> &m = met<T>(ctx);
   ph_begin(ctx, PH_PROJECT);
   launch_project<T>(ctx->geo, m, (const T *)ctx->rhs_p, mixed ? ctx->kz0 : nullptr, mixed ? ctx->kz0g : nullptr,
                     S[0], S[1], S[2],
@@ -1115,7 +1119,7 @@ static void enq_rhs(blgpu_ctx *ctx, int mode, int in, int o, int outb, double c1
   T **So = reinterpret_cast<T **>(ctx->S[o]);
   T **Sn = reinterpret_cast<T **>(ctx->S[outb]);
   T **F = reinterpret_cast<T **>(ctx->F1);
-  const MetT<T> &m = *reinterpret_cast<const MetT<T> *>(ctx->fp64 ? (const void *)&ctx->m64 : (const void *)&ctx->m32);
+  const MetT<T> &m = met<T>(ctx);
   ph_begin(ctx, PH_RHS);
   launch_rhs_rk<T>(ctx->geo, m, mode, ctx->cfg.les_model != 0, Si[0], Si[1], Si[2], (const T *)ctx->nut, So[0], So[1],
                    So[2], F[0], F[1], F[2], Sn[0], Sn[1], Sn[2], ctx->sc, c1, c2, ctx->tiles,
@@ -1162,7 +1166,7 @@ static int enq_step(blgpu_ctx *ctx, int a, bool with_dt) {
     if (ctx->cfg.les_model == 1) {  // Smagorinsky from the substep's state (time_integration.f90:341-346)
       T **Si = reinterpret_cast<T **>(ctx->S[in]);
       ph_begin(ctx, PH_MISC);
-      launch_smagorinsky<T>(ctx->geo, Si[0], Si[1], Si[2], ctx->d_cs2, (T *)ctx->nut, ctx->st);
+      launch_smagorinsky<T>(ctx->geo, met<T>(ctx), Si[0], Si[1], Si[2], ctx->d_cs2, (T *)ctx->nut, ctx->st);
       ph_end(ctx, 1);
     } else if (ctx->dyn) {  // dynamic Smagorinsky, same place (LES = 2, 3)
       T **Si = reinterpret_cast<T **>(ctx->S[in]);
@@ -1483,14 +1487,14 @@ int blgpu_eddy_viscosity(blgpu_ctx *ctx) {
       ctx->launches += launch_dyn_smagorinsky<double>(ctx->geo, S[0], S[1], S[2], ctx->dyn, ctx->cfg.les_model,
                                                       (double *)ctx->nut, ctx->st);
     else
-      launch_smagorinsky<double>(ctx->geo, S[0], S[1], S[2], ctx->d_cs2, (double *)ctx->nut, ctx->st);
+      launch_smagorinsky<double>(ctx->geo, ctx->m64, S[0], S[1], S[2], ctx->d_cs2, (double *)ctx->nut, ctx->st);
   } else {
     float **S = reinterpret_cast<float **>(ctx->S[ctx->cur]);
     if (ctx->dyn)
       ctx->launches += launch_dyn_smagorinsky<float>(ctx->geo, S[0], S[1], S[2], ctx->dyn, ctx->cfg.les_model,
                                                      (float *)ctx->nut, ctx->st);
     else
-      launch_smagorinsky<float>(ctx->geo, S[0], S[1], S[2], ctx->d_cs2, (float *)ctx->nut, ctx->st);
+      launch_smagorinsky<float>(ctx->geo, ctx->m32, S[0], S[1], S[2], ctx->d_cs2, (float *)ctx->nut, ctx->st);
   }
   if (!ctx->dyn) ctx->launches += 1;
   CK(cudaGetLastError());

@@ -14,6 +14,7 @@
 #include <cstring>
 
 #include "kernels.cuh"
+#include "strain.cuh"
 #include "tma.cuh"
 
 namespace blgpu {
@@ -1819,52 +1820,35 @@ __global__ void __launch_bounds__(256) k_maxdiv(Geo g, const T *__restrict__ U, 
 // initialization.f90:586).  Interior points i=2..nxg-1, j=2..nyg-1,
 // k=2..nzg-1 only.
 // ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ T sij4(const Geo &g, const T *U, const T *V, int i, int j, int k) {
-  const long long c = bidx(g, i, j, k);
-  return (T)0.5 * ((U[c - 1] - U[c - 1 - g.px]) / (T)(g.yg[j] - g.yg[j - 1]) +
-                   (V[c - g.px] - V[c - 1 - g.px]) / (T)(g.xg[i] - g.xg[i - 1]));
-}
-template <typename T>
-__device__ __forceinline__ T sij5(const Geo &g, const T *U, const T *W, int i, int j, int k) {
-  const long long c = bidx(g, i, j, k);
-  return (T)0.5 * ((U[c - 1] - U[c - 1 - g.plane]) / (T)(g.zg[k] - g.zg[k - 1]) +
-                   (W[c - g.plane] - W[c - 1 - g.plane]) / (T)(g.xg[i] - g.xg[i - 1]));
-}
-template <typename T>
-__device__ __forceinline__ T sij6(const Geo &g, const T *V, const T *W, int i, int j, int k) {
-  const long long c = bidx(g, i, j, k);
-  return (T)0.5 * ((V[c - g.px] - V[c - g.px - g.plane]) / (T)(g.zg[k] - g.zg[k - 1]) +
-                   (W[c - g.plane] - W[c - g.px - g.plane]) / (T)(g.yg[j] - g.yg[j - 1]));
-}
+// A thread walks a column of cells (StrainColumn, strain.cuh): 17 loads and 19
+// three-instruction quotients a cell, where one thread per cell took 48 loads
+// and 27 divisions.
+template <typename T> struct LdT {
+  const T *U, *V, *W;
+  long long c, px, pl;  // c: box index of (i-1, j, k = 0)
+  __device__ __forceinline__ T at(const T *a, int s, int dj, int k) const { return __ldg(a + c + s + dj * px + k * pl); }
+  __device__ __forceinline__ T u(int s, int dj, int k) const { return at(U, s, dj, k); }
+  __device__ __forceinline__ T v(int s, int dj, int k) const { return at(V, s, dj, k); }
+  __device__ __forceinline__ T w(int s, int dj, int k) const { return at(W, s, dj, k); }
+};
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_smagorinsky(Geo g, const T *__restrict__ U, const T *__restrict__ V,
-                                                     const T *__restrict__ W, const double *__restrict__ cs2,
-                                                     T *__restrict__ nut) {
+__global__ void __launch_bounds__(256) k_smagorinsky(Geo g, MetT<T> m, const T *__restrict__ U,
+                                                     const T *__restrict__ V, const T *__restrict__ W,
+                                                     const double *__restrict__ cs2, T *__restrict__ nut, int kchunk) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
-  const int k = blockIdx.z + 2;
-  if (i > g.nxg - 1 || j > g.nyg - 1 || k > g.nzg - 1) return;
-  const long long c = bidx(g, i, j, k);
-  const T s1 = (U[c] - U[c - 1]) / (T)(g.x[i] - g.x[i - 1]);
-  const T s2 = (V[c] - V[c - g.px]) / (T)(g.y[j] - g.y[j - 1]);
-  const T s3 = (W[c] - W[c - g.plane]) / (T)(g.z[k] - g.z[k - 1]);
-  const T q = (T)0.25;
-  const T s4 = q * (sij4<T>(g, U, V, i, j, k) + sij4<T>(g, U, V, i + 1, j, k) + sij4<T>(g, U, V, i, j + 1, k) +
-                    sij4<T>(g, U, V, i + 1, j + 1, k));
-  const T s5 = q * (sij5<T>(g, U, W, i, j, k) + sij5<T>(g, U, W, i + 1, j, k) + sij5<T>(g, U, W, i, j, k + 1) +
-                    sij5<T>(g, U, W, i + 1, j, k + 1));
-  const T s6 = q * (sij6<T>(g, V, W, i, j, k) + sij6<T>(g, V, W, i, j + 1, k) + sij6<T>(g, V, W, i, j, k + 1) +
-                    sij6<T>(g, V, W, i, j + 1, k + 1));
-  T S = 0;
-  S = S + (T)2 * s1 * s1;
-  S = S + (T)2 * s2 * s2;
-  S = S + (T)2 * s3 * s3;
-  S = S + (T)4 * s4 * s4;
-  S = S + (T)4 * s5 * s5;
-  S = S + (T)4 * s6 * s6;
-  nut[c] = (T)cs2[j] * sqrt(S);
+  if (i > g.nxg - 1 || j > g.nyg - 1) return;
+  const int k0 = 2 + blockIdx.z * kchunk, k1 = min(k0 + kchunk - 1, g.nzg - 1);
+  const LdT<T> ld{U, V, W, bidx(g, i - 1, j, 0), g.px, g.plane};
+  StrainColumn<T, LdT<T>> col(ld, m.xF, m.xrF, m.xC, m.xrC, m.yF, m.yrF, m.yC, m.yrC, m.zF, m.zrF, m.zC, m.zrC, i, j);
+  const T c2 = (T)cs2[j];
+  col.start(k0);
+  for (int k = k0; k <= k1; ++k) {
+    T s[6];
+    const T n = col.cell(k, s);
+    nut[bidx(g, i, j, k)] = c2 * n;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2209,9 +2193,11 @@ void launch_maxdiv(const Geo &g, const T *U, const T *V, const T *W, unsigned lo
 }
 
 template <typename T>
-void launch_smagorinsky(const Geo &g, const T *U, const T *V, const T *W, const double *cs2, T *nut, cudaStream_t st) {
-  dim3 block(32, 8), grid((g.nxg - 2 + 31) / 32, (g.nyg - 2 + 7) / 8, g.nzg - 2);
-  k_smagorinsky<T><<<grid, block, 0, st>>>(g, U, V, W, cs2, nut);
+void launch_smagorinsky(const Geo &g, const MetT<T> &m, const T *U, const T *V, const T *W, const double *cs2, T *nut,
+                        cudaStream_t st) {
+  const int kchunk = 16;
+  k_smagorinsky<T><<<vol_grid(g.nxg - 2, g.nyg - 2, g.nzg - 2, kchunk), dim3(32, 8), 0, st>>>(g, m, U, V, W, cs2, nut,
+                                                                                           kchunk);
 }
 
 template <typename T>
@@ -2239,7 +2225,7 @@ void launch_law_of_wall(const Geo &g, const T *U, double *utau, int *iters, int 
   template void launch_dt<T>(const Geo &, const T *, const T *, const T *, Scalars *, double, double, bool,        \
                              cudaStream_t);                                                                         \
   template void launch_maxdiv<T>(const Geo &, const T *, const T *, const T *, unsigned long long *, cudaStream_t); \
-  template void launch_smagorinsky<T>(const Geo &, const T *, const T *, const T *, const double *, T *,            \
+  template void launch_smagorinsky<T>(const Geo &, const MetT<T> &, const T *, const T *, const T *, const double *, T *, \
                                       cudaStream_t);                                                                \
   template void launch_stats<T>(const Geo &, const T *, const T *, const T *, const T *, const T *, double *,       \
                                 cudaStream_t);                                                                      \

@@ -39,6 +39,29 @@ def test_smagorinsky_matches_oracle(gpu, grid):
     s.close()
 
 
+@pytest.mark.parametrize("grid", [(5, 4, 5), (33, 9, 17), (34, 10, 18), (65, 8, 33)])
+def test_smagorinsky_tile_edges(gpu, grid):
+    """Column kernel at its tile edges: the smallest box, 32 interior columns
+    and one more, 8 rows and one more, z chunks of 16 planes and one more (17
+    and 32 interior planes).  FP64 repeats the oracle's expressions; FP32
+    forms some 40 rounded operations from differences of O(1) velocities
+    (each 6e-8 of |u|, over the smallest spacing)."""
+    c = noisy(*grid, seed=sum(grid), amp=0.05)
+    ref = oracle.oracle_for(c).smagorinsky()
+    inner = (slice(1, -1), slice(1, -1), slice(1, -1))
+    h = min(np.diff(a).min() for a in (c.x, c.y, c.z))
+    for prec in (FP64, MIXED):
+        s = cases.solver_for(c, precision=prec, les_model=1)
+        nut = s.compute_eddy_viscosity()
+        if prec == FP64:
+            tol = 1e-14 * np.abs(ref).max()
+        else:  # (Cs Delta)^2 times the strain's rounding, 4 differences of two rounded values
+            tol = 40 * 6e-8 * np.abs(ref).max() + 8 * 6e-8 / h * 0.11 ** 2 * np.diff(c.y).max() ** (2 / 3) * (
+                np.diff(c.x).min() * np.diff(c.z).min()) ** (2 / 3)
+        assert np.abs(nut[inner] - ref[inner]).max() <= tol
+        s.close()
+
+
 def test_les_steps_match_oracle(gpu):
     c = noisy(40, 13, 18, seed=22, amp=2e-3, cfl=-2e-3)
     s = cases.solver_for(c, les_model=1)
