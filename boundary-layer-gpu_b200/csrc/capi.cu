@@ -65,7 +65,7 @@ struct blgpu_ctx {
   uint32_t *utab = nullptr;   // mixed form: tcgen05 z transforms, tables (or null)
   ZdftMaps umaps{};           // and their TMA maps
   ThomasMaps tmaps{};         // TMA maps of C and the pivots for the tiled y-solve
-  RhsMaps rmaps[4]{};         // TMA maps of U, V, W of each state buffer and of F1 (TMA-fed RHS)
+  RhsMaps rmaps[5]{};         // TMA maps of U, V, W of each state buffer, of F1 and of nu_t (TMA-fed RHS)
   bool have_rmaps = false;
   CufftPath *cf = nullptr;    // poisson = BLGPU_POISSON_CUFFT: plans and work arrays
   int cf_status = 0;          // first failing cufftExec status of an enqueued step (0: none)
@@ -277,20 +277,22 @@ int blgpu_create(const blgpu_config *cfg, blgpu_ctx **out) {
   for (int b = 0; b < 3; ++b)
     for (int q = 0; q < 3; ++q) TRY(dalloc(ctx, &ctx->S[b][q], box));
   for (int q = 0; q < 3; ++q) TRY(dalloc(ctx, &ctx->F1[q], box));
+  if (cfg->les_model) TRY(dalloc(ctx, &ctx->nut, box));
   {  // plane maps of the TMA-fed RHS: each state buffer and F1
     const Geo gb = ctx->geo_box();
-    auto enc = [&](void *const *f, RhsMaps *out) {
-      return ctx->fp64 ? rhs_maps64(gb, (const double *)f[0], (const double *)f[1], (const double *)f[2], out)
-                       : rhs_maps(gb, (const float *)f[0], (const float *)f[1], (const float *)f[2], out);
+    const bool one = ctx->fp64 || cfg->les_model != 0;
+    auto enc = [&](void *const *f, int nf, RhsMaps *out) {
+      return ctx->fp64 ? rhs_maps<double>(gb, one, (const double *const *)f, nf, out)
+                       : rhs_maps<float>(gb, one, (const float *const *)f, nf, out);
     };
     ctx->have_rmaps = true;
     for (int b = 0; b < 3; ++b)
-      if (!enc(ctx->S[b], &ctx->rmaps[b])) ctx->have_rmaps = false;
-    if (!enc(ctx->F1, &ctx->rmaps[3])) ctx->have_rmaps = false;
+      if (!enc(ctx->S[b], 3, &ctx->rmaps[b])) ctx->have_rmaps = false;
+    if (!enc(ctx->F1, 3, &ctx->rmaps[3])) ctx->have_rmaps = false;
+    if (cfg->les_model && !enc(&ctx->nut, 1, &ctx->rmaps[4])) ctx->have_rmaps = false;
   }
   TRY(dalloc(ctx, &ctx->P, box));
   TRY(dalloc(ctx, &ctx->rhs_p, box));
-  if (cfg->les_model) TRY(dalloc(ctx, &ctx->nut, box));
   if (cfg->les_model == 2 || cfg->les_model == 3)
     TRY(dalloc(ctx, (void **)&ctx->dyn, dyn_smagorinsky_work_bytes(ctx->nxg, ctx->nyg, ctx->nzg)));
   Spec &s = ctx->spec;
@@ -1124,7 +1126,7 @@ static void enq_rhs(blgpu_ctx *ctx, int mode, int in, int o, int outb, double c1
   launch_rhs_rk<T>(ctx->geo, m, mode, ctx->cfg.les_model != 0, Si[0], Si[1], Si[2], (const T *)ctx->nut, So[0], So[1],
                    So[2], F[0], F[1], F[2], Sn[0], Sn[1], Sn[2], ctx->sc, c1, c2, ctx->tiles,
                    ctx->have_rmaps ? &ctx->rmaps[in] : nullptr, ctx->have_rmaps ? &ctx->rmaps[o] : nullptr,
-                   ctx->have_rmaps ? &ctx->rmaps[3] : nullptr, &ctx->sc->err, ctx->wait_limit, ctx->st);
+                   ctx->have_rmaps ? &ctx->rmaps[3] : nullptr, ctx->have_rmaps && ctx->nut ? &ctx->rmaps[4] : nullptr, &ctx->sc->err, ctx->wait_limit, ctx->st);
   ph_end(ctx, 1);
 }
 

@@ -68,19 +68,19 @@ struct RhsMaps {  // CUtensorMap bytes of the planes of U, V, W of one FP32 buff
   alignas(64) unsigned char f[3][128];  // neighbourhood tiles (72 x 10)
   alignas(64) unsigned char p[3][128];  // point-wise tiles (64 x 8)
 };
-// false when a map cannot be encoded (the RHS then uses the kernels with
-// global loads)
-bool rhs_maps(const Geo &g, const float *U, const float *V, const float *W, RhsMaps *out);
-bool rhs_maps64(const Geo &g, const double *U, const double *V, const double *W, RhsMaps *out);
-// mi, mo, mf: tensor maps of the buffers of U V W, Uo Vo Wo and F1 (the
-// TMA-fed DNS kernels: FP32 with rhs_pts 0 or 4, FP64 unless rhs_pts 1), or null; err: device flag, bit 64 set when a plane
+// maps of nf fields (U, V, W, or nu_t alone) with the tiles of the packed FP32
+// DNS kernel or, one_point, of the kernel of FP64 and LES; false when a map
+// cannot be encoded (the RHS then uses the kernels with global loads)
+template <typename T> bool rhs_maps(const Geo &g, bool one_point, const T *const *f, int nf, RhsMaps *out);
+// mi, mo, mf, mn: tensor maps of the buffers of U V W, Uo Vo Wo, F1 and nu_t (the
+// TMA-fed DNS kernels: FP32 with rhs_pts 0 or 4, FP64 with rhs_pts 4; the LES kernel unless rhs_pts 1), or null; err: device flag, bit 64 set when a plane
 // copy missed its wait limit; wait_limit: mbarrier polls before giving up
 // (< 0: the built-in limit)
 template <typename T>
 void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *U, const T *V, const T *W,
                    const T *nut, const T *Uo, const T *Vo, const T *Wo, T *F1u, T *F1v, T *F1w, T *Un, T *Vn, T *Wn,
                    const Scalars *sc, double c1, double c2, const Tiles &tl, const RhsMaps *mi, const RhsMaps *mo,
-                   const RhsMaps *mf, int *err, int wait_limit, cudaStream_t st);
+                   const RhsMaps *mf, const RhsMaps *mn, int *err, int wait_limit, cudaStream_t st);
 template <typename T>
 void launch_project(const Geo &g, const MetT<T> &m, const T *p, const double *p0, const float *p0g, T *U, T *V,
                     T *W, T *P,

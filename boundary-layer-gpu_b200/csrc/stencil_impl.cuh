@@ -983,54 +983,67 @@ drain:
 }
 
 // ---------------------------------------------------------------------------
-// The FP64 DNS RHS fed by TMA.  The arithmetic is rhs_*_at and the RK update
-// of k_rhs_rk, term for term (the FP64 unit is compiled without contraction,
-// so the results are those of k_rhs_rk bit for bit); only the operands come
+// The one-point RHS fed by TMA: the FP64 DNS form (rhs_pts = 4) and the LES
+// form of both precisions, where the viscosity's neighbourhood makes four
+// fields of 27 points each.  The arithmetic is rhs_*_at and the RK update of
+// k_rhs_rk, term for term (the FP64 unit is compiled without contraction, so
+// its results are those of k_rhs_rk bit for bit); only the operands come
 // from shared memory.  A CTA of 32 x 8 threads owns 32 x-points (one per
-// thread) by 8 rows and walks a chunk of k-planes.  Plane p of U, V, W
-// arrives as one 36 x 10 x 1 tensor copy per field (x from the CTA's first
-// point - 2, so the copy starts on a 16-byte boundary; rows j-1 .. j+8) and,
-// for the planes the CTA updates, Uo, Vo, Wo and F1 as 32 x 8 x 1 copies.  A
-// ring of 5 stages holds plane p in stage (p - k0 + 1) mod 5: plane k is
-// computed from planes k-1, k and k+1 while k+2 and k+3 are in flight, and
-// after a CTA barrier the stage of plane k-1 takes plane k+4.  The k loop is
-// unrolled by the ring length.  Wait limits and the drain as in k_rhs_rk_tma.
+// thread) by 8 rows and walks a chunk of k-planes.  Plane p of U, V, W (and
+// nu_t) arrives as one tensor copy of 10 rows per field (rows j-1 .. j+8),
+// 36 doubles from the CTA's first point - 2 or 40 floats from the point - 4,
+// so the copy starts on a 16-byte boundary, and, for the planes the CTA
+// updates, Uo, Vo, Wo and F1 as 32 x 8 x 1 copies.  A ring of R1_NS stages
+// holds plane p in stage (p - k0 + 1) mod R1_NS: plane k is computed from
+// planes k-1, k and k+1 while the next ones are in flight, and after a CTA
+// barrier the stage of plane k-1 is refilled.  The k loop is unrolled by the
+// ring length.  Wait limits and the drain as in k_rhs_rk_tma.
 // ---------------------------------------------------------------------------
-constexpr int R64_NS = 5, R64_TW = 36, R64_BY = 8, R64_TH = R64_BY + 2;
-constexpr int R64_FS = (R64_TH * R64_TW * 8 + 127) / 128 * 16;  // doubles per field tile (a 128-byte multiple)
-constexpr int R64_PS = 32 * R64_BY;                             // doubles per point-wise tile
-__host__ __device__ constexpr int r64_stage(int mode) { return 3 * R64_FS + rt_npw(mode) * R64_PS; }  // doubles
-__host__ __device__ constexpr size_t r64_smem(int mode) {
-  return (size_t)R64_NS * r64_stage(mode) * 8 + R64_NS * 8 + 16;
-}
+constexpr int R64_BY = 8, R64_TH = R64_BY + 2;
+// ring length: 4 with LES, where a fifth stage would cost a CTA per SM
+template <bool LES> constexpr int R1_NS = LES ? 4 : 5;
+// x from the CTA's first point - R1_XO, R1_TW values a row
+template <typename T> constexpr int R1_XO = sizeof(T) == 8 ? 2 : 4;
+template <typename T> constexpr int R1_TW = sizeof(T) == 8 ? 36 : 40;
+// values per field tile (a 128-byte multiple) and per point-wise tile
+template <typename T> constexpr int R1_FS = (R64_TH * R1_TW<T> * (int)sizeof(T) + 127) / 128 * (128 / (int)sizeof(T));
+constexpr int R64_PS = 32 * R64_BY;
+template <typename T, int MODE, bool LES>
+constexpr int R1_STAGE = (LES ? 4 : 3) * R1_FS<T> + rt_npw(MODE) * R64_PS;
+template <typename T, int MODE, bool LES>
+constexpr size_t R1_SMEM = (size_t)R1_NS<LES> * R1_STAGE<T, MODE, LES> * sizeof(T) + R1_NS<LES> * 8 + 16;
 
 // operand loader of rhs_*_at over the staged planes k-1, k, k+1 (pointers at
 // the thread's point; di, dj, dk in -1..1 are compile-time at every call)
-struct SmemLd64 {
-  const double *pb, *pc, *pt;
-  __device__ __forceinline__ double operator()(long long, int di, int dj, int dk) const {
-    return (dk < 0 ? pb : dk > 0 ? pt : pc)[di + dj * R64_TW];
+template <typename T> struct SmemLd1 {
+  const T *pb, *pc, *pt;
+  __device__ __forceinline__ T operator()(long long, int di, int dj, int dk) const {
+    return (dk < 0 ? pb : dk > 0 ? pt : pc)[di + dj * R1_TW<T>];
   }
 };
 
-template <int MODE>
-__global__ void __launch_bounds__(32 * R64_BY, 2)
-    k_rhs_rk_tma64(const __grid_constant__ CUtensorMap mu, const __grid_constant__ CUtensorMap mv,
+template <typename T, int MODE, bool LES>
+__global__ void __launch_bounds__(32 * R64_BY, sizeof(T) == 8 ? 2 : 3)
+    k_rhs_rk_tma1(const __grid_constant__ CUtensorMap mu, const __grid_constant__ CUtensorMap mv,
                    const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mou,
                    const __grid_constant__ CUtensorMap mov, const __grid_constant__ CUtensorMap mow,
                    const __grid_constant__ CUtensorMap mfu, const __grid_constant__ CUtensorMap mfv,
-                   const __grid_constant__ CUtensorMap mfw, Geo g, MetT<double> m, double *__restrict__ F1u,
-                   double *__restrict__ F1v, double *__restrict__ F1w, double *__restrict__ Un,
-                   double *__restrict__ Vn, double *__restrict__ Wn, const Scalars *__restrict__ sc, double c1,
+                   const __grid_constant__ CUtensorMap mfw, const __grid_constant__ CUtensorMap mn, Geo g, MetT<T> m, T *__restrict__ F1u,
+                   T *__restrict__ F1v, T *__restrict__ F1w, T *__restrict__ Un,
+                   T *__restrict__ Vn, T *__restrict__ Wn, const Scalars *__restrict__ sc, double c1,
                    double c2, int kchunk, int *err, int wait_limit) {
-  constexpr int NS = R64_NS, TW = R64_TW, NPW = rt_npw(MODE), SS = r64_stage(MODE);
-  constexpr uint32_t FIELD_BYTES = 3u * TW * R64_TH * 8u, PW_BYTES = (uint32_t)NPW * R64_PS * 8u;
-  extern __shared__ __align__(1024) double r64_sm[];
+  constexpr int NS = R1_NS<LES>, TW = R1_TW<T>, FS = R1_FS<T>, NF = LES ? 4 : 3, NPW = rt_npw(MODE),
+                SS = R1_STAGE<T, MODE, LES>;
+  constexpr uint32_t ES = sizeof(T);
+  constexpr uint32_t FIELD_BYTES = NF * TW * R64_TH * ES, PW_BYTES = (uint32_t)NPW * R64_PS * ES;
+  extern __shared__ __align__(1024) unsigned char r1_raw[];
+  T *r64_sm = reinterpret_cast<T *>(r1_raw);
   uint64_t *full = reinterpret_cast<uint64_t *>(r64_sm + NS * SS);
   volatile int *bad = reinterpret_cast<volatile int *>(full + NS);
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
   const int istart = 2 + 32 * blockIdx.x, jstart = 2 + R64_BY * blockIdx.y;
   const int i = istart + tx, j = jstart + ty;
+  const int xs = istart + 2 - R1_XO<T>;  // box column of point i is i + 2
   const int k0 = blockIdx.z * kchunk + 2;
   const int k1 = min(k0 + kchunk - 1, g.nz);
   if (k0 > k1) return;  // whole CTA
@@ -1047,14 +1060,15 @@ __global__ void __launch_bounds__(32 * R64_BY, 2)
   }
   auto issue = [&](int p) {  // thread 0: plane p into its stage
     const int s = (p - k0 + 1) % NS;
-    double *st = r64_sm + s * SS;
+    T *st = r64_sm + s * SS;
     const bool pw = NPW > 0 && p >= k0 && p <= k1;
     tma::mbar_expect_tx(&full[s], FIELD_BYTES + (pw ? PW_BYTES : 0u));
-    tma::load_3d(st, &mu, istart, jstart - 2, p - 1, &full[s]);
-    tma::load_3d(st + R64_FS, &mv, istart, jstart - 2, p - 1, &full[s]);
-    tma::load_3d(st + 2 * R64_FS, &mw, istart, jstart - 2, p - 1, &full[s]);
+    tma::load_3d(st, &mu, xs, jstart - 2, p - 1, &full[s]);
+    tma::load_3d(st + FS, &mv, xs, jstart - 2, p - 1, &full[s]);
+    tma::load_3d(st + 2 * FS, &mw, xs, jstart - 2, p - 1, &full[s]);
+    if (LES) tma::load_3d(st + 3 * FS, &mn, xs, jstart - 2, p - 1, &full[s]);
     if (pw) {
-      double *pt = st + 3 * R64_FS;
+      T *pt = st + NF * FS;
       tma::load_3d(pt, &mou, istart + 2, jstart - 1, p - 1, &full[s]);
       tma::load_3d(pt + R64_PS, &mov, istart + 2, jstart - 1, p - 1, &full[s]);
       tma::load_3d(pt + 2 * R64_PS, &mow, istart + 2, jstart - 1, p - 1, &full[s]);
@@ -1078,12 +1092,12 @@ __global__ void __launch_bounds__(32 * R64_BY, 2)
     }
   };
   // per-thread offsets: field tiles at row j (tile row ty + 1), column of
-  // point i (tx + 2); point-wise tiles at row ty, column tx
-  const double *fo = r64_sm + (ty + 1) * TW + 2 + tx;
-  const double *po = r64_sm + 3 * R64_FS + ty * 32 + tx;
+  // point i (tx + R1_XO); point-wise tiles at row ty, column tx
+  const T *fo = r64_sm + (ty + 1) * TW + R1_XO<T> + tx;
+  const T *po = r64_sm + NF * FS + ty * 32 + tx;
   double dt = 0.0;
   if (MODE != 0) dt = sc->dt;
-  const double cdt1 = dt * c1, tdt = dt, tc1 = c1, tc2 = c2;
+  const T cdt1 = (T)(dt * c1), tdt = (T)dt, tc1 = (T)c1, tc2 = (T)c2;
   const bool du = (i <= g.nx - 1), dv = (j <= g.ny - 1);
   wait_plane(k0 - 1);
   wait_plane(k0);
@@ -1093,25 +1107,26 @@ __global__ void __launch_bounds__(32 * R64_BY, 2)
       const int SB = u, SC = (u + 1) % NS, ST = (u + 2) % NS;  // stages of planes k-1, k, k+1
       wait_plane(k + 1);
       if (act) {
-        const SmemLd64 LU{fo + SB * SS, fo + SC * SS, fo + ST * SS};
-        const SmemLd64 LV{fo + SB * SS + R64_FS, fo + SC * SS + R64_FS, fo + ST * SS + R64_FS};
-        const SmemLd64 LW{fo + SB * SS + 2 * R64_FS, fo + SC * SS + 2 * R64_FS, fo + ST * SS + 2 * R64_FS};
-        const double *pw = po + SC * SS;
+        const SmemLd1<T> LU{fo + SB * SS, fo + SC * SS, fo + ST * SS};
+        const SmemLd1<T> LV{fo + SB * SS + FS, fo + SC * SS + FS, fo + ST * SS + FS};
+        const SmemLd1<T> LW{fo + SB * SS + 2 * FS, fo + SC * SS + 2 * FS, fo + ST * SS + 2 * FS};
+        const SmemLd1<T> LN{fo + SB * SS + (NF - 1) * FS, fo + SC * SS + (NF - 1) * FS, fo + ST * SS + (NF - 1) * FS};
+        const T *pw = po + SC * SS;
         const long long c = bidx(g, i, j, k);
         if (du) {
-          double f = (i == g.nx - 1) ? 0.0 : rhs_u_at<double, false, SmemLd64>(g, m, LU, LV, LW, LU, c, i, j, k);
+          T f = (i == g.nx - 1) ? (T)0 : rhs_u_at<T, LES, SmemLd1<T>>(g, m, LU, LV, LW, LN, c, i, j, k);
           if (MODE == 0) F1u[c] = f;
           else if (MODE == 1) { F1u[c] = f; Un[c] = pw[0] + cdt1 * f; }
           else Un[c] = pw[0] + tdt * (tc1 * pw[3 * R64_PS] + tc2 * f);
         }
         if (dv) {
-          double f = (i == g.nx) ? 0.0 : rhs_v_at<double, false, SmemLd64>(g, m, LU, LV, LW, LU, c, i, j, k);
+          T f = (i == g.nx) ? (T)0 : rhs_v_at<T, LES, SmemLd1<T>>(g, m, LU, LV, LW, LN, c, i, j, k);
           if (MODE == 0) F1v[c] = f;
           else if (MODE == 1) { F1v[c] = f; Vn[c] = pw[R64_PS] + cdt1 * f; }
           else Vn[c] = pw[R64_PS] + tdt * (tc1 * pw[4 * R64_PS] + tc2 * f);
         }
         if (k <= g.nz - 1) {
-          double f = (i == g.nx) ? 0.0 : rhs_w_at<double, false, SmemLd64>(g, m, LU, LV, LW, LU, c, i, j, k);
+          T f = (i == g.nx) ? (T)0 : rhs_w_at<T, LES, SmemLd1<T>>(g, m, LU, LV, LW, LN, c, i, j, k);
           if (MODE == 0) F1w[c] = f;
           else if (MODE == 1) { F1w[c] = f; Wn[c] = pw[2 * R64_PS] + cdt1 * f; }
           else Wn[c] = pw[2 * R64_PS] + tdt * (tc1 * pw[5 * R64_PS] + tc2 * f);
@@ -1944,18 +1959,20 @@ static inline dim3 vol_grid(int ni, int nj, int nk, int kchunk, int by = 8) {
   return dim3((ni + 31) / 32, (nj + by - 1) / by, (nk + kchunk - 1) / kchunk);
 }
 
-#ifndef BLGPU_STENCIL_PRIMARY
-// planes of U, V, W as (px, py, nzg) FP32 tensors: boxes of 72 x 10 x 1
-// (neighbourhood tiles) and 64 x 8 x 1 (point-wise tiles)
-bool rhs_maps(const Geo &g, const float *U, const float *V, const float *W, RhsMaps *out) {
+// planes of U, V, W (or nu_t alone) as (px, py, nzg) tensors: boxes of the
+// neighbourhood and the point-wise tiles of the kernel that reads them, the
+// packed FP32 DNS kernel or the one-point one
+template <typename T>
+bool rhs_maps(const Geo &g, bool one_point, const T *const *f, int nf, RhsMaps *out) {
+  const CUtensorMapDataType ty = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   const cuuint64_t dims[3] = {(cuuint64_t)g.px, (cuuint64_t)g.py, (cuuint64_t)g.nzg};
-  const cuuint64_t strides[2] = {(cuuint64_t)g.px * 4, (cuuint64_t)g.plane * 4};
-  const cuuint32_t fbox[3] = {RT_TW, RT_TH, 1}, pbox[3] = {64, RT_BY, 1};
-  const float *a[3] = {U, V, W};
-  for (int q = 0; q < 3; ++q) {
+  const cuuint64_t strides[2] = {(cuuint64_t)g.px * sizeof(T), (cuuint64_t)g.plane * sizeof(T)};
+  const cuuint32_t fbox[3] = {(cuuint32_t)(one_point ? R1_TW<T> : RT_TW), (cuuint32_t)(one_point ? R64_TH : RT_TH), 1};
+  const cuuint32_t pbox[3] = {(cuuint32_t)(one_point ? 32 : 64), (cuuint32_t)(one_point ? R64_BY : RT_BY), 1};
+  for (int q = 0; q < nf; ++q) {
     CUtensorMap mf, mp;
-    if (!tma::encode(&mf, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(a[q]), dims, strides, fbox) ||
-        !tma::encode(&mp, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(a[q]), dims, strides, pbox))
+    if (!tma::encode(&mf, ty, 3, const_cast<T *>(f[q]), dims, strides, fbox) ||
+        !tma::encode(&mp, ty, 3, const_cast<T *>(f[q]), dims, strides, pbox))
       return false;
     static_assert(sizeof(CUtensorMap) == sizeof(out->f[0]), "tensor map size");
     memcpy(out->f[q], &mf, sizeof mf);
@@ -1963,49 +1980,25 @@ bool rhs_maps(const Geo &g, const float *U, const float *V, const float *W, RhsM
   }
   return true;
 }
-#endif
+template bool rhs_maps<BLGPU_STENCIL_T>(const Geo &, bool, const BLGPU_STENCIL_T *const *, int, RhsMaps *);
 
-#ifdef BLGPU_STENCIL_PRIMARY
-// planes of U, V, W as (px, py, nzg) FP64 tensors: boxes of 36 x 10 x 1
-// (neighbourhood tiles) and 32 x 8 x 1 (point-wise tiles)
-bool rhs_maps64(const Geo &g, const double *U, const double *V, const double *W, RhsMaps *out) {
-  const cuuint64_t dims[3] = {(cuuint64_t)g.px, (cuuint64_t)g.py, (cuuint64_t)g.nzg};
-  const cuuint64_t strides[2] = {(cuuint64_t)g.px * 8, (cuuint64_t)g.plane * 8};
-  const cuuint32_t fbox[3] = {R64_TW, R64_TH, 1}, pbox[3] = {32, R64_BY, 1};
-  const double *a[3] = {U, V, W};
-  for (int q = 0; q < 3; ++q) {
-    CUtensorMap mf, mp;
-    if (!tma::encode(&mf, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(a[q]), dims, strides, fbox) ||
-        !tma::encode(&mp, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(a[q]), dims, strides, pbox))
-      return false;
-    memcpy(out->f[q], &mf, sizeof mf);
-    memcpy(out->p[q], &mp, sizeof mp);
-  }
-  return true;
-}
-#endif
-
-template <int MODE>
-static void launch_rhs_tma64(const Geo &g, const MetT<double> &m, const RhsMaps &mi, const RhsMaps &mo,
-                             const RhsMaps &mf, double *F1u, double *F1v, double *F1w, double *Un, double *Vn,
-                             double *Wn, const Scalars *sc, double c1, double c2, int kc, int *err, int wait_limit,
-                             cudaStream_t st) {
-  CUtensorMap t[9];
+template <typename T, int MODE, bool LES>
+static void launch_rhs_tma1(const Geo &g, const MetT<T> &m, const RhsMaps &mi, const RhsMaps &mo, const RhsMaps &mf,
+                            const RhsMaps &mn, T *F1u, T *F1v, T *F1w, T *Un, T *Vn, T *Wn, const Scalars *sc,
+                            double c1, double c2, int kc, int *err, int wait_limit, cudaStream_t st) {
+  CUtensorMap t[10];
   for (int q = 0; q < 3; ++q) {
     memcpy(&t[q], mi.f[q], sizeof(CUtensorMap));
     memcpy(&t[3 + q], mo.p[q], sizeof(CUtensorMap));
     memcpy(&t[6 + q], mf.p[q], sizeof(CUtensorMap));
   }
-  const size_t sm = r64_smem(MODE);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_rhs_rk_tma64<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr = true;
-  }
+  memcpy(&t[9], mn.f[0], sizeof(CUtensorMap));
+  constexpr size_t sm = R1_SMEM<T, MODE, LES>;
+  cudaFuncSetAttribute(k_rhs_rk_tma1<T, MODE, LES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   const dim3 grid = vol_grid(g.nx - 1, g.ny - 1, g.nz - 1, kc, R64_BY);
-  k_rhs_rk_tma64<MODE><<<grid, dim3(32, R64_BY), sm, st>>>(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], g,
-                                                           m, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, kc, err,
-                                                           wait_limit < 0 ? tma::WAIT_LIMIT : wait_limit);
+  k_rhs_rk_tma1<T, MODE, LES><<<grid, dim3(32, R64_BY), sm, st>>>(
+      t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], g, m, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, kc, err,
+      wait_limit < 0 ? tma::WAIT_LIMIT : wait_limit);
 }
 
 template <int MODE>
@@ -2035,13 +2028,20 @@ template <typename T>
 void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *U, const T *V, const T *W,
                    const T *nut, const T *Uo, const T *Vo, const T *Wo, T *F1u, T *F1v, T *F1w, T *Un, T *Vn, T *Wn,
                    const Scalars *sc, double c1, double c2, const Tiles &tl, const RhsMaps *mi, const RhsMaps *mo,
-                   const RhsMaps *mf, int *err, int wait_limit, cudaStream_t st) {
+                   const RhsMaps *mf, const RhsMaps *mn, int *err, int wait_limit, cudaStream_t st) {
   const int kchunk = tl.rhs_kc > 0 ? tl.rhs_kc : 8;
   const int by = tl.rhs_by > 0 ? tl.rhs_by : 8;
   dim3 grid = vol_grid(g.nx - 1, g.ny - 1, g.nz - 1, kchunk, by), block(32, by);
 #define BLGPU_RHS_CASE(M, L)                                                                             \
   k_rhs_rk<T, M, L><<<grid, block, 0, st>>>(g, m, U, V, W, nut, Uo, Vo, Wo, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, \
                                             c2, kchunk)
+#define BLGPU_TMA1_CASE(L, KC, MN)                                                                                    \
+  switch (mode) {                                                                                                   \
+    case 0: launch_rhs_tma1<T, 0, L>(g, m, *mi, *mo, *mf, MN, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, KC, err, wait_limit, st); break; \
+    case 1: launch_rhs_tma1<T, 1, L>(g, m, *mi, *mo, *mf, MN, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, KC, err, wait_limit, st); break; \
+    case 2: launch_rhs_tma1<T, 2, L>(g, m, *mi, *mo, *mf, MN, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, KC, err, wait_limit, st); break; \
+    default: launch_rhs_tma1<T, 3, L>(g, m, *mi, *mo, *mf, MN, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, KC, err, wait_limit, st); break; \
+  }
   if (!les && sizeof(T) == 4) {  // FP32: register-window kernel (FP64 keeps the lower-register form)
     const bool pair = tl.rhs_pts != 1;
     // the TMA-fed kernel serves the default where its maps exist (16 planes
@@ -2095,12 +2095,7 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
       }
       if (tl.rhs_pts == 4 && mi && mo && mf) {
         const int kc = tl.rhs_kc > 0 ? tl.rhs_kc : 32;
-        switch (mode) {
-          case 0: launch_rhs_tma64<0>(g, m, *mi, *mo, *mf, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, kc, err, wait_limit, st); break;
-          case 1: launch_rhs_tma64<1>(g, m, *mi, *mo, *mf, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, kc, err, wait_limit, st); break;
-          case 2: launch_rhs_tma64<2>(g, m, *mi, *mo, *mf, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, kc, err, wait_limit, st); break;
-          default: launch_rhs_tma64<3>(g, m, *mi, *mo, *mf, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, c2, kc, err, wait_limit, st); break;
-        }
+        BLGPU_TMA1_CASE(false, kc, *mi);
         return;
       }
     }
@@ -2110,6 +2105,8 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
       case 2: BLGPU_RHS_CASE(2, false); break;
       default: BLGPU_RHS_CASE(3, false); break;
     }
+  } else if (tl.rhs_pts != 1 && mi && mo && mf && mn) {
+    BLGPU_TMA1_CASE(true, tl.rhs_kc > 0 ? tl.rhs_kc : 16, *mn);
   } else {
     switch (mode) {
       case 0: BLGPU_RHS_CASE(0, true); break;
@@ -2119,6 +2116,7 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
     }
   }
 #undef BLGPU_RHS_CASE
+#undef BLGPU_TMA1_CASE
 }
 
 template <typename T>
@@ -2216,7 +2214,7 @@ void launch_law_of_wall(const Geo &g, const T *U, double *utau, int *iters, int 
   template void launch_rhs_rk<T>(const Geo &, const MetT<T> &, int, bool, const T *, const T *, const T *,          \
                                  const T *, const T *, const T *, const T *, T *, T *, T *, T *, T *, T *,          \
                                  const Scalars *, double, double, const Tiles &, const RhsMaps *, const RhsMaps *,  \
-                                 const RhsMaps *, int *, int, cudaStream_t);                                        \
+                                 const RhsMaps *, const RhsMaps *, int *, int, cudaStream_t);                        \
   template void launch_project<T>(const Geo &, const MetT<T> &, const T *, const double *, const float *, T *,    \
                                   T *, T *, T *,                                                                    \
                                   const Scalars *, int, const Tiles &, cudaStream_t);                               \

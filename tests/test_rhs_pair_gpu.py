@@ -101,3 +101,31 @@ def test_packed_forms_agree_bitwise(gpu):
         s.close()
     for a, b in zip(*runs):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("grid", [(5, 4, 5), (26, 14, 11), (33, 9, 17), (34, 10, 18), (35, 17, 33), (66, 8, 20)])
+@pytest.mark.parametrize("prec", [FP64, MIXED])
+def test_les_rhs_tma_matches_global_loads(gpu, grid, prec):
+    """The LES RHS with TMA-staged planes of U, V, W and nu_t (the default)
+    against the same expressions on global loads (rhs_pts 1), at the edges of
+    its tiles (32 points and 8 rows a CTA, chunks of 16 planes): the FP64
+    values are the same bits; in FP32 the two compilations may contract sums
+    of about 60 rounded terms differently."""
+    c = noisy(*grid, seed=sum(grid) + 1)
+    rng = np.random.default_rng(sum(grid))
+    nut = np.asfortranarray(1e-3 * rng.random((c.nx + 1, c.ny + 1, c.nz + 1)))
+    got = []
+    for pts in (0, 1):
+        s = cases.solver_for(c, precision=prec, les_model=-1)  # viscosity from the host
+        s.set_nu_t(nut)
+        s.set_tiles(rhs_pts=pts)
+        got.append(s.compute_rhs(c.U, c.V, c.W))
+        s.set_dt(1e-3)
+        s.time_step()
+        got[-1] = got[-1] + s.download_state()[:3]
+        s.close()
+    for a, b in zip(*got):
+        if prec == FP64:
+            assert np.array_equal(a, b)
+        else:
+            assert np.linalg.norm(a - b) <= 1e-5 * max(np.linalg.norm(b), 1e-3)
