@@ -29,6 +29,7 @@ SOURCES = {
     "capi_mlp.cu": [],
     "zdft_tc.cu": [],
     "zdft_umma.cu": [],
+    "zsum.cu": [],
     "snapshot.cpp": [],
     "thomas_tma.cu": [],
     "cufft_path.cu": [],

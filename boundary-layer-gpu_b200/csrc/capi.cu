@@ -75,6 +75,7 @@ struct blgpu_ctx {
   Scalars *sc = nullptr;
   unsigned long long *d_maxdiv = nullptr;
   void *tw = nullptr, *post = nullptr, *ztab = nullptr;
+  float *ztab32 = nullptr;  // mixed form, M/2+1 > 96: cos and -sin tables of the FP32 products (zsum.cu)
   void *ztab64 = nullptr;  // cos and sin tables of the FP64 z transforms on the FP64 MMA
   FftPlan<double> pl64{};
   FftPlan<float> pl32{};
@@ -329,6 +330,13 @@ int blgpu_create(const blgpu_config *cfg, blgpu_ctx **out) {
     TRY(check_cuda(ctx, cudaMemcpy(ctx->utab, ut.data(), ut.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
                    "tcgen05 z-transform tables"));
     if (!zdft_umma_maps(s, (float *)ctx->R, (float2 *)ctx->C, &ctx->umaps)) ctx->utab = nullptr;
+  }
+  if (!ctx->fp64 && zsum_serves(s)) {
+    std::vector<float> zt;
+    zsum_tables(s, zt);
+    TRY(dalloc(ctx, (void **)&ctx->ztab32, zt.size() * sizeof(float)));
+    TRY(check_cuda(ctx, cudaMemcpy(ctx->ztab32, zt.data(), zt.size() * sizeof(float), cudaMemcpyHostToDevice),
+                   "z-transform tables"));
   }
   if (!ctx->fp64) {
     // the modes kx < klow of kz = 0 carry the box-scale pressure of a step's
@@ -1054,7 +1062,7 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
     cufft_path_extract_solve<T>(ctx->cf, s, ctx->post, ctx->piv, sp + s.NM, sp + 2 * s.NM, mixed ? ctx->kz0h : nullptr,
                                 ctx->klow, ctx->st);
     if (mixed) launch_kz0_idct(s, ctx->kz0h, ctx->klow, ctx->cmat, ctx->kz0, ctx->kz0g, ctx->st);
-    ph_end(ctx, mixed ? 4 : 2);
+    ph_end(ctx, mixed ? 3 : 2);
     ph_begin(ctx, PH_IDFTZ);
     r = cufft_path_inverse_z<T>(ctx->cf);
     if (r && !ctx->cf_status) ctx->cf_status = r;
@@ -1073,7 +1081,8 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
   ph_begin(ctx, PH_DIVDCT);
   launch_div_dct<T>(ctx->geo, s, pl, S[0], S[1], S[2], (T *)ctx->R, ctx->tiles.dct_nw, ctx->tiles.xfft, ctx->st);
   ph_end(ctx, 1);
-  // z transforms: tcgen05 (zdft 0 or 3), mma.sync TF32 (0 without tcgen05, or 2), FP32/FP64 sums (1)
+  // z transforms: tcgen05 (zdft 0 or 3), mma.sync TF32 (0 without tcgen05, or 2), FP32 products
+  // (M/2+1 > 96), FP32/FP64 sums (1)
   const int zd = ctx->tiles.zdft;
   const bool um = mixed && ctx->utab && (zd == 0 || zd == 3);
   const bool tc = mixed && !um && ctx->zfrag && (zd == 0 || zd == 2);
@@ -1081,6 +1090,7 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
   if (um) launch_zdft_umma(s, ctx->umaps, (float *)ctx->R, (float2 *)ctx->C, ctx->utab, 0, ctx->nsm, &ctx->sc->err, ctx->st);
   else if (tc) launch_zdft_tc(s, ctx->zmaps, (float *)ctx->R, (float2 *)ctx->C, ctx->zfrag, 0, ctx->nsm, &ctx->sc->err, ctx->st);
   else if (ctx->ztab64) launch_zdft64(s, (double *)ctx->R, (double2 *)ctx->C, (const double *)ctx->ztab64, 0, ctx->st);
+  else if (ctx->ztab32) launch_zsum(s, (float *)ctx->R, (float2 *)ctx->C, ctx->ztab32, 0, ctx->st);
   else launch_dft_z<T>(s, (T *)ctx->R, (T2 *)ctx->C, (const T2 *)ctx->ztab, 0, ctx->tiles.dftz_rk, ctx->st);
   ph_end(ctx, 1);
   const double *sp = ctx->d_spec;
@@ -1096,11 +1106,12 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
                      ctx->st);
   if (mixed)  // the box-scale pressure (kz = 0, kx < klow) in FP64
     launch_kz0_idct(s, ctx->kz0h, ctx->klow, ctx->cmat, ctx->kz0, ctx->kz0g, ctx->st);
-  ph_end(ctx, mixed ? 3 : 1);
+  ph_end(ctx, mixed ? 2 : 1);
   ph_begin(ctx, PH_IDFTZ);
   if (um) launch_zdft_umma(s, ctx->umaps, (float *)ctx->R, (float2 *)ctx->C, ctx->utab, 1, ctx->nsm, &ctx->sc->err, ctx->st);
   else if (tc) launch_zdft_tc(s, ctx->zmaps, (float *)ctx->R, (float2 *)ctx->C, ctx->zfrag, 1, ctx->nsm, &ctx->sc->err, ctx->st);
   else if (ctx->ztab64) launch_zdft64(s, (double *)ctx->R, (double2 *)ctx->C, (const double *)ctx->ztab64, 1, ctx->st);
+  else if (ctx->ztab32) launch_zsum(s, (float *)ctx->R, (float2 *)ctx->C, ctx->ztab32, 1, ctx->st);
   else launch_dft_z<T>(s, (T *)ctx->R, (T2 *)ctx->C, (const T2 *)ctx->ztab, 1, ctx->tiles.dftz_rk, ctx->st);
   ph_end(ctx, 1);
   ph_begin(ctx, PH_IDCT);

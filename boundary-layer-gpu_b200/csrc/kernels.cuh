@@ -183,6 +183,10 @@ bool zdft_tc_maps(const Spec &s, float *R, float2 *C, ZdftMaps *out);
 // flag, bit 2 set when a TMA copy did not complete within the wait limit
 void launch_zdft_tc(const Spec &s, const ZdftMaps &maps, float *R, float2 *C, const uint32_t *frag, int inverse,
                     int nsm, int *err, cudaStream_t st);
+// ---- zsum.cu: the mixed form's z transforms as FP32 products, M/2+1 > 96 ----
+bool zsum_serves(const Spec &s);  // M/2+1 > 96 and its columns fit shared memory (M up to about 770)
+void zsum_tables(const Spec &s, std::vector<float> &t);
+void launch_zsum(const Spec &s, float *R, float2 *C, const float *tab, int inverse, cudaStream_t st);
 // ---- cufft_path.cu: the cuFFT comparison path (solve_poisson_gpu with cuFFT plans) ----
 struct CufftPath;
 // plans (set to stream st) and the 2N plane / mode arrays; 0 or -1 with msg

@@ -64,3 +64,56 @@ def test_tensor_core_path_steps_close_to_fp64(gpu, form):
     A, B = a.download_state()[:3], b.download_state()[:3]
     for x, y in zip(A, B):
         assert rel(x, y) < 1e-5
+
+
+@pytest.mark.parametrize("nx,nz", [(34, 194), (71, 195), (66, 225), (35, 255), (67, 256), (130, 257), (34, 258),
+                                   (36, 259), (34, 402)])
+def test_long_z_transform_products_close_to_fp64(gpu, nx, nz):
+    """z lengths beyond the tensor-core kernels (M/2+1 = 97 .. 201, odd and
+    even M): slabs of 16 table rows (97 and 113 leave 15 padded, 128 none),
+    row tiles of 128 (128 and 129 rows), columns that end inside a 64-column
+    tile (N = 32, 69) and inside a group of four (69, 33, 65)."""
+    c = cases.laminar_case(nx=nx, ny=9, nz=nz, lx=10.0, ly=5.0, lz=8.0)
+    rng = np.random.default_rng(nz)
+    for q in "UVW":
+        a = getattr(c, q)
+        setattr(c, q, np.asfortranarray(a + 0.05 * rng.standard_normal(a.shape)))
+    c.cfl = -0.01
+    out = []
+    for prec in (MIXED, FP64):
+        s = cases.solver_for(c, precision=prec)
+        s.apply_boundary_conditions(1)
+        s.compute_projection_step(1)
+        s.apply_boundary_conditions(1)
+        out.append((s.download_state()[:3], s.rhs_p()))
+        s.close()
+    (A, pa), (B, pb) = out
+    assert rel(pa, pb) < 3e-5  # the direct sums' bar above
+    for a, b in zip(A, B):
+        assert rel(a, b) < 1e-5
+
+
+@pytest.mark.parametrize("nx,ny", [(5, 4), (64, 5), (65, 6), (66, 9), (128, 8), (129, 17), (200, 10)])
+def test_box_scale_pressure_tiles(gpu, nx, ny):
+    """The mixed form's FP64 box-scale pressure and its differences at the
+    edges of their tiles: 63 columns (N = 62, 63, 64, 126, 127), 4 rows
+    (ny-1 = 3, 4, 5, 8, 7, 16, 9) and fewer modes than 128 (N = 3): the
+    projected velocities against FP64."""
+    c = cases.laminar_case(nx=nx, ny=ny, nz=12, lx=10.0, ly=5.0, lz=4.0)
+    rng = np.random.default_rng(nx)
+    for q in "UVW":
+        a = getattr(c, q)
+        setattr(c, q, np.asfortranarray(a + 0.05 * rng.standard_normal(a.shape)))
+    c.cfl = -0.01
+    out = []
+    for prec in (MIXED, FP64):
+        s = cases.solver_for(c, precision=prec)
+        s.apply_boundary_conditions(1)
+        s.compute_projection_step(1)
+        s.apply_boundary_conditions(1)
+        out.append((s.download_state()[:3], s.rhs_p()))
+        s.close()
+    (A, pa), (B, pb) = out
+    assert rel(pa, pb) < 3e-5
+    for a, b in zip(A, B):
+        assert rel(a, b) < 1e-5
