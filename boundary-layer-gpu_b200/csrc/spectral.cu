@@ -1396,56 +1396,64 @@ __global__ void __launch_bounds__(128) k_thomas(Spec s, T2<T> *__restrict__ C, c
 // low kx, so k_thomas solves the modes kz = 0, kx < klow in FP64 into H0
 // (their forcing, the FP32 transform of the divergence, is accurate to FP32
 // relative to |div|), and
-//   k_kz0_idct: p0(i,j) = sum_{kx<klow} H0(kx,j) w_kx cos(pi kx (2i+1)/2N)/(N M)
-//               (w_0 = 1, w_kx = 2), a dense product with a cosine table;
-//   k_kz0_grad: the x and y differences of p0 taken in FP64, stored as FP32
+//   k_kz0: p0(i,j) = sum_{kx<klow} H0(kx,j) w_kx cos(pi kx (2i+1)/2N)/(N M)
+//          (w_0 = 1, w_kx = 2), a dense product with a cosine table, and the
+//          x and y differences of p0 taken in FP64, stored as FP32,
 // and the projection adds them to the differences of the FP32 part.
 // ---------------------------------------------------------------------------
-// p0[b][i] = sum_{kx < K} H[b][kx] cm[kx][i]: 32 x 64 output tiles, k-tiles of 32
-__global__ void __launch_bounds__(256) k_kz0_idct(Spec s, const double *__restrict__ H, int K,
-                                                  const double *__restrict__ cm, double *__restrict__ p0) {
-  constexpr int BM = 16, BN = 64, BK = 32;  // 16-row tiles: 208 CTAs at 812 x 256
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN];
-  const int N = s.N, NM = s.NM;
-  const int b0 = blockIdx.y * BM, i0 = blockIdx.x * BN;
-  const int t = threadIdx.x, tr = t >> 4, tc = t & 15;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    for (int q = t; q < BM * BK; q += 256) {
-      const int r = q / BK, c = q % BK;
-      As[c][r] = (b0 + r < NM && k0 + c < K) ? H[(long long)(b0 + r) * K + k0 + c] : 0.0;
-    }
-    for (int q = t; q < BK * BN; q += 256) {
-      const int r = q / BN, c = q % BN;
-      Bs[r][c] = (k0 + r < K && i0 + c < N) ? cm[(long long)(k0 + r) * N + i0 + c] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < BK; ++kk) {
-      const double a0 = As[kk][tr];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] += a0 * Bs[kk][tc + 16 * q];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int b = b0 + tr, i = i0 + tc + 16 * q;
-    if (b < NM && i < N) p0[(long long)b * N + i] = acc[q];
-  }
-}
+// p0[b][i] = sum_{kx < K} H[b][kx] cm[kx][i] and its differences in one launch.
+// A CTA forms KZ_R rows by KZ_C columns and one more row and column for the
+// differences; thread (column, group) sums the kx of its quarter, each cosine
+// read serving the KZ_R + 1 rows, and the four groups' sums are added in
+// order in shared memory.  (With 16 x 64 tiles, K in shared-memory steps and
+// the differences in a launch of their own: 18.8 + 3.2 us at N = 510, NM = 95,
+// whatever the box's size, as few CTAs ran a chain of K FP64 sums.)
+//   gx[b][i] = p0[b][min(i+1,N-1)] - p0[b][i], gy[b][i] = p0[b+1][i] - p0[b][i]
+constexpr int KZ_R = 4, KZ_C = 63, KZ_G = 4;
 
-// FP32 copies of the p0 differences the projection uses (taken in FP64):
-// gx[b][i] = p0[b][min(i+1,N-1)] - p0[b][i], gy[b][i] = p0[b+1][i] - p0[b][i]
-__global__ void k_kz0_grad(Spec s, const double *__restrict__ p0, float *__restrict__ gx, float *__restrict__ gy) {
+__global__ void __launch_bounds__(64 * KZ_G) k_kz0(Spec s, const double *__restrict__ H, int K,
+                                                   const double *__restrict__ cm, double *__restrict__ p0,
+                                                   float *__restrict__ gx, float *__restrict__ gy) {
+  __shared__ double Hs[KZ_R + 1][128];
+  __shared__ double ps[KZ_G][KZ_R + 1][64];
   const int N = s.N, NM = s.NM;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= N * NM) return;
-  const int b = q / N, i = q % N;
-  const double v = p0[q];
-  gx[q] = (float)(p0[(long long)b * N + min(i + 1, N - 1)] - v);
-  gy[q] = b < NM - 1 ? (float)(p0[q + N] - v) : 0.f;
+  const int b0 = blockIdx.y * KZ_R, i0 = blockIdx.x * KZ_C;
+  const int c = threadIdx.x, grp = threadIdx.y, t = grp * 64 + c;
+  for (int q = t; q < (KZ_R + 1) * 128; q += 64 * KZ_G) {
+    const int r = q >> 7, k = q & 127;
+    Hs[r][k] = (b0 + r < NM && k < K) ? __ldg(H + (long long)(b0 + r) * K + k) : 0.0;
+  }
+  __syncthreads();
+  const int i = min(i0 + c, N - 1);  // the column past the last repeats it: its difference is 0
+  double acc[KZ_R + 1];
+#pragma unroll
+  for (int r = 0; r <= KZ_R; ++r) acc[r] = 0.0;
+  const int kq = (K + KZ_G - 1) / KZ_G, ka = grp * kq, kb = min(ka + kq, K);
+#pragma unroll 8
+  for (int k = ka; k < kb; ++k) {
+    const double w = __ldg(cm + (long long)k * N + i);
+#pragma unroll
+    for (int r = 0; r <= KZ_R; ++r) acc[r] += Hs[r][k] * w;
+  }
+#pragma unroll
+  for (int r = 0; r <= KZ_R; ++r) ps[grp][r][c] = acc[r];
+  __syncthreads();
+  for (int r = grp; r <= KZ_R; r += KZ_G) {
+    double v = ps[0][r][c];
+#pragma unroll
+    for (int q = 1; q < KZ_G; ++q) v += ps[q][r][c];
+    ps[0][r][c] = v;
+  }
+  __syncthreads();
+  if (c < KZ_C && i0 + c < N)
+    for (int r = grp; r < KZ_R && b0 + r < NM; r += KZ_G) {
+      const int b = b0 + r;
+      const long long q = (long long)b * N + i0 + c;
+      const double v = ps[0][r][c];
+      p0[q] = v;
+      gx[q] = (float)(ps[0][r][c + 1] - v);
+      gy[q] = b < NM - 1 ? (float)(ps[0][r + 1][c] - v) : 0.f;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1644,8 +1652,8 @@ void launch_thomas_factors(const Spec &s, double *piv, const double *dd, const d
 
 void launch_kz0_idct(const Spec &s, const double *H0, int klow, const double *cm, double *p0, float *grad,
                      cudaStream_t st) {
-  k_kz0_idct<<<dim3((s.N + 63) / 64, (s.NM + 15) / 16), 256, 0, st>>>(s, H0, klow, cm, p0);
-  k_kz0_grad<<<(s.N * s.NM + 255) / 256, 256, 0, st>>>(s, p0, grad, grad + (long long)s.N * s.NM);
+  k_kz0<<<dim3((s.N + KZ_C - 1) / KZ_C, (s.NM + KZ_R - 1) / KZ_R), dim3(64, KZ_G), 0, st>>>(
+      s, H0, klow, cm, p0, grad, grad + (long long)s.N * s.NM);
 }
 
 #define BLGPU_SPEC_INST(T)                                                                                        \
