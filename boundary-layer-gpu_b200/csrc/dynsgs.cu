@@ -181,6 +181,8 @@ __device__ __forceinline__ void put_periodic(const Geo &g, T *__restrict__ nut, 
   if (gi && gk) put_rows(g, nut, gi, j, gk, v);
 }
 
+__device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // Lij, Mij and their contractions.  A warp owns 32 columns of one row j and
 // gives its 30 inner ones; it walks up k.  Per plane a lane forms the y sums
 // of the 15 filtered quantities at its own column (the centre velocities are
@@ -212,6 +214,18 @@ __global__ void __launch_bounds__(32 * DC_ROWS, 3)
   for (int q = 0; q < 15; ++q) lo[q] = mid[q] = 0.0;
   for (int kk = k0 - 1; kk <= k1 + 1; ++kk) {
     const int km = zmap(kk, g.nzg);
+    if (kk < k1) {  // row j two planes ahead (the block's other rows come from its other warps)
+      const int kn = zmap(kk + 2, g.nzg);
+      const long long b = bidx(g, ic, j, kn), c = dix(im, j, kn, g), o = dix(ic, j, kk + 1, g);
+      prefetch(U + b);
+      prefetch(V + b);
+      prefetch(W + b);
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        prefetch(SS.p[m] + c);
+        prefetch(M0.p[m] + o);
+      }
+    }
     double v[15];
     {
       double a[3], b[3], c[3];  // centre velocities at (im, rows, km): the products' entries
