@@ -243,39 +243,57 @@ __device__ __forceinline__ T2<T> *fft_warp(T2<T> *a, T2<T> *b, const FftPlan<T> 
         a[jj + (R - q) * nb] = sub<T>(y1, y2);
       }
       __syncwarp();
-      for (int t = lane; t < nb * (H + 1); t += 32) {
-        const int jj = t % nb, k = t / nb;
+      // a lane takes the outputs k = kg + KG u, u = 0..KB-1, of one butterfly:
+      // each s_q, d_q it reads serves KB table values, and the KB chains of
+      // sums are independent
+      constexpr int KB = 4;
+      const int KG = (H + KB) / KB;  // groups covering k = 0..H
+      for (int t = lane; t < nb * KG; t += 32) {
+        const int jj = t % nb, kg = t / nb;
         const int jm = jj % Ns;
         const int idxD = (jj - jm) * R + jm;
         const T2<T> y0 = a[jj];
-        T ax = y0.x, ay = y0.y;
-        if (k == 0) {
-          for (int q = 1; q <= H; ++q) {
-            const T2<T> sq = a[jj + q * nb];
-            ax += sq.x;
-            ay += sq.y;
-          }
-          b[idxD] = mk<T>(ax, ay);
-          continue;
+        T ax[KB], ay[KB], bx[KB], by[KB];  // bx, by: sums of d_q times the table's imaginary part (-sin)
+        int m[KB], dk[KB];                 // n (q k mod R) / R, and its increment
+#pragma unroll
+        for (int u = 0; u < KB; ++u) {
+          const int k = kg + KG * u;
+          ax[u] = y0.x;
+          ay[u] = y0.y;
+          bx[u] = by[u] = 0;
+          m[u] = 0;
+          dk[u] = (k <= H ? k : 0) * nb;
         }
-        T bx = 0, by = 0;  // sums of d_q times the table's imaginary part (-sin)
-        int m = 0;         // q k mod R
+        const T2<T> *as = a + jj, *ad = a + jj + (R - 1) * nb;
+#pragma unroll 2
         for (int q = 1; q <= H; ++q) {
-          m += k;
-          if (m >= R) m -= R;
-          const T2<T> w = tw[m * nb];  // W_R^m = (cos, -sin)(2 pi m / R)
-          const T2<T> sq = a[jj + q * nb], dq = a[jj + (R - q) * nb];
-          ax += sq.x * w.x;
-          ay += sq.y * w.x;
-          bx += dq.x * w.y;
-          by += dq.y * w.y;
+          as += nb;
+          const T2<T> sq = *as, dq = *ad;
+          ad -= nb;
+#pragma unroll
+          for (int u = 0; u < KB; ++u) {
+            m[u] += dk[u];
+            if (m[u] >= n) m[u] -= n;
+            const T2<T> w = tw[m[u]];  // (cos, -sin)(2 pi q k / R)
+            ax[u] += sq.x * w.x;
+            ay[u] += sq.y * w.x;
+            bx[u] += dq.x * w.y;
+            by[u] += dq.y * w.y;
+          }
         }
-        if (!INV) {
-          b[idxD + k * Ns] = mk<T>(ax - by, ay + bx);
-          b[idxD + (R - k) * Ns] = mk<T>(ax + by, ay - bx);
-        } else {
-          b[idxD + k * Ns] = mk<T>(ax + by, ay - bx);
-          b[idxD + (R - k) * Ns] = mk<T>(ax - by, ay + bx);
+#pragma unroll
+        for (int u = 0; u < KB; ++u) {
+          const int k = kg + KG * u;
+          if (k > H) continue;
+          if (k == 0) {
+            b[idxD] = mk<T>(ax[u], ay[u]);
+          } else if (!INV) {
+            b[idxD + k * Ns] = mk<T>(ax[u] - by[u], ay[u] + bx[u]);
+            b[idxD + (R - k) * Ns] = mk<T>(ax[u] + by[u], ay[u] - bx[u]);
+          } else {
+            b[idxD + k * Ns] = mk<T>(ax[u] + by[u], ay[u] - bx[u]);
+            b[idxD + (R - k) * Ns] = mk<T>(ax[u] - by[u], ay[u] + bx[u]);
+          }
         }
       }
       __syncwarp();

@@ -118,3 +118,27 @@ def test_fp64_two_pass_matches_stockham(gpu, nx, ny, nz):
         assert rel(x, y) < 1e-13
     for x, y in zip(a + (pa,), d + (pd,)):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [37, 41, 43, 74, 111, 148, 254, 259, 509])
+def test_prime_stage_outputs(gpu, n):
+    """x lengths with a prime stage above the register butterflies (37, 41,
+    43, 2 37, 3 37, 4 37, 2 127, 7 37, 509): four outputs per lane, where the
+    number of outputs per butterfly, (R+1)/2 = 19, 21, 22, 64, 255, is or is
+    not a multiple of four; FP64 against the oracle (the projection's bar),
+    mixed against FP64 at the Stockham transform's FP32 rounding."""
+    import oracle
+    c = noisy(n + 2, 6, 9, n)
+    o = oracle.oracle_for(c)
+    o.set_dt(0.01)
+    o.apply_bc(1)
+    o.projection(1)
+    ref = o.rhs_p()
+    for prec, tol in ((FP64, 1e-11), (MIXED, 1e-4)):
+        s = cases.solver_for(c, precision=prec)
+        s.apply_boundary_conditions(1)
+        s.compute_projection_step(1)
+        assert rel(s.rhs_p(), ref) < tol
+        for a, b in zip(s.download_state()[:3], o.state()[:3]):
+            assert rel(a, b) < (1e-12 if prec == FP64 else 1e-5)
+        s.close()
