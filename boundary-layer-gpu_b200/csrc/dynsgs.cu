@@ -59,8 +59,15 @@ __device__ __forceinline__ int zmap_w(int k, int nz) { return k <= 1 ? nz - 1 : 
 template <typename T> struct LdBox {
   const T *U, *V, *W;
   long long c, px, pl;  // c: box index of (i-1, j, k = 0)
+  int nz;
   __device__ LdBox(const Geo &g, const T *u, const T *v, const T *w, int i, int j, int)
-      : U(u), V(v), W(w), c(bidx(g, i - 1, j, 0)), px(g.px), pl(g.plane) {}
+      : U(u), V(v), W(w), c(bidx(g, i - 1, j, 0)), px(g.px), pl(g.plane), nz(g.nz) {}
+  __device__ __forceinline__ void pre(int k) const {
+    const long long o = c + 1 + min(k, nz) * pl;
+    prefetch_l1(U + o);
+    prefetch_l1(V + o);
+    prefetch_l1(W + o);
+  }
   __device__ __forceinline__ double at(const T *a, int s, int dj, int k) const {
     return (double)__ldg(a + c + s + dj * px + k * pl);
   }
@@ -78,6 +85,12 @@ struct LdHat {
       : U(u), V(v), W(w), j(j_), nxg(g.nxg), nz(g.nz), nzg(g.nzg), pl((long long)g.nxg * g.nyg) {
     for (int s = 0; s < 2; ++s) xu[s] = xmap(i - 1 + s, g.nx, periodic, true) - 1;
     for (int s = 0; s < 3; ++s) xc[s] = xmap(i - 1 + s, g.nxg, periodic, false) - 1;
+  }
+  __device__ __forceinline__ void pre(int k) const {  // interior planes only
+    const long long o = (min(k, nz - 1) - 1) * pl + (j - 1) * nxg;
+    prefetch_l1(U + o + xu[1]);
+    prefetch_l1(V + o + xc[1]);
+    prefetch_l1(W + o + xc[1]);
   }
   __device__ __forceinline__ double u(int s, int dj, int k) const {
     return __ldg(U + (zmap(k, nzg) - 1) * pl + (j + dj - 1) * nxg + xu[s]);
@@ -153,6 +166,7 @@ __global__ void __launch_bounds__(256) k_dyn_filter(Geo g, const T *__restrict__
   double lo = plane(k0 - 1), mid = plane(k0);
   double *__restrict__ o = q == 0 ? out.p[0] : q == 1 ? out.p[1] : out.p[2];
   for (int k = k0; k <= k1; ++k) {
+    prefetch_l1(a + oo + min(k + 3, n3) * g.plane);
     const double hi = plane(k + 1);
     o[dix(i, j, k, g)] = f141(lo, mid, hi);
     lo = mid;
@@ -180,8 +194,6 @@ __device__ __forceinline__ void put_periodic(const Geo &g, T *__restrict__ nut, 
   if (gk) put_rows(g, nut, i, j, gk, v);
   if (gi && gk) put_rows(g, nut, gi, j, gk, v);
 }
-
-__device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // Lij, Mij and their contractions.  A warp owns 32 columns of one row j and
 // gives its 30 inner ones; it walks up k.  Per plane a lane forms the y sums
@@ -217,13 +229,13 @@ __global__ void __launch_bounds__(32 * DC_ROWS, 3)
     if (kk < k1) {  // row j two planes ahead (the block's other rows come from its other warps)
       const int kn = zmap(kk + 2, g.nzg);
       const long long b = bidx(g, ic, j, kn), c = dix(im, j, kn, g), o = dix(ic, j, kk + 1, g);
-      prefetch(U + b);
-      prefetch(V + b);
-      prefetch(W + b);
+      prefetch_l1(U + b);
+      prefetch_l1(V + b);
+      prefetch_l1(W + b);
 #pragma unroll
       for (int m = 0; m < 6; ++m) {
-        prefetch(SS.p[m] + c);
-        prefetch(M0.p[m] + o);
+        prefetch_l1(SS.p[m] + c);
+        prefetch_l1(M0.p[m] + o);
       }
     }
     double v[15];

@@ -1841,6 +1841,13 @@ __global__ void __launch_bounds__(256) k_maxdiv(Geo g, const T *__restrict__ U, 
 template <typename T> struct LdT {
   const T *U, *V, *W;
   long long c, px, pl;  // c: box index of (i-1, j, k = 0)
+  int nz;
+  __device__ __forceinline__ void pre(int k) const {
+    const long long o = c + 1 + min(k, nz) * pl;
+    prefetch_l1(U + o);
+    prefetch_l1(V + o);
+    prefetch_l1(W + o);
+  }
   __device__ __forceinline__ T at(const T *a, int s, int dj, int k) const { return __ldg(a + c + s + dj * px + k * pl); }
   __device__ __forceinline__ T u(int s, int dj, int k) const { return at(U, s, dj, k); }
   __device__ __forceinline__ T v(int s, int dj, int k) const { return at(V, s, dj, k); }
@@ -1855,7 +1862,7 @@ __global__ void __launch_bounds__(256) k_smagorinsky(Geo g, MetT<T> m, const T *
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
   if (i > g.nxg - 1 || j > g.nyg - 1) return;
   const int k0 = 2 + blockIdx.z * kchunk, k1 = min(k0 + kchunk - 1, g.nzg - 1);
-  const LdT<T> ld{U, V, W, bidx(g, i - 1, j, 0), g.px, g.plane};
+  const LdT<T> ld{U, V, W, bidx(g, i - 1, j, 0), g.px, g.plane, g.nz};
   StrainColumn<T, LdT<T>> col(ld, m.xF, m.xrF, m.xC, m.xrC, m.yF, m.yrF, m.yC, m.yrC, m.zF, m.zrF, m.zC, m.zrC, i, j);
   const T c2 = (T)cs2[j];
   col.start(k0);
