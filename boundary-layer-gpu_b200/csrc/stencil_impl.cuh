@@ -1975,6 +1975,17 @@ __global__ void __launch_bounds__(256) k_law_of_wall(Geo g, const T *__restrict_
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+// Built-in chunk of k-planes of an RHS kernel whose CTAs cover `tiles` x-y
+// tiles: kc, halved while the grid would hold fewer than 200 CTAs.  A chunk's
+// two extra planes cost little next to SMs without a CTA: per launch at
+// 128 x 64 x 32 (16 x-y tiles) 20.8 us with 16 planes, 10.6 with 2 (mixed),
+// 31.7 and 14.7 (FP64); at 256 x 65 x 96 (32 tiles, 192 CTAs) 8 and 16 planes
+// tie (26.9, 26.7), and at 301 x 98 x 75 (65 tiles) shorter chunks lose.
+static inline int rhs_chunk(int kc, int tiles, int nk) {
+  while (kc > 1 && tiles * ((nk + kc - 1) / kc) < 200) kc /= 2;
+  return kc;
+}
+
 static inline dim3 vol_grid(int ni, int nj, int nk, int kchunk, int by = 8) {
   return dim3((ni + 31) / 32, (nj + by - 1) / by, (nk + kchunk - 1) / kchunk);
 }
@@ -2049,8 +2060,13 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
                    const T *nut, const T *Uo, const T *Vo, const T *Wo, T *F1u, T *F1v, T *F1w, T *Un, T *Vn, T *Wn,
                    const Scalars *sc, double c1, double c2, const Tiles &tl, const RhsMaps *mi, const RhsMaps *mo,
                    const RhsMaps *mf, const RhsMaps *mn, int *err, int wait_limit, cudaStream_t st) {
-  const int kchunk = tl.rhs_kc > 0 ? tl.rhs_kc : 8;
   const int by = tl.rhs_by > 0 ? tl.rhs_by : 8;
+  // chunk for kernels of 32 threads x rows with pts points per thread
+  auto chunk = [&](int kc, int pts, int rows) {
+    const int nx = pts == 2 ? g.nx / 2 : g.nx - 1;
+    return tl.rhs_kc > 0 ? tl.rhs_kc : rhs_chunk(kc, (nx + 31) / 32 * ((g.ny - 1 + rows - 1) / rows), g.nz - 1);
+  };
+  const int kchunk = chunk(8, 1, by);
   dim3 grid = vol_grid(g.nx - 1, g.ny - 1, g.nz - 1, kchunk, by), block(32, by);
 #define BLGPU_RHS_CASE(M, L)                                                                             \
   k_rhs_rk<T, M, L><<<grid, block, 0, st>>>(g, m, U, V, W, nut, Uo, Vo, Wo, F1u, F1v, F1w, Un, Vn, Wn, sc, c1, \
@@ -2067,7 +2083,7 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
     // the TMA-fed kernel serves the default where its maps exist (16 planes
     // per CTA: the two extra planes a chunk reads cost 1/8 of its loads)
     const bool tma_fed = (tl.rhs_pts == 4 || tl.rhs_pts == 0) && mi && mo && mf;
-    const int kc = tl.rhs_kc > 0 ? tl.rhs_kc : (tma_fed ? 16 : pair ? 8 : 32);
+    const int kc = tma_fed ? chunk(16, 2, RT_BY) : pair ? chunk(8, 2, by) : chunk(32, 1, by);
     // pairs cover i = 2..nx two points at a time
     dim3 gd = vol_grid(pair ? g.nx / 2 : g.nx - 1, g.ny - 1, g.nz - 1, kc, by);
 #define BLGPU_DNS_CASE(M)                                                                                           \
@@ -2102,7 +2118,7 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
       // k_rhs_rk: its shared and carried terms are the same expressions), the
       // TMA-fed one-point kernel (rhs_pts 4) or the global-load kernel (1)
       if (tl.rhs_pts == 2 || tl.rhs_pts == 0) {
-        const int kc = tl.rhs_kc > 0 ? tl.rhs_kc : 16;
+        const int kc = chunk(16, 2, 8);
         dim3 gd = vol_grid(g.nx / 2, g.ny - 1, g.nz - 1, kc, 8);
         dim3 blk(32, 8);
         switch (mode) {
@@ -2114,7 +2130,7 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
         return;
       }
       if (tl.rhs_pts == 4 && mi && mo && mf) {
-        const int kc = tl.rhs_kc > 0 ? tl.rhs_kc : 32;
+        const int kc = chunk(32, 1, R64_BY);
         BLGPU_TMA1_CASE(false, kc, *mi);
         return;
       }
@@ -2126,7 +2142,8 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
       default: BLGPU_RHS_CASE(3, false); break;
     }
   } else if (tl.rhs_pts != 1 && mi && mo && mf && mn) {
-    BLGPU_TMA1_CASE(true, tl.rhs_kc > 0 ? tl.rhs_kc : 16, *mn);
+    const int kc = chunk(16, 1, R64_BY);
+    BLGPU_TMA1_CASE(true, kc, *mn);
   } else {
     switch (mode) {
       case 0: BLGPU_RHS_CASE(0, true); break;
