@@ -17,6 +17,9 @@
 //               rhs_p in the box layout together with the x-Neumann and
 //               z-periodic copies of apply_periodic_z_pressure
 //               (projection.f90:295-303).
+#include <algorithm>
+#include <cstdlib>
+
 #include "kernels.cuh"
 #include "divergence.cuh"
 #include "tma.cuh"
@@ -210,11 +213,25 @@ __device__ __forceinline__ bool reg_radix(int R) {
   return R == 5 || R == 7 || R == 11 || R == 13 || R == 17 || R == 19 || R == 23 || R == 29 || R == 31;
 }
 
-// warp-level Stockham FFT of one complex line in shared memory (no block
-// barriers: each warp owns its line, stages are separated by __syncwarp)
-template <typename T, bool INV, int MAXR>
-__device__ __forceinline__ T2<T> *fft_warp(T2<T> *a, T2<T> *b, const FftPlan<T> &pl, const T2<T> *tw, int lane) {
-  const int n = pl.n;
+// The lanes that share one complex line: one warp, or several that meet at a
+// named barrier.  Shared memory holds two buffers per line (16 KB at N = 1022
+// in FP32, 32 KB in FP64), so a box of long lines keeps 4 to 13 of them per SM
+// and one warp each leaves the SM idle between dependent loads.
+template <bool GROUP> struct LineGroup {
+  int lane, lanes, bar;  // lane of 32 w, named barrier of the line (w > 1)
+  __device__ __forceinline__ int nl() const { return GROUP ? lanes : 32; }
+  __device__ __forceinline__ void sync() const {
+    if (GROUP) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(lanes) : "memory");
+    else __syncwarp();
+  }
+};
+
+// Stockham FFT of one complex line in shared memory by its lane group (no
+// block barriers: stages are separated by the group's)
+template <typename T, bool INV, int MAXR, bool GROUP>
+__device__ __forceinline__ T2<T> *fft_line(T2<T> *a, T2<T> *b, const FftPlan<T> &pl, const T2<T> *tw,
+                                           const LineGroup<GROUP> &lg) {
+  const int n = pl.n, lane = lg.lane, nl = lg.nl();
   int Ns = 1;
   for (int s = 0; s < pl.nst; ++s) {
     const int R = pl.rad[s];
@@ -231,7 +248,7 @@ __device__ __forceinline__ T2<T> *fft_warp(T2<T> *a, T2<T> *b, const FftPlan<T> 
       // (signs swapped for the inverse): H terms for two outputs instead of
       // R terms for one.
       const int H = (R - 1) / 2;
-      for (int t = lane; t < nb * H; t += 32) {
+      for (int t = lane; t < nb * H; t += nl) {
         const int jj = t % nb, q = 1 + t / nb;
         const int tstep = (jj % Ns) * tsc;
         T2<T> y1 = a[jj + q * nb], y2 = a[jj + (R - q) * nb];
@@ -242,13 +259,13 @@ __device__ __forceinline__ T2<T> *fft_warp(T2<T> *a, T2<T> *b, const FftPlan<T> 
         a[jj + q * nb] = add<T>(y1, y2);
         a[jj + (R - q) * nb] = sub<T>(y1, y2);
       }
-      __syncwarp();
+      lg.sync();
       // a lane takes the outputs k = kg + KG u, u = 0..KB-1, of one butterfly:
       // each s_q, d_q it reads serves KB table values, and the KB chains of
       // sums are independent
       constexpr int KB = 4;
       const int KG = (H + KB) / KB;  // groups covering k = 0..H
-      for (int t = lane; t < nb * KG; t += 32) {
+      for (int t = lane; t < nb * KG; t += nl) {
         const int jj = t % nb, kg = t / nb;
         const int jm = jj % Ns;
         const int idxD = (jj - jm) * R + jm;
@@ -296,14 +313,14 @@ __device__ __forceinline__ T2<T> *fft_warp(T2<T> *a, T2<T> *b, const FftPlan<T> 
           }
         }
       }
-      __syncwarp();
+      lg.sync();
       T2<T> *t = a;
       a = b;
       b = t;
       Ns *= R;
       continue;
     }
-    for (int jj = lane; jj < nb; jj += 32) {
+    for (int jj = lane; jj < nb; jj += nl) {
       const int jm = jj % Ns;
       const int tstep = jm * tsc;
       const int idxD = (jj - jm) * R + jm;
@@ -320,7 +337,7 @@ __device__ __forceinline__ T2<T> *fft_warp(T2<T> *a, T2<T> *b, const FftPlan<T> 
       else if (MAXR >= 29 && R == 29) bf_odd<29, T, INV>(a, b, jj, nb, tstep, idxD, Ns, n, tw);
       else if (MAXR >= 31 && R == 31) bf_odd<31, T, INV>(a, b, jj, nb, tstep, idxD, Ns, n, tw);
     }
-    __syncwarp();
+    lg.sync();
     T2<T> *t = a;
     a = b;
     b = t;
@@ -458,7 +475,8 @@ __device__ __forceinline__ void dft_reg(V (&x)[R]) {
 // FFT engines of the x transforms: the shared-memory twiddle table, the
 // per-line buffer and the transform of one line by one warp (result in
 // natural order).  Stockham: any N, ping-pong buffers of N values.
-template <typename T, int MAXR> struct StockhamX {
+template <typename T, int MAXR, bool GROUP = false> struct StockhamX {
+  static constexpr bool grouped = GROUP;  // several warps per line
   static constexpr int max_threads = sizeof(T) == 4 ? 512 : 256, min_blocks = 0;  // 16 or 8 lines, no bound
   static size_t line(int N) { return 2 * (size_t)N; }
   __device__ static size_t dline(int N) { return 2 * (size_t)N; }
@@ -466,14 +484,15 @@ template <typename T, int MAXR> struct StockhamX {
     for (int t = tid; t < pl.n; t += nt) tw[t] = pl.tw[t];
   }
   template <bool INV>
-  __device__ static T2<T> *run(T2<T> *buf, const FftPlan<T> &pl, const T2<T> *tw, int lane) {
-    return fft_warp<T, INV, MAXR>(buf, buf + pl.n, pl, tw, lane);
+  __device__ static T2<T> *run(T2<T> *buf, const FftPlan<T> &pl, const T2<T> *tw, const LineGroup<GROUP> &lg) {
+    return fft_line<T, INV, MAXR, GROUP>(buf, buf + pl.n, pl, tw, lg);
   }
 };
 
 // Two-pass: N = A B (A, B <= 32), one buffer of max(N, A (B | 1)) values;
 // the table holds W_N^{n2 k1} at [k1][n2] (row pitch B)
 template <int A, int B, typename T = float> struct TwoPassX {
+  static constexpr bool grouped = false;
   // LINE even keeps every line buffer 16-byte aligned
   static constexpr int N = A * B, SB = B | 1, LINE = ((N > A * SB ? N : A * SB) + 1) & ~1;
   static_assert(A <= 32 && B <= 32, "one lane per butterfly");
@@ -490,7 +509,8 @@ template <int A, int B, typename T = float> struct TwoPassX {
     }
   }
   template <bool INV>
-  __device__ static T2<T> *run(T2<T> *buf, const FftPlan<T> &, const T2<T> *tw, int lane) {
+  __device__ static T2<T> *run(T2<T> *buf, const FftPlan<T> &, const T2<T> *tw, const LineGroup<false> &lg) {
+    const int lane = lg.lane;
     {
       T2<T> x[A];
       if (lane < B) {
@@ -532,11 +552,13 @@ template <int A, int B, typename T = float> struct TwoPassX {
 // buffer in the DCT's reordered positions (point i at i/2 when even, at
 // N-1-i/2 when odd), FP32, four consecutive points per lane with 16-byte
 // loads (the box rows start 16-byte aligned at i = 2); U at i-1 of the first
-// point comes from the previous lane, or from the previous round for lane 0.
+// point comes from the previous lane, for lane 0 from the previous round.
 // rfx: the FP32 reciprocal x spacings of the points, N rounded up to 4.
+template <bool GROUP>
 __device__ __forceinline__ void div_pair_vec(const Geo &g, const Spec &s, const float *__restrict__ U,
                                              const float *__restrict__ V, const float *__restrict__ W,
-                                             const float *rfx, float2 *bufA, int q, int lane) {
+                                             const float *rfx, float2 *bufA, int q, const LineGroup<GROUP> &lg) {
+  const int lane = lg.lane & 31;
   const int N = s.N, N4 = (N + 3) & ~3;
   const int nlines = s.NM * s.M;
   const bool hb = q + 1 < nlines;
@@ -548,8 +570,19 @@ __device__ __forceinline__ void div_pair_vec(const Geo &g, const Spec &s, const 
   const int jb = hb ? bb + 2 : ba + 2, kbb = hb ? kb + 2 : ka + 2;
   const float ryA = (float)g.ay.rF[ba + 2], rzA = (float)g.az.rF[ka + 2];
   const float ryB = (float)g.ay.rF[jb], rzB = (float)g.az.rF[kbb];
-  float carA = __ldg(U + ca - 1), carB = __ldg(U + cbb - 1);
-  for (int base = 0; base < N; base += 128) {
+  // each warp of the group takes every (nl/32)-th round of 128 points; a warp
+  // alone carries U at the last point of a round to the next one (a load for
+  // it costs 8 % of the forward transform at N = 812)
+  float carA = 0.f, carB = 0.f;
+  if (!GROUP) {
+    carA = __ldg(U + ca - 1);
+    carB = __ldg(U + cbb - 1);
+  }
+  for (int base = GROUP ? 4 * (lg.lane & ~31) : 0; base < N; base += 4 * lg.nl()) {
+    if (GROUP) {
+      carA = __ldg(U + ca + base - 1);
+      carB = __ldg(U + cbb + base - 1);
+    }
     const int i4 = base + 4 * lane, ic = i4 < N4 ? i4 : N4 - 4;  // in-row address for idle lanes
     const float4 rx = *reinterpret_cast<const float4 *>(rfx + ic);
     float fa[4], fb[4];
@@ -562,11 +595,12 @@ __device__ __forceinline__ void div_pair_vec(const Geo &g, const Spec &s, const 
       const float4 w = __ldg(reinterpret_cast<const float4 *>(W + c));
       const float4 wm = __ldg(reinterpret_cast<const float4 *>(W + c - g.plane));
       float um0 = __shfl_up_sync(0xffffffffu, u.w, 1);
-      const float car = l ? carB : carA;
-      if (lane == 0) um0 = car;
-      const float nc = __shfl_sync(0xffffffffu, u.w, 31);
-      if (l) carB = nc;
-      else carA = nc;
+      if (lane == 0) um0 = l ? carB : carA;
+      if (!GROUP) {
+        const float nc = __shfl_sync(0xffffffffu, u.w, 31);
+        if (l) carB = nc;
+        else carA = nc;
+      }
       const float ry = l ? ryB : ryA, rz = l ? rzB : rzA;
       float *f = l ? fb : fa;
       // projection.f90:42-44, as div_at
@@ -597,11 +631,11 @@ __device__ __forceinline__ void div_pair_vec(const Geo &g, const Spec &s, const 
 
 // The DCT coefficients of the two lines from their packed transform res:
 // V_A = (Z_k + conj Z_{N-k})/2, V_B = (Z_k - conj Z_{N-k})/(2i), c = Re(e^{-i pi k/2N} V)
-template <typename T>
+template <typename T, bool GROUP>
 __device__ __forceinline__ void dct_pair_out(const T2<T> *res, const T2<T> *post, T *ra, int rx, int N, bool hb,
-                                             int lane) {
+                                             const LineGroup<GROUP> &lg) {
   T *rb = ra + rx;
-  for (int k = lane; k < N; k += 32) {
+  for (int k = lg.lane; k < N; k += lg.nl()) {
     const T2<T> z = res[k];
     const T2<T> zr = res[k == 0 ? 0 : N - k];
     const T2<T> p = post[k];
@@ -619,13 +653,15 @@ template <typename T> struct DctCta { static constexpr int max_threads = sizeof(
 template <typename T, class E>
 __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_div_dct(Geo g, Spec s, FftPlan<T> pl, const T *__restrict__ U,
                                                  const T *__restrict__ V, const T *__restrict__ W,
-                                                 T *__restrict__ R) {
+                                                 T *__restrict__ R, int wpl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int N = s.N;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int nl = E::grouped ? 32 * wpl : 32;
+  const int line = threadIdx.x / nl, nw = blockDim.x / nl;  // the line of this CTA, lines per CTA
+  const LineGroup<E::grouped> lg{(int)threadIdx.x % nl, nl, 1 + line};
   T2<T> *tw = reinterpret_cast<T2<T> *>(smem_raw);
   T2<T> *post = tw + N;
-  T2<T> *bufA = post + N + (size_t)warp * E::dline(N);
+  T2<T> *bufA = post + N + (size_t)line * E::dline(N);
   // FP32: the reciprocal x spacings of the points, N rounded up to 4
   const int N4 = (N + 3) & ~3;
   float *rfx = reinterpret_cast<float *>(post + N + (size_t)nw * E::dline(N));
@@ -635,7 +671,7 @@ __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_div_dct(Geo g
     for (int t = threadIdx.x; t < N4; t += blockDim.x) rfx[t] = t < N ? (float)g.ax.rF[t + 2] : 0.f;
   __syncthreads();
   const int nlines = s.NM * s.M;
-  const int q = (blockIdx.x * nw + warp) * 2;
+  const int q = (blockIdx.x * nw + line) * 2;
   if (q >= nlines) return;
   const bool hb = q + 1 < nlines;
   const int ba = q / s.M, ka = q - ba * s.M;
@@ -648,10 +684,11 @@ __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_div_dct(Geo g
                    ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(W)) &
                     15) == 0 && (g.px & 3) == 0;
   if constexpr (sizeof(T) == 4) {
-    if (vec) div_pair_vec(g, s, U, V, W, rfx, bufA, q, lane);
+    if (vec) div_pair_vec(g, s, U, V, W, rfx, bufA, q, lg);
   }
   // batches of 4 points per lane: all 48 loads issued before any use
-  for (int base = 0; base < N && !vec; base += 128) {
+  const int lane = lg.lane & 31;
+  for (int base = 4 * (lg.lane & ~31); base < N && !vec; base += 4 * nl) {
     T fa[4], fb[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -669,9 +706,9 @@ __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_div_dct(Geo g
       }
     }
   }
-  __syncwarp();
-  const T2<T> *res = E::template run<false>(bufA, pl, tw, lane);
-  dct_pair_out<T>(res, post, R + (long long)q * s.rx, s.rx, N, hb, lane);
+  lg.sync();
+  const T2<T> *res = E::template run<false>(bufA, pl, tw, lg);
+  dct_pair_out<T>(res, post, R + (long long)q * s.rx, s.rx, N, hb, lg);
 }
 
 // ---------------------------------------------------------------------------
@@ -681,23 +718,25 @@ __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_div_dct(Geo g
 // ---------------------------------------------------------------------------
 template <typename T, class E>
 __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_idct(Geo g, Spec s, FftPlan<T> pl, const T *__restrict__ R,
-                                              T *__restrict__ p) {
+                                              T *__restrict__ p, int wpl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int N = s.N;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int nl = E::grouped ? 32 * wpl : 32;
+  const int line = threadIdx.x / nl, nw = blockDim.x / nl;  // the line of this CTA, lines per CTA
+  const LineGroup<E::grouped> lg{(int)threadIdx.x % nl, nl, 1 + line};
   T2<T> *tw = reinterpret_cast<T2<T> *>(smem_raw);
   T2<T> *post = tw + N;
-  T2<T> *bufA = post + N + (size_t)warp * E::dline(N);
+  T2<T> *bufA = post + N + (size_t)line * E::dline(N);
   E::fill(tw, pl, threadIdx.x, blockDim.x);
   for (int t = threadIdx.x; t < N; t += blockDim.x) post[t] = pl.post[t];
   __syncthreads();
   const int nlines = s.NM * s.M;
-  const int q = (blockIdx.x * nw + warp) * 2;
+  const int q = (blockIdx.x * nw + line) * 2;
   if (q >= nlines) return;
   const bool hb = q + 1 < nlines;
   const T *ra = R + (long long)q * s.rx;
   const T *rb = ra + s.rx;
-  for (int k = lane; k < N; k += 32) {
+  for (int k = lg.lane; k < N; k += nl) {
     const T xa = ra[k], xan = k ? ra[N - k] : (T)0;
     const T xb = hb ? rb[k] : (T)0, xbn = (hb && k) ? rb[N - k] : (T)0;
     // V_k = exp(+i pi k/2N) (X_k - i X_{N-k});  Z = V_A + i V_B
@@ -706,14 +745,14 @@ __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_idct(Geo g, S
     const T2<T> vb = cmul<T>(e, mk<T>(xb, -xbn));
     bufA[k] = mk<T>(va.x - vb.y, va.y + vb.x);
   }
-  __syncwarp();
-  const T2<T> *res = E::template run<true>(bufA, pl, tw, lane);
+  lg.sync();
+  const T2<T> *res = E::template run<true>(bufA, pl, tw, lg);
   const T inv = (T)1 / (T)N;
   const int ba = q / s.M, ka = q - ba * s.M;
   const int bb = hb ? (q + 1) / s.M : ba, kb = hb ? (q + 1) - bb * s.M : ka;
   const long long ca = bidx(g, 2, ba + 2, ka + 2), cb = bidx(g, 2, bb + 2, kb + 2);
   const long long zsh = (long long)s.M * g.plane;  // k = 2 -> k = nzp+2
-  for (int ip = lane; ip < N; ip += 32) {
+  for (int ip = lg.lane; ip < N; ip += nl) {
     const int pos = (ip & 1) ? (N - 1 - (ip >> 1)) : (ip >> 1);
     const T2<T> z = res[pos];
     const T va = z.x * inv, vb = z.y * inv;
@@ -1539,55 +1578,112 @@ static int radix_class(const int *rad, int nst) {
   return 31;
 }
 
-template <typename T, class E>
-static void launch_div_dct_e(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *U, const T *V, const T *W,
-                             T *R, int nw, size_t sm, int grid, cudaStream_t st) {
-  cudaFuncSetAttribute(k_div_dct<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  cudaFuncSetAttribute(k_div_dct<T, E>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  k_div_dct<T, E><<<grid, 32 * nw, sm, st>>>(g, s, pl, U, V, W, R);
+// launch shape of an x-transform kernel: lines per CTA, warps per line,
+// shared memory and grid
+struct XShape {
+  int nw, wpl;
+  size_t sm;
+  int grid;
+};
+
+// Lines per CTA and warps per line.  Several warps share a line of the
+// Stockham kernels where a prime stage above the register butterflies makes
+// its work (items of independent sums) and long lines leave few of them on an
+// SM; lengths without one lose by it (the register butterflies number n/R, and
+// every stage meets at a barrier: N = 385 0.069 -> 0.084, 299 0.037 -> 0.042 ms
+// with two warps), and below N = 400 one warp per line fills the SM.  ms per
+// launch, forward / inverse, one warp -> this shape:
+//   N = 1022 (2 7 73), 1024 x 129 x 128   mixed 0.333 / 0.226 -> 0.225 / 0.226, FP64 0.970 / 0.574 -> 0.452 / 0.353
+//   N =  887 (prime),   889 x 65 x 130    mixed 0.692 / 0.608 -> 0.541 / 0.539, FP64 2.08 / 1.88 -> 1.03 / 0.98
+//   N =  698 (2 349),   700 x 65 x 130    mixed 0.229 / 0.182 -> 0.183 / 0.185, FP64 0.403 / 0.318 -> 0.343 / 0.296
+//   N =  555 (3 5 37),  557 x 129 x 128   mixed 0.120 / 0.097 -> 0.108 / 0.091, FP64 0.256 / 0.152 -> 0.207 / 0.146
+//   N =  453 (3 151),   455 x 97 x 128    mixed 0.112 / 0.101 -> 0.099 / 0.086, FP64 0.225 / 0.164 -> 0.199 / 0.164
+template <typename T>
+static XShape x_shape(const Spec &s, const FftPlan<T> &pl, int nw_req, int split, bool inverse) {
+  int rmax = 0;
+  for (int q = 0; q < pl.nst; ++q) rmax = std::max(rmax, pl.rad[q]);
+  XShape x;
+  x.nw = nw_req > 0 ? nw_req : dct_lines_per_cta(s.N, sizeof(T), inverse, split);
+  x.wpl = 1;
+  if (!split && nw_req <= 0 && rmax > 31 && s.N >= 400) {
+    if (s.N >= 600) {  // two CTAs per SM need half its shared memory
+      x.nw = dct_smem_bytes(s.N, sizeof(T), 2, 0) <= 113 * 1024 ? 2 : 1;
+      x.wpl = 4;
+    } else if (sizeof(T) == 4) {
+      x.nw = inverse ? 6 : 4;
+      x.wpl = inverse ? 1 : 2;
+    } else {
+      x.nw = inverse ? 4 : 2;
+      x.wpl = 2;
+    }
+  }
+  x.sm = dct_smem_bytes(s.N, sizeof(T), x.nw, split);
+  x.grid = ((s.NM * s.M + 1) / 2 + x.nw - 1) / x.nw;
+  return x;
 }
 
 template <typename T, class E>
-static void launch_idct_e(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *R, T *p, int nw, size_t sm,
-                          int grid, cudaStream_t st) {
-  cudaFuncSetAttribute(k_idct<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  cudaFuncSetAttribute(k_idct<T, E>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  k_idct<T, E><<<grid, 32 * nw, sm, st>>>(g, s, pl, R, p);
+static void launch_div_dct_e(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *U, const T *V, const T *W,
+                             T *R, XShape x, cudaStream_t st) {
+  cudaFuncSetAttribute(k_div_dct<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x.sm);
+  cudaFuncSetAttribute(k_div_dct<T, E>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  k_div_dct<T, E><<<x.grid, 32 * x.nw * x.wpl, x.sm, st>>>(g, s, pl, U, V, W, R, x.wpl);
 }
+
+template <typename T, class E>
+static void launch_idct_e(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *R, T *p, XShape x,
+                          cudaStream_t st) {
+  cudaFuncSetAttribute(k_idct<T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x.sm);
+  cudaFuncSetAttribute(k_idct<T, E>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  k_idct<T, E><<<x.grid, 32 * x.nw * x.wpl, x.sm, st>>>(g, s, pl, R, p, x.wpl);
+}
+
+// the Stockham kernel of the plan's radix class, several warps per line or one
+#define BLGPU_STOCKHAM(CALL)                                                         \
+  do {                                                                               \
+    if (x.wpl > 1) switch (radix_class(pl.rad, pl.nst)) {                            \
+        case 7: CALL(StockhamX<T BLGPU_C 7 BLGPU_C true>); break;                    \
+        case 13: CALL(StockhamX<T BLGPU_C 13 BLGPU_C true>); break;                  \
+        case 19: CALL(StockhamX<T BLGPU_C 19 BLGPU_C true>); break;                  \
+        case 29: CALL(StockhamX<T BLGPU_C 29 BLGPU_C true>); break;                  \
+        default: CALL(StockhamX<T BLGPU_C 31 BLGPU_C true>); break;                  \
+      }                                                                              \
+    else switch (radix_class(pl.rad, pl.nst)) {                                      \
+        case 7: CALL(StockhamX<T BLGPU_C 7>); break;                                 \
+        case 13: CALL(StockhamX<T BLGPU_C 13>); break;                               \
+        case 19: CALL(StockhamX<T BLGPU_C 19>); break;                               \
+        case 29: CALL(StockhamX<T BLGPU_C 29>); break;                               \
+        default: CALL(StockhamX<T BLGPU_C 31>); break;                               \
+      }                                                                              \
+  } while (0)
+#define BLGPU_C ,
 
 template <typename T>
 void launch_div_dct(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *U, const T *V, const T *W, T *R,
                     int nw_req, int xfft, cudaStream_t st) {
   int split = xfft != 1 ? xfft_split(s.N) : 0;
   if (sizeof(T) == 8 && split != 29) split = 0;  // FP64 two-pass built for N = 812 only
-  const int nw = nw_req > 0 ? nw_req : dct_lines_per_cta(s.N, sizeof(T), false, split);
-  const size_t sm = dct_smem_bytes(s.N, sizeof(T), nw, split);
-  const int ncl = (s.NM * s.M + 1) / 2;  // complex lines
-  const int grid = (ncl + nw - 1) / nw;
+  const XShape x = x_shape<T>(s, pl, nw_req, split, false);
   if constexpr (sizeof(T) == 8) {
-    if (split == 29) return launch_div_dct_e<T, TwoPassX<29, 28, T>>(g, s, pl, U, V, W, R, nw, sm, grid, st);
+    if (split == 29) return launch_div_dct_e<T, TwoPassX<29, 28, T>>(g, s, pl, U, V, W, R, x, st);
   }
   if constexpr (sizeof(T) == 4) {
-    if (split == 29) return launch_div_dct_e<T, TwoPassX<29, 28>>(g, s, pl, U, V, W, R, nw, sm, grid, st);
-    if (split == 17) return launch_div_dct_e<T, TwoPassX<17, 30>>(g, s, pl, U, V, W, R, nw, sm, grid, st);
-    if (split == 19) return launch_div_dct_e<T, TwoPassX<19, 10>>(g, s, pl, U, V, W, R, nw, sm, grid, st);
-    if (split == 14) return launch_div_dct_e<T, TwoPassX<14, 9>>(g, s, pl, U, V, W, R, nw, sm, grid, st);
+    if (split == 29) return launch_div_dct_e<T, TwoPassX<29, 28>>(g, s, pl, U, V, W, R, x, st);
+    if (split == 17) return launch_div_dct_e<T, TwoPassX<17, 30>>(g, s, pl, U, V, W, R, x, st);
+    if (split == 19) return launch_div_dct_e<T, TwoPassX<19, 10>>(g, s, pl, U, V, W, R, x, st);
+    if (split == 14) return launch_div_dct_e<T, TwoPassX<14, 9>>(g, s, pl, U, V, W, R, x, st);
   }
-  switch (radix_class(pl.rad, pl.nst)) {
-    case 7: launch_div_dct_e<T, StockhamX<T, 7>>(g, s, pl, U, V, W, R, nw, sm, grid, st); break;
-    case 13: launch_div_dct_e<T, StockhamX<T, 13>>(g, s, pl, U, V, W, R, nw, sm, grid, st); break;
-    case 19: launch_div_dct_e<T, StockhamX<T, 19>>(g, s, pl, U, V, W, R, nw, sm, grid, st); break;
-    case 29: launch_div_dct_e<T, StockhamX<T, 29>>(g, s, pl, U, V, W, R, nw, sm, grid, st); break;
-    default: launch_div_dct_e<T, StockhamX<T, 31>>(g, s, pl, U, V, W, R, nw, sm, grid, st); break;
-  }
+#define BLGPU_FWD(...) launch_div_dct_e<T, __VA_ARGS__>(g, s, pl, U, V, W, R, x, st)
+  BLGPU_STOCKHAM(BLGPU_FWD);
+#undef BLGPU_FWD
 }
 
 template <int A, int B, typename T>
-static void launch_idct2(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *R, T *p, int nw, size_t sm,
-                         int grid, int *err, cudaStream_t st) {
-  cudaFuncSetAttribute(k_idct2<A, B, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+static void launch_idct2(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *R, T *p, XShape x, int *err,
+                         cudaStream_t st) {
+  cudaFuncSetAttribute(k_idct2<A, B, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x.sm);
   cudaFuncSetAttribute(k_idct2<A, B, T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  k_idct2<A, B, T><<<grid, 32 * nw, sm, st>>>(g, s, pl, R, p, err);
+  k_idct2<A, B, T><<<x.grid, 32 * x.nw, x.sm, st>>>(g, s, pl, R, p, err);
 }
 
 // the two rows of the bulk copy fit one line buffer of the two-pass kernel
@@ -1600,33 +1696,28 @@ void launch_idct(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *R, 
                  cudaStream_t st) {
   int split = xfft != 1 ? xfft_split(s.N) : 0;
   if (sizeof(T) == 8 && split != 29) split = 0;  // FP64 two-pass built for N = 812 only
-  const int nw = nw_req > 0 ? nw_req : dct_lines_per_cta(s.N, sizeof(T), true, split);
-  const size_t sm = dct_smem_bytes(s.N, sizeof(T), nw, split);
-  const int ncl = (s.NM * s.M + 1) / 2;
-  const int grid = (ncl + nw - 1) / nw;
+  const XShape x = x_shape<T>(s, pl, nw_req, split, true);
   const bool fused = idct2_fits(s, split) && (reinterpret_cast<uintptr_t>(R) & 15) == 0;
   if constexpr (sizeof(T) == 8) {
-    if (split == 29 && fused) return launch_idct2<29, 28, T>(g, s, pl, R, p, nw, sm, grid, err, st);
-    if (split == 29) return launch_idct_e<T, TwoPassX<29, 28, T>>(g, s, pl, R, p, nw, sm, grid, st);
+    if (split == 29 && fused) return launch_idct2<29, 28, T>(g, s, pl, R, p, x, err, st);
+    if (split == 29) return launch_idct_e<T, TwoPassX<29, 28, T>>(g, s, pl, R, p, x, st);
   }
   if constexpr (sizeof(T) == 4) {
-    if (split == 29 && fused) return launch_idct2<29, 28, T>(g, s, pl, R, p, nw, sm, grid, err, st);
-    if (split == 17 && fused) return launch_idct2<17, 30, T>(g, s, pl, R, p, nw, sm, grid, err, st);
-    if (split == 19 && fused) return launch_idct2<19, 10, T>(g, s, pl, R, p, nw, sm, grid, err, st);
-    if (split == 14 && fused) return launch_idct2<14, 9, T>(g, s, pl, R, p, nw, sm, grid, err, st);
-    if (split == 29) return launch_idct_e<T, TwoPassX<29, 28>>(g, s, pl, R, p, nw, sm, grid, st);
-    if (split == 17) return launch_idct_e<T, TwoPassX<17, 30>>(g, s, pl, R, p, nw, sm, grid, st);
-    if (split == 19) return launch_idct_e<T, TwoPassX<19, 10>>(g, s, pl, R, p, nw, sm, grid, st);
-    if (split == 14) return launch_idct_e<T, TwoPassX<14, 9>>(g, s, pl, R, p, nw, sm, grid, st);
+    if (split == 29 && fused) return launch_idct2<29, 28, T>(g, s, pl, R, p, x, err, st);
+    if (split == 17 && fused) return launch_idct2<17, 30, T>(g, s, pl, R, p, x, err, st);
+    if (split == 19 && fused) return launch_idct2<19, 10, T>(g, s, pl, R, p, x, err, st);
+    if (split == 14 && fused) return launch_idct2<14, 9, T>(g, s, pl, R, p, x, err, st);
+    if (split == 29) return launch_idct_e<T, TwoPassX<29, 28>>(g, s, pl, R, p, x, st);
+    if (split == 17) return launch_idct_e<T, TwoPassX<17, 30>>(g, s, pl, R, p, x, st);
+    if (split == 19) return launch_idct_e<T, TwoPassX<19, 10>>(g, s, pl, R, p, x, st);
+    if (split == 14) return launch_idct_e<T, TwoPassX<14, 9>>(g, s, pl, R, p, x, st);
   }
-  switch (radix_class(pl.rad, pl.nst)) {
-    case 7: launch_idct_e<T, StockhamX<T, 7>>(g, s, pl, R, p, nw, sm, grid, st); break;
-    case 13: launch_idct_e<T, StockhamX<T, 13>>(g, s, pl, R, p, nw, sm, grid, st); break;
-    case 19: launch_idct_e<T, StockhamX<T, 19>>(g, s, pl, R, p, nw, sm, grid, st); break;
-    case 29: launch_idct_e<T, StockhamX<T, 29>>(g, s, pl, R, p, nw, sm, grid, st); break;
-    default: launch_idct_e<T, StockhamX<T, 31>>(g, s, pl, R, p, nw, sm, grid, st); break;
-  }
+#define BLGPU_INVT(...) launch_idct_e<T, __VA_ARGS__>(g, s, pl, R, p, x, st)
+  BLGPU_STOCKHAM(BLGPU_INVT);
+#undef BLGPU_INVT
 }
+#undef BLGPU_STOCKHAM
+#undef BLGPU_C
 
 template <typename T, int RK>
 static void launch_dft_z_rk(const Spec &s, const T *R, T2<T> *C, const T2<T> *tz, int inverse, cudaStream_t st) {

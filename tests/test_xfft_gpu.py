@@ -142,3 +142,24 @@ def test_prime_stage_outputs(gpu, n):
         for a, b in zip(s.download_state()[:3], o.state()[:3]):
             assert rel(a, b) < (1e-12 if prec == FP64 else 1e-5)
         s.close()
+
+
+@pytest.mark.parametrize("n", [400, 401, 453, 555, 599, 601, 698, 887, 1022, 1259])
+@pytest.mark.parametrize("prec", [FP64, MIXED])
+def test_warps_per_line(gpu, n, prec):
+    """Lengths at the limits of the rule that gives a line several warps (a
+    prime factor above 31 and N >= 400: 401, 453 = 3 151, 555 = 3 5 37, 599
+    below 600; 601, 698, 887, 1022 from it on; 1259, where two FP64 lines are
+    half an SM's shared memory; 400 = 2^4 5^2 keeps one): an explicit line
+    count runs one warp per line, and the values are the same bits."""
+    c = noisy(n + 2, 5, 9, n)
+    runs = []
+    for nw in (0, 1):
+        s = cases.solver_for(c, precision=prec)
+        s.set_tiles(xfft=1, dct_nw=nw, idct_nw=nw)
+        s.apply_boundary_conditions(1)
+        s.compute_projection_step(1)
+        runs.append(s.download_state()[:3] + (s.rhs_p(),))
+        s.close()
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
