@@ -1035,13 +1035,12 @@ template <typename T> static const MetT<T> &met(const blgpu_ctx *ctx) {
 }
 
 template <typename T>
-static void enq_bc(blgpu_ctx *ctx, int b, int o, int rk_step) {
+static void enq_bc(blgpu_ctx *ctx, int b, int o, int rk_step, double tc = -1.0, bool save_to = false) {
   T **S = reinterpret_cast<T **>(ctx->S[b]);
   T **So = reinterpret_cast<T **>(ctx->S[o]);
   ph_begin(ctx, PH_BC);
-  launch_bc<T>(ctx->geo, ctx->bc, S[0], S[1], S[2], So[0], So[1], So[2], ctx->sc, ctx->rk_t[rk_step], ctx->qx_part,
-               ctx->qy, ctx->length_y, ctx->st);
-  ph_end(ctx, 2);
+  ph_end(ctx, launch_bc<T>(ctx->geo, ctx->bc, S[0], S[1], S[2], So[0], So[1], So[2], ctx->sc, ctx->rk_t[rk_step],
+                           ctx->qx_part, ctx->qy, ctx->length_y, tc, save_to, ctx->st));
 }
 
 template <typename T>
@@ -1075,7 +1074,7 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
     ph_begin(ctx, PH_PROJECT);
     launch_project<T>(ctx->geo, m, (const T *)ctx->rhs_p, mixed ? ctx->kz0 : nullptr, mixed ? ctx->kz0g : nullptr,
                       S[0], S[1], S[2], (T *)ctx->P, ctx->sc, rk_step == 1 ? 1 : 0, ctx->tiles, ctx->st);
-    ph_end(ctx, rk_step == 1 ? 2 : 1);
+    ph_end(ctx, 1);
     return;
   }
   ph_begin(ctx, PH_DIVDCT);
@@ -1123,7 +1122,7 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
   launch_project<T>(ctx->geo, m, (const T *)ctx->rhs_p, mixed ? ctx->kz0 : nullptr, mixed ? ctx->kz0g : nullptr,
                     S[0], S[1], S[2],
                     (T *)ctx->P, ctx->sc, rk_step == 1 ? 1 : 0, ctx->tiles, ctx->st);
-  ph_end(ctx, rk_step == 1 ? 2 : 1);
+  ph_end(ctx, 1);
 }
 
 template <typename T>
@@ -1159,14 +1158,10 @@ static int enq_wall_model(blgpu_ctx *ctx, const T *U, const T *W) {
 template <typename T>
 static int enq_step(blgpu_ctx *ctx, int a, bool with_dt) {
   const int b = (a + 1) % 3, c = (a + 2) % 3;
-  if (with_dt && ctx->cfg.cfl > 0) {  // dt, and the step's start time saved by the same launch
+  if (with_dt && ctx->cfg.cfl > 0) {
     T **S = reinterpret_cast<T **>(ctx->S[a]);
     ph_begin(ctx, PH_DT);
-    launch_dt<T>(ctx->geo, S[0], S[1], S[2], ctx->sc, ctx->cfg.cfl, ctx->dtvis, true, ctx->st);
-    ph_end(ctx, 1);
-  } else {
-    ph_begin(ctx, PH_MISC);
-    launch_set_time(ctx->sc, 0, 0.0, ctx->st);
+    launch_dt<T>(ctx->geo, S[0], S[1], S[2], ctx->sc, ctx->cfg.cfl, ctx->dtvis, ctx->st);
     ph_end(ctx, 1);
   }
   if (ctx->lund.mode) {  // Lund inflow once per step from the step's start fields
@@ -1175,7 +1170,9 @@ static int enq_step(blgpu_ctx *ctx, int a, bool with_dt) {
     launch_lund<T>(ctx->geo, ctx->lund, S[0], S[1], S[2], ctx->sc, 1, ctx->st);
     ph_end(ctx, 3);
   }
-  auto sub = [&](int mode, int in, int outb, double c1, double c2, double tc, int rk_step) {
+  // the first boundary pass moves the time to to + tc dt; the last one of the
+  // step saves it as the next step's start time
+  auto sub = [&](int mode, int in, int outb, double c1, double c2, double tc, int rk_step, bool last) {
     if (ctx->cfg.les_model == 1) {  // Smagorinsky from the substep's state (time_integration.f90:341-346)
       T **Si = reinterpret_cast<T **>(ctx->S[in]);
       ph_begin(ctx, PH_MISC);
@@ -1193,25 +1190,22 @@ static int enq_step(blgpu_ctx *ctx, int a, bool with_dt) {
       ph_end(ctx, enq_wall_model<T>(ctx, Si[0], Si[2]));
     }
     enq_rhs<T>(ctx, mode, in, a, outb, c1, c2);
-    ph_begin(ctx, PH_MISC);
-    launch_set_time(ctx->sc, 1, tc, ctx->st);
-    ph_end(ctx, 1);
-    enq_bc<T>(ctx, outb, a, rk_step);
+    enq_bc<T>(ctx, outb, a, rk_step, tc);
     enq_projection<T>(ctx, outb, rk_step);
-    enq_bc<T>(ctx, outb, a, rk_step);
+    enq_bc<T>(ctx, outb, a, rk_step, -1.0, last);
   };
   switch (ctx->cfg.rk_scheme) {
     case 3:  // time_integration.f90:305-465, initialization.f90:517-530
-      sub(1, a, b, 8.0 / 15.0, 0.0, 8.0 / 15.0, 1);
-      sub(2, b, c, 1.0 / 4.0, 5.0 / 12.0, 2.0 / 3.0, 2);
-      sub(3, c, b, 1.0 / 4.0, 3.0 / 4.0, 1.0, 3);
+      sub(1, a, b, 8.0 / 15.0, 0.0, 8.0 / 15.0, 1, false);
+      sub(2, b, c, 1.0 / 4.0, 5.0 / 12.0, 2.0 / 3.0, 2, false);
+      sub(3, c, b, 1.0 / 4.0, 3.0 / 4.0, 1.0, 3, true);
       return b;
     case 2:  // time_integration.f90:145-300, initialization.f90:504-513
-      sub(1, a, b, 1.0 / 2.0, 0.0, 1.0 / 2.0, 1);
-      sub(2, b, c, 0.0, 1.0, 1.0, 2);
+      sub(1, a, b, 1.0 / 2.0, 0.0, 1.0 / 2.0, 1, false);
+      sub(2, b, c, 0.0, 1.0, 1.0, 2, true);
       return c;
     default:  // Euler, time_integration.f90:24-114 (rk_step = 3)
-      sub(1, a, b, 1.0, 0.0, 1.0, 3);
+      sub(1, a, b, 1.0, 0.0, 1.0, 3, true);
       return b;
   }
 }
@@ -1300,10 +1294,10 @@ int blgpu_compute_dt(blgpu_ctx *ctx, double *dt) {
     CK(cudaMemcpy(&ctx->sc->dt, &v, sizeof v, cudaMemcpyHostToDevice));
   } else if (ctx->fp64) {
     double **S = reinterpret_cast<double **>(ctx->S[ctx->cur]);
-    launch_dt<double>(ctx->geo, S[0], S[1], S[2], ctx->sc, ctx->cfg.cfl, ctx->dtvis, false, ctx->st);
+    launch_dt<double>(ctx->geo, S[0], S[1], S[2], ctx->sc, ctx->cfg.cfl, ctx->dtvis, ctx->st);
   } else {
     float **S = reinterpret_cast<float **>(ctx->S[ctx->cur]);
-    launch_dt<float>(ctx->geo, S[0], S[1], S[2], ctx->sc, ctx->cfg.cfl, ctx->dtvis, false, ctx->st);
+    launch_dt<float>(ctx->geo, S[0], S[1], S[2], ctx->sc, ctx->cfg.cfl, ctx->dtvis, ctx->st);
   }
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));

@@ -86,15 +86,14 @@ void launch_project(const Geo &g, const MetT<T> &m, const T *p, const double *p0
                     T *W, T *P,
                     const Scalars *sc, int save_p, const Tiles &tl, cudaStream_t st);
 int bc_x_parts(const Geo &g);
+// tc >= 0: the call also moves the time to to + tc dt; save_to: it saves the
+// time as the next step's start time.  Returns the number of kernels launched.
 template <typename T>
-void launch_bc(const Geo &g, const BcData &bc, T *U, T *V, T *W, const T *Uo, const T *Vo, const T *Wo,
-               Scalars *sc, double rkt, double *qx_part, double qy, double length_y, cudaStream_t st);
-// save_time: the reduction's last block also saves the step's start time
-// (sc->to = sc->t, what launch_set_time phase 0 does)
+int launch_bc(const Geo &g, const BcData &bc, T *U, T *V, T *W, const T *Uo, const T *Vo, const T *Wo, Scalars *sc,
+              double rkt, double *qx_part, double qy, double length_y, double tc, bool save_to, cudaStream_t st);
 template <typename T>
 void launch_dt(const Geo &g, const T *U, const T *V, const T *W, Scalars *sc, double cfl, double dtvis,
-               bool save_time, cudaStream_t st);
-void launch_set_time(Scalars *sc, int phase, double coef, cudaStream_t st);
+               cudaStream_t st);
 template <typename T>
 void launch_maxdiv(const Geo &g, const T *U, const T *V, const T *W, unsigned long long *out, cudaStream_t st);
 

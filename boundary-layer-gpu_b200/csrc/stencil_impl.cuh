@@ -1221,59 +1221,40 @@ __global__ void __launch_bounds__(256) k_project_v(Geo g, MetT<T> m, const T *__
     Vec q;
 #pragma unroll
     for (int e = 0; e < VN; ++e) {
-      double pv = (double)pc.e[e];
-      if (p0 && i0 + e <= g.nx) pv += p0r[min(i0 + e - 2, N - 1)];
-      q.e[e] = (i0 + e <= g.nx) ? (T)(pv / den) : (T)0;
+      const int i = min(i0 + e, g.nx);  // past the interior: the ghost nxg takes the value at nx
+      double pv = (double)pc.e[i - i0];
+      if (p0) pv += p0r[min(i - 2, N - 1)];
+      q.e[e] = (i0 + e <= g.nxg) ? (T)(pv / den) : (T)0;
     }
-    *reinterpret_cast<VT *>(P + c) = q.v;
+    // The ghosts of projection.f90:78-83: the source copies the x ghosts, then
+    // the y ghosts (over every i, the x ghosts included), then the z ghosts
+    // (over every i, j), so every ghost point ends with the interior value at
+    // its clamped indices and the thread of that value writes them all.
+    const int jg = j == 2 ? 1 : j == g.nyg - 1 ? g.nyg : 0, kg = k == 2 ? 1 : k == g.nzg - 1 ? g.nzg : 0;
+    auto row = [&](int jj, int kk) {
+      const long long a = bidx(g, i0, jj, kk);
+      *reinterpret_cast<VT *>(P + a) = q.v;
+      if (i0 == 2) P[a - 1] = q.e[0];
+      if (i0 + VN == g.nxg) P[a + VN] = q.e[VN - 1];  // nx ends the vector
+    };
+    row(j, k);
+    if (jg) row(jg, k);
+    if (kg) {
+      row(j, kg);
+      if (jg) row(jg, kg);
+    }
   }
-}
-
-// P ghost planes, projection.f90:78-83.  The source copies the x ghosts, then
-// the y ghosts (over every i, the x ghosts included), then the z ghosts (over
-// every i, j); each copy takes the neighbouring layer, so every ghost point
-// ends with the interior value at its clamped indices (1 -> 2, n -> n-1 in
-// each direction), which this launch writes in one pass: blocks take the x
-// faces over (j, k), the y faces over (i, k) and the z faces over (i, j);
-// edges and corners are written alike by each face they lie on, and no
-// source value is a ghost.
-template <typename T>
-__global__ void k_p_ghost(Geo g, T *__restrict__ P, int bx, int by) {
-  int blk = blockIdx.x;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  auto cl = [](int v, int n) { return v == 1 ? 2 : v == n ? n - 1 : v; };
-  const int nxg = g.nxg, nyg = g.nyg, nzg = g.nzg;
-  if (blk < bx) {  // x faces, (j, k)
-    const int tj = (nyg + 31) / 32;
-    const int j = (blk % tj) * 32 + tx + 1, k = (blk / tj) * 8 + ty + 1;
-    if (j > nyg || k > nzg) return;
-    const int cj = cl(j, nyg), ck = cl(k, nzg);
-    P[bidx(g, 1, j, k)] = P[bidx(g, 2, cj, ck)];
-    P[bidx(g, nxg, j, k)] = P[bidx(g, nxg - 1, cj, ck)];
-    return;
-  }
-  blk -= bx;
-  const int ti = (nxg + 31) / 32;
-  if (blk < by) {  // y faces, (i, k)
-    const int i = (blk % ti) * 32 + tx + 1, k = (blk / ti) * 8 + ty + 1;
-    if (i > nxg || k > nzg) return;
-    const int ci = cl(i, nxg), ck = cl(k, nzg);
-    P[bidx(g, i, 1, k)] = P[bidx(g, ci, 2, ck)];
-    P[bidx(g, i, nyg, k)] = P[bidx(g, ci, nyg - 1, ck)];
-    return;
-  }
-  blk -= by;  // z faces, (i, j)
-  const int i = (blk % ti) * 32 + tx + 1, j = (blk / ti) * 8 + ty + 1;
-  if (i > nxg || j > nyg) return;
-  const int ci = cl(i, nxg), cj = cl(j, nyg);
-  P[bidx(g, i, j, 1)] = P[bidx(g, ci, cj, 2)];
-  P[bidx(g, i, j, nzg)] = P[bidx(g, ci, cj, nzg - 1)];
 }
 
 // ---------------------------------------------------------------------------
 // Boundary conditions, boundary_conditions.f90:127-262, in two ordered
 // launches: k_bc_all (every boundary value but the mass correction, and the
-// x mass-flux sum) and k_bc_mass (the correction of U(nx-1), U(nx)).
+// x mass-flux sum) and k_bc_mass (the correction of U(nx-1), U(nx)).  (The
+// correction by the last block of k_bc_all saves a launch, but its 256
+// threads take longer over the plane than the launch: 0.094 -> 0.200 ms per
+// step at 256 x 65 x 96.)  The first call of a substep also moves the time
+// (tc >= 0: t = to + tc dt, time_integration.f90:349,383,417), the last one
+// of a step saves it as the next step's start time.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double mode_sum(const double2 *__restrict__ q, int ld, int j, int nm, int mm,
                                            const double *__restrict__ zmode, const double *__restrict__ tmode,
@@ -1380,8 +1361,13 @@ __global__ void __launch_bounds__(256) k_bc_all(Geo g, BcData bc, BcGrid G, T *_
                                                 T *__restrict__ W, const T *__restrict__ Uo,
                                                 const T *__restrict__ Vo, const T *__restrict__ Wo,
                                                 Scalars *__restrict__ sc, double rkt, double *__restrict__ qx_part,
-                                                double qy, double length_y) {
+                                                double qy, double length_y, double tc, int save_to) {
   int blk = blockIdx.x;
+  const double t = tc >= 0.0 ? __dadd_rn(sc->to, __dmul_rn(tc, sc->dt)) : sc->t;
+  if (blk == 0 && threadIdx.x == 0) {
+    if (tc >= 0.0) sc->t = t;
+    if (save_to) sc->to = t;
+  }
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int nx = g.nx, nxg = g.nxg, ny = g.ny, nyg = g.nyg, nz = g.nz, nzg = g.nzg;
   typedef BcX<T> X;
@@ -1390,7 +1376,7 @@ __global__ void __launch_bounds__(256) k_bc_all(Geo g, BcData bc, BcGrid G, T *_
     const int bb = (blk - G.nx_blocks) % G.nx_blocks;
     const int j = (bb % G.x_tiles) * 32 + tx + 1, k = (bb / G.x_tiles) * 8 + ty + 1;
     if (j > nyg || k > nzg) return;
-    const double t = sc->t, cc = rkt * sc->dt * bc.U_top[nx];
+    const double cc = rkt * sc->dt * bc.U_top[nx];
     if (blk < 2 * G.nx_blocks) {
       if (j > ny) return;  // V at i = 1, nxg-1, nxg
       const int kv = X::ks_uv(g, k);
@@ -1438,8 +1424,8 @@ __global__ void __launch_bounds__(256) k_bc_all(Geo g, BcData bc, BcGrid G, T *_
     const int j = (blk % G.x_tiles) * 32 + tx + 1, k = (blk / G.x_tiles) * 8 + ty + 1;
     double q = 0.0;
     if (j <= nyg && k <= nzg) {
-      const double t = sc->t, cc = rkt * sc->dt * bc.U_top[nx];
-      // U at i = 1 and nx-1 (k_bc_mass sets i = nx)
+      const double cc = rkt * sc->dt * bc.U_top[nx];
+      // U at i = 1 and nx-1 (the mass correction sets i = nx)
       const int ku = X::ks_uv(g, k);
       T u1, un;
       if (j == nyg) {
@@ -1569,7 +1555,7 @@ __global__ void k_bc_mass(Geo g, T *__restrict__ U, const Scalars *__restrict__ 
 // ---------------------------------------------------------------------------
 // dt from the maxima of the reduction (time_integration.f90:580-590), by the
 // last block to finish: the arrival counter after every block's atomics
-__device__ __forceinline__ void dt_finish_last(Scalars *sc, double cfl, double dtvis, int save_time) {
+__device__ __forceinline__ void dt_finish_last(Scalars *sc, double cfl, double dtvis) {
   __threadfence();
   const unsigned int nb = gridDim.x * gridDim.y * gridDim.z;
   if (atomicAdd(&sc->dt_arrived, 1u) != nb - 1) return;
@@ -1582,13 +1568,12 @@ __device__ __forceinline__ void dt_finish_last(Scalars *sc, double cfl, double d
   sc->dt = fmin(dt_conv, dtvis);
   sc->lmax[0] = sc->lmax[1] = sc->lmax[2] = 0ull;
   sc->dt_arrived = 0u;
-  if (save_time) sc->to = sc->t;  // the step's start time (k_set_time phase 0)
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_dt_reduce(Geo g, const T *__restrict__ U, const T *__restrict__ V,
                                                    const T *__restrict__ W, Scalars *__restrict__ sc, int kchunk,
-                                                   double cfl, double dtvis, int save_time) {
+                                                   double cfl, double dtvis) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
   double mu = 0.0, mv = 0.0, mw = 0.0;
@@ -1636,7 +1621,7 @@ __global__ void __launch_bounds__(256) k_dt_reduce(Geo g, const T *__restrict__ 
     atomicMax(&sc->lmax[0], (unsigned long long)__double_as_longlong(mu));
     atomicMax(&sc->lmax[1], (unsigned long long)__double_as_longlong(mv));
     atomicMax(&sc->lmax[2], (unsigned long long)__double_as_longlong(mw));
-    dt_finish_last(sc, cfl, dtvis, save_time);
+    dt_finish_last(sc, cfl, dtvis);
   }
 }
 
@@ -1650,7 +1635,7 @@ __global__ void __launch_bounds__(256) k_dt_reduce(Geo g, const T *__restrict__ 
 template <typename T>  // double
 __global__ void __launch_bounds__(256) k_dt_reduce2(Geo g, const T *__restrict__ U, const T *__restrict__ V,
                                                     const T *__restrict__ W, Scalars *__restrict__ sc, int kchunk,
-                                                    double cfl, double dtvis, int save_time) {
+                                                    double cfl, double dtvis) {
   const int i0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
   double mu = 0.0, mv = 0.0, mw = 0.0;
@@ -1713,7 +1698,7 @@ __global__ void __launch_bounds__(256) k_dt_reduce2(Geo g, const T *__restrict__
     atomicMax(&sc->lmax[0], (unsigned long long)__double_as_longlong(mu));
     atomicMax(&sc->lmax[1], (unsigned long long)__double_as_longlong(mv));
     atomicMax(&sc->lmax[2], (unsigned long long)__double_as_longlong(mw));
-    dt_finish_last(sc, cfl, dtvis, save_time);
+    dt_finish_last(sc, cfl, dtvis);
   }
 }
 
@@ -1723,7 +1708,7 @@ __global__ void __launch_bounds__(256) k_dt_reduce2(Geo g, const T *__restrict__
 template <typename T>  // float
 __global__ void __launch_bounds__(256) k_dt_reduce4(Geo g, const T *__restrict__ U, const T *__restrict__ V,
                                                     const T *__restrict__ W, Scalars *__restrict__ sc, int kchunk,
-                                                    double cfl, double dtvis, int save_time) {
+                                                    double cfl, double dtvis) {
   const int i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x) + 2;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 2;
   double mu = 0.0, mv = 0.0, mw = 0.0;
@@ -1787,20 +1772,12 @@ __global__ void __launch_bounds__(256) k_dt_reduce4(Geo g, const T *__restrict__
     atomicMax(&sc->lmax[0], (unsigned long long)__double_as_longlong(mu));
     atomicMax(&sc->lmax[1], (unsigned long long)__double_as_longlong(mv));
     atomicMax(&sc->lmax[2], (unsigned long long)__double_as_longlong(mw));
-    dt_finish_last(sc, cfl, dtvis, save_time);
+    dt_finish_last(sc, cfl, dtvis);
   }
 }
 
 // time_integration.f90:560-575 (dt = min(dt_conv, dt_vis)); also arms the
 // accumulators for the next call and records to = t for the RK substeps.
-
-#ifdef BLGPU_STENCIL_PRIMARY
-__global__ void k_set_time(Scalars *sc, int phase, double coef) {
-  // phase 0: to = t (save at step start); phase 1: t = to + coef*dt
-  if (phase == 0) sc->to = sc->t;
-  else sc->t = sc->to + coef * sc->dt;
-}
-#endif
 
 // check_divergence (projection.f90:399-408): max |div| over i=2..nxg-2
 template <typename T>
@@ -2165,11 +2142,6 @@ void launch_project(const Geo &g, const MetT<T> &m, const T *p, const double *p0
   const int by = tl.proj_by > 0 ? tl.proj_by : 4;  // 4 rows: the autotuner's choice at 814 x 257 x 193 in both precisions
   dim3 block(32, by), grid((ngrp + 31) / 32, (g.ny - 1 + by - 1) / by, g.nz - 1);
   k_project_v<T><<<grid, block, 0, st>>>(g, m, p, p0, p0g, U, V, W, P, sc, save_p);
-  if (save_p) {
-    const int bx = ((g.nyg + 31) / 32) * ((g.nzg + 7) / 8), by = ((g.nxg + 31) / 32) * ((g.nzg + 7) / 8);
-    const int bz = ((g.nxg + 31) / 32) * ((g.nyg + 7) / 8);
-    k_p_ghost<T><<<bx + by + bz, 256, 0, st>>>(g, P, bx, by);
-  }
 }
 
 #ifdef BLGPU_STENCIL_PRIMARY
@@ -2177,8 +2149,8 @@ int bc_x_parts(const Geo &g) { return ((g.nyg + 31) / 32) * ((g.nzg + 7) / 8); }
 #endif
 
 template <typename T>
-void launch_bc(const Geo &g, const BcData &bc, T *U, T *V, T *W, const T *Uo, const T *Vo, const T *Wo,
-               Scalars *sc, double rkt, double *qx_part, double qy, double length_y, cudaStream_t st) {
+int launch_bc(const Geo &g, const BcData &bc, T *U, T *V, T *W, const T *Uo, const T *Vo, const T *Wo, Scalars *sc,
+              double rkt, double *qx_part, double qy, double length_y, double tc, bool save_to, cudaStream_t st) {
   BcGrid G;
   G.x_tiles = (g.nyg + 31) / 32;
   G.nx_blocks = G.x_tiles * ((g.nzg + 7) / 8);  // = bc_x_parts(g)
@@ -2186,14 +2158,15 @@ void launch_bc(const Geo &g, const BcData &bc, T *U, T *V, T *W, const T *Uo, co
   G.nz_blocks = G.zi_tiles * ((g.nyg - 2 + 7) / 8);
   G.yi_tiles = G.zi_tiles;
   G.ny_blocks = G.yi_tiles * ((g.nzg + 7) / 8);
-  k_bc_all<T><<<3 * G.nx_blocks + G.nz_blocks + G.ny_blocks, 256, 0, st>>>(g, bc, G, U, V, W, Uo, Vo, Wo, sc, rkt,
-                                                                         qx_part, qy, length_y);
+  k_bc_all<T><<<3 * G.nx_blocks + G.nz_blocks + G.ny_blocks, 256, 0, st>>>(
+      g, bc, G, U, V, W, Uo, Vo, Wo, sc, rkt, qx_part, qy, length_y, tc, save_to ? 1 : 0);
   k_bc_mass<T><<<dim3((g.nyg + 31) / 32, (g.nzg + 7) / 8), dim3(32, 8), 0, st>>>(g, U, sc);
+  return 2;
 }
 
 template <typename T>
 void launch_dt(const Geo &g, const T *U, const T *V, const T *W, Scalars *sc, double cfl, double dtvis,
-               bool save_time, cudaStream_t st) {
+               cudaStream_t st) {
   const int kchunk = 32;
   // 16-byte vectors: rows of 4 floats / 2 doubles from i = 2 (element i + 2 of a row)
   const bool vec = (g.px & (sizeof(T) == 4 ? 3 : 1)) == 0 &&
@@ -2202,23 +2175,17 @@ void launch_dt(const Geo &g, const T *U, const T *V, const T *W, Scalars *sc, do
   if (vec) {
     if constexpr (sizeof(T) == 4) {
       dim3 grid = vol_grid((g.nxg - 2 + 3) / 4, g.nyg - 2, g.nzg - 2, kchunk), block(32, 8);
-      k_dt_reduce4<T><<<grid, block, 0, st>>>(g, U, V, W, sc, kchunk, cfl, dtvis, save_time ? 1 : 0);
+      k_dt_reduce4<T><<<grid, block, 0, st>>>(g, U, V, W, sc, kchunk, cfl, dtvis);
     } else {
       dim3 grid = vol_grid((g.nxg - 2 + 1) / 2, g.nyg - 2, g.nzg - 2, kchunk), block(32, 8);
-      k_dt_reduce2<T><<<grid, block, 0, st>>>(g, U, V, W, sc, kchunk, cfl, dtvis, save_time ? 1 : 0);
+      k_dt_reduce2<T><<<grid, block, 0, st>>>(g, U, V, W, sc, kchunk, cfl, dtvis);
     }
   }
   if (!vec) {
     dim3 grid = vol_grid(g.nxg - 2, g.nyg - 2, g.nzg - 2, kchunk), block(32, 8);
-    k_dt_reduce<T><<<grid, block, 0, st>>>(g, U, V, W, sc, kchunk, cfl, dtvis, save_time ? 1 : 0);
+    k_dt_reduce<T><<<grid, block, 0, st>>>(g, U, V, W, sc, kchunk, cfl, dtvis);
   }
 }
-
-#ifdef BLGPU_STENCIL_PRIMARY
-void launch_set_time(Scalars *sc, int phase, double coef, cudaStream_t st) {
-  k_set_time<<<1, 1, 0, st>>>(sc, phase, coef);
-}
-#endif
 
 template <typename T>
 void launch_maxdiv(const Geo &g, const T *U, const T *V, const T *W, unsigned long long *out, cudaStream_t st) {
@@ -2255,9 +2222,9 @@ void launch_law_of_wall(const Geo &g, const T *U, double *utau, int *iters, int 
   template void launch_project<T>(const Geo &, const MetT<T> &, const T *, const double *, const float *, T *,    \
                                   T *, T *, T *,                                                                    \
                                   const Scalars *, int, const Tiles &, cudaStream_t);                               \
-  template void launch_bc<T>(const Geo &, const BcData &, T *, T *, T *, const T *, const T *, const T *,         \
-                             Scalars *, double, double *, double, double, cudaStream_t);                            \
-  template void launch_dt<T>(const Geo &, const T *, const T *, const T *, Scalars *, double, double, bool,        \
+  template int launch_bc<T>(const Geo &, const BcData &, T *, T *, T *, const T *, const T *, const T *,         \
+                             Scalars *, double, double *, double, double, double, bool, cudaStream_t);              \
+  template void launch_dt<T>(const Geo &, const T *, const T *, const T *, Scalars *, double, double,              \
                              cudaStream_t);                                                                         \
   template void launch_maxdiv<T>(const Geo &, const T *, const T *, const T *, unsigned long long *, cudaStream_t); \
   template void launch_smagorinsky<T>(const Geo &, const MetT<T> &, const T *, const T *, const T *, const double *, T *, \

@@ -317,3 +317,38 @@ def test_tile_scan_y_solve_oracle_steps(gpu):
         assert rel(a, b) < REL10
     assert s.check_divergence() < 1e-12
     s.close()
+
+
+@pytest.mark.parametrize("grid", [(5, 4, 5), (6, 5, 6), (7, 4, 8), (8, 9, 5), (9, 6, 7), (34, 20, 19)])
+@pytest.mark.parametrize("rk", [1, 2, 3])
+def test_step_pressure_ghosts_and_time(gpu, grid, rk):
+    """A step's pressure with its ghosts, written by the projection (rows of 4
+    FP32 or 2 FP64 values: nx = 5 .. 9 ends a row at each place), and the time
+    moved and saved by the boundary pass (inflow modes read it at every
+    substep of RK3, RK2 and Euler, three steps in a row at a fixed dt):
+    against the oracle at the bars of the steps above."""
+    c = noisy_laminar(*grid, seed=sum(grid), amp=1e-3, cfl=-1e-3, rk_scheme=rk)
+    ny, nyg = grid[1], grid[1] + 1
+    rng = np.random.default_rng(5)
+    q = lambda n: 1e-3 * (rng.standard_normal((n, 2, 1)) + 1j * rng.standard_normal((n, 2, 1)))
+    modes = (np.array([0.0, 2.0]), np.array([30.0]), q(nyg), q(ny), q(nyg))
+    o = oracle.oracle_for(c)
+    o.set_modes(*modes)
+    o.advance(3)
+    ref = o.state()
+    for prec in (FP64, MIXED):
+        s = cases.solver_for(c, precision=prec)
+        s.set_inflow_modes(*modes)
+        s.time_step()
+        s.advance(2)
+        got = s.download_state()
+        assert got[4] == pytest.approx(ref[4], rel=1e-14)
+        for a, b in zip(got[:3], ref[:3]):
+            assert rel(a, b) < (REL10 if prec == FP64 else 1e-3)
+        P = got[3]
+        # ghosts equal the interior values at their clamped indices, to the bit
+        cl = lambda n: np.clip(np.arange(n), 1, n - 2)
+        assert np.array_equal(P, P[np.ix_(*(cl(n) for n in P.shape))])
+        if prec == FP64:
+            assert rel(P, ref[3]) < 1e-8
+        s.close()
