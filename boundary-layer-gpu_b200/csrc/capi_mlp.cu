@@ -40,8 +40,8 @@ struct blgpu_mlp {
   float *Xq = nullptr, *Yq = nullptr;
   int *idq = nullptr;
   int qcap = 0;
-  // training graph
-  cudaGraphExec_t graph = nullptr;
+  // training graphs: one step, and GRAPH_STEPS steps in a row
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int graph_B = 0;
   float graph_lr = 0.f;
   std::string err;
@@ -75,9 +75,9 @@ static unsigned long long splitmix(unsigned long long &s) {
 static double unif(unsigned long long &s) { return (double)(splitmix(s) >> 11) * (1.0 / 9007199254740992.0); }
 
 static void drop_graph(blgpu_mlp *m) {
-  if (m->graph) {
-    cudaGraphExecDestroy(m->graph);
-    m->graph = nullptr;
+  for (cudaGraphExec_t &g : m->graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
   }
 }
 
@@ -307,8 +307,30 @@ int blgpu_mlp_get_data(blgpu_mlp *m, float *X, float *T, int rows) {
   return BLGPU_OK;
 }
 
-// `steps` Adam steps of `batch` samples each, replayed from a CUDA graph of
-// one step (gradient; fixed-order reduction + update + repack; offset).
+// `steps` Adam steps of `batch` samples each, replayed from CUDA graphs of one
+// step (gradient; fixed-order reduction + update + repack; offset) and of
+// GRAPH_STEPS steps: within a graph a step's launches follow each other
+// without the gap between two graphs (400 steps of 8192 samples: 11.9 ->
+// 11.2 ms).
+static constexpr int GRAPH_STEPS = 16;
+
+static int capture_steps(blgpu_mlp *m, int n, int batch, float lr, cudaGraphExec_t *out) {
+  cudaGraph_t gr = nullptr;
+  MCK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeRelaxed));
+  for (int s = 0; s < n; ++s) {
+    launch_mlp_grad(m->pack, m->bias, m->X, m->T, m->perm, m->n, reinterpret_cast<const int *>(m->stv + 1), batch,
+                    m->part, m->st);
+    launch_mlp_adam(m->part, mlp_train_ctas(batch), m->params, m->m1, m->m2, m->stv, lr, batch, m->n, m->hist,
+                    m->hist_n, m->pack, m->bias, m->st);
+  }
+  cudaError_t e = cudaStreamEndCapture(m->st, &gr);
+  if (e != cudaSuccess) return merr(m, BLGPU_ECUDA, "training capture: %s", cudaGetErrorString(e));
+  e = cudaGraphInstantiate(out, gr, 0);
+  cudaGraphDestroy(gr);
+  if (e != cudaSuccess) return merr(m, BLGPU_ECUDA, "training graph: %s", cudaGetErrorString(e));
+  return BLGPU_OK;
+}
+
 int blgpu_mlp_train(blgpu_mlp *m, int steps, int batch, float lr, float *loss_last) {
   if (!m || steps < 0 || batch < 1 || !(lr > 0.f)) return merr(m, BLGPU_EINVAL, "blgpu_mlp_train: bad argument");
   if (m->n < 1) return merr(m, BLGPU_ESTATE, "blgpu_mlp_train: no training samples");
@@ -316,23 +338,15 @@ int blgpu_mlp_train(blgpu_mlp *m, int steps, int batch, float lr, float *loss_la
   MCK(cudaSetDevice(m->device));
   int rc = reshuffle(m);
   if (rc) return rc;
-  if (m->graph && (m->graph_B != batch || m->graph_lr != lr)) drop_graph(m);
-  if (!m->graph) {
-    cudaGraph_t gr = nullptr;
-    MCK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeRelaxed));
-    launch_mlp_grad(m->pack, m->bias, m->X, m->T, m->perm, m->n, reinterpret_cast<const int *>(m->stv + 1), batch,
-                    m->part, m->st);
-    launch_mlp_adam(m->part, mlp_train_ctas(batch), m->params, m->m1, m->m2, m->stv, lr, batch, m->n, m->hist,
-                    m->hist_n, m->pack, m->bias, m->st);
-    cudaError_t e = cudaStreamEndCapture(m->st, &gr);
-    if (e != cudaSuccess) return merr(m, BLGPU_ECUDA, "training capture: %s", cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&m->graph, gr, 0);
-    cudaGraphDestroy(gr);
-    if (e != cudaSuccess) return merr(m, BLGPU_ECUDA, "training graph: %s", cudaGetErrorString(e));
-    m->graph_B = batch;
-    m->graph_lr = lr;
+  if (m->graph_B != batch || m->graph_lr != lr) drop_graph(m);
+  m->graph_B = batch;
+  m->graph_lr = lr;
+  for (int s = 0; s < steps;) {
+    const int big = steps - s >= GRAPH_STEPS ? 1 : 0, n = big ? GRAPH_STEPS : 1;
+    if (!m->graph[big] && (rc = capture_steps(m, n, batch, lr, &m->graph[big]))) return rc;
+    MCK(cudaGraphLaunch(m->graph[big], m->st));
+    s += n;
   }
-  for (int s = 0; s < steps; ++s) MCK(cudaGraphLaunch(m->graph, m->st));
   MCK(cudaGetLastError());
   if (loss_last) MCK(cudaMemcpyAsync(loss_last, m->stv + 2, sizeof(float), cudaMemcpyDeviceToHost, m->st));
   MCK(cudaStreamSynchronize(m->st));

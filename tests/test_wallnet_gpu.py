@@ -66,6 +66,22 @@ def test_training_is_deterministic_and_fits(gpu):
     assert np.isfinite(hist).all() and hist[-50:].mean() < hist[:50].mean()
 
 
+@pytest.mark.parametrize("steps", [1, 15, 16, 17, 35])
+def test_training_leg_equals_single_steps(gpu, steps):
+    """Legs below, at and above the length of the multi-step graph."""
+    X, T = inputs(3000, 4)
+    out = []
+    for legs in ([steps], [1] * steps):
+        net = WallNet(seed=6)
+        net.add_data(X, T)
+        for n in legs:
+            net.train(n, batch=512, lr=1e-3)
+        out.append((net.params, net.loss_history(steps)))
+        net.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
+
+
 def test_wall_samples_match_fields(gpu):
     c = wallmodel.dns_boxes(retheta=(1100.0,), nx=40, nz=12)[0]
     s = cases.solver_for(c, precision=FP64, inflow=False)
