@@ -1055,11 +1055,18 @@ __global__ void __launch_bounds__(256) k_dft_z_inv(Spec s, const T2<T> *__restri
 //   inverse  f_p, f_{M-p} = (C_0 + 2 (P_p -+ Q_p) [+ (-1)^p C_{M/2}]) / M,
 //            P_p = sum_{k=1..H} Re C_k cos(2 pi p k/M), Q_p = sum Im C_k sin(...)
 // are each a product (rows r or p) x (K = H terms) x (32 x columns of a CTA)
-// with the tables tc[r][k-1] = cos, ts[r][k-1] = sin (rows to MHp = MH
-// rounded up to 16, columns to Kp = H rounded up to 4, zero beyond H and
-// MH).  A CTA owns one row b and 32 kx; its column data sit in shared memory
-// transposed ([x][k], pitch PZ = 4 mod 16 doubles, so the B fragments meet
-// two wavefronts); the forward folds S_k, D_k in place (F[x][k], F[x][M-k]).
+// with the tables cos, sin (rows to MH rounded up to 16, columns to Kp = H
+// rounded up to 4, zero beyond H and MH), stored in the order the lanes read
+// them: for row tile rt and K step ks, lane l's four values (cos at rows
+// 16 rt + l/4 and + 8, column 4 ks + l%4; sin at the same) are contiguous, so
+// a step is two coalesced 16-byte loads per lane.  A CTA owns one row b and
+// 32 kx; its column data sit in shared memory as [k][x] with pitch ZP = 4 mod
+// 16 doubles: the rows are written without bank conflicts and the B fragments
+// meet two wavefronts.  The forward folds S_k (row k) and D_k (row M-k) while
+// it loads.  The L1 (shared memory and table reads) bounded the kernel before
+// that: the table read row by row cost four times the wavefronts, and a
+// transposed [x][k] layout eight-way conflicts of every store.  At
+// 814 x 257 x 193: forward 412 -> 329 us, inverse 372 -> 346 us per launch.
 // Warp w computes rows 16w .. 16w+15 by 2 x 4 MMA tiles of 8 x 8, K in steps
 // of 4.  Fragments (PTX m8n8k4 .f64): A a0 at (row lane/4, col lane%4), B b0
 // at (row lane%4, col lane/4), C c0, c1 at (row lane/4, cols 2 (lane%4) + i).
@@ -1071,35 +1078,50 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 }
 __host__ __device__ inline int zd64_kp(int M) { return ((M - 1) / 2 + 3) / 4 * 4; }
 __host__ __device__ inline int zd64_rows(int M) { return (M / 2 + 1 + 15) / 16 * 16; }
-// pitch of the transposed column data: >= the larger of M and Kp + 1, = 4 mod 16
-__host__ __device__ inline int zd64_pitch(int len) { return (len + 11) / 16 * 16 + 4; }
+// rows of the inverse's column data: kz = 0 .. M/2 and the products' K range 1 .. Kp
+__host__ __device__ inline int zd64_crows(int M) { return zd64_kp(M) + 1 > M / 2 + 1 ? zd64_kp(M) + 1 : M / 2 + 1; }
+// 112 registers: three CTAs of six warps per SM (M = 191), two at the 126 and 118 taken otherwise
+#define ZD64_REGS __maxnreg__(112)
+constexpr int ZP = 36;  // pitch of the [k][x] column data, 32 columns
 
-__global__ void __launch_bounds__(256) k_zdft64_fwd(Spec s, const double *__restrict__ R, double2 *__restrict__ C,
-                                                    const double *__restrict__ tc, const double *__restrict__ ts) {
-  extern __shared__ double zf[];  // [32][PZ]
-  const int M = s.M, MH = s.MH, H = (M - 1) / 2, Kp = zd64_kp(M), PZ = zd64_pitch(M);
+// lane l's table fragments of row tile rt: two double2 (cos, sin) per K step
+__device__ __forceinline__ const double2 *zd64_frag(const double *tab, int rt, int ks, int lane) {
+  return reinterpret_cast<const double2 *>(tab) + ((size_t)rt * ks * 32 + lane) * 2;
+}
+
+__global__ void ZD64_REGS k_zdft64_fwd(Spec s, const double *__restrict__ R,
+                                                              double2 *__restrict__ C,
+                                                              const double *__restrict__ tab) {
+  extern __shared__ __align__(16) double zf[];  // [M][ZP]
+  const int M = s.M, MH = s.MH, H = (M - 1) / 2, Kp = zd64_kp(M);
+  const bool even = (M & 1) == 0;
   const int b = blockIdx.y, x0 = blockIdx.x * 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const bool xin = x0 + lane < s.N;
-  // rows in batches of 8 per warp, every load of a batch issued before the
-  // stores (the slab comes from DRAM)
-  for (int k8 = warp * 8; k8 < PZ; k8 += nw * 8) {
-    double v[8];
+  // rows k and M-k in batches of 4 pairs per warp, every load of a batch
+  // issued before the stores (the slab comes from DRAM)
+  const double *Rc = R + (long long)b * M * s.rx + x0 + lane;
+  for (int k4 = 1 + warp * 4; k4 <= H; k4 += nw * 4) {
+    double v[4], w[4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int k = k8 + u;
-      v[u] = (k < M && xin) ? __ldcs(R + ((long long)b * M + k) * s.rx + x0 + lane) : 0.0;
+    for (int u = 0; u < 4; ++u) {
+      const int k = k4 + u;
+      const bool in = k <= H && xin;
+      v[u] = in ? __ldcs(Rc + (long long)k * s.rx) : 0.0;
+      w[u] = in ? __ldcs(Rc + (long long)(M - k) * s.rx) : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (k8 + u < PZ) zf[lane * PZ + k8 + u] = v[u];
+    for (int u = 0; u < 4; ++u) {
+      const int k = k4 + u;
+      if (k <= H) {
+        zf[k * ZP + lane] = v[u] + w[u];
+        zf[(M - k) * ZP + lane] = v[u] - w[u];
+      }
+    }
   }
-  __syncthreads();
-  for (int t = tid; t < 32 * H; t += blockDim.x) {
-    const int x = t & 31, k = 1 + (t >> 5);
-    const double a = zf[x * PZ + k], c = zf[x * PZ + M - k];
-    zf[x * PZ + k] = a + c;
-    zf[x * PZ + M - k] = a - c;
+  if (warp == nw - 1) {  // the rows without a partner
+    zf[lane] = xin ? __ldcs(Rc) : 0.0;
+    if (even) zf[M / 2 * ZP + lane] = xin ? __ldcs(Rc + (long long)(M / 2) * s.rx) : 0.0;
   }
   __syncthreads();
   const int r0 = 16 * warp;
@@ -1107,21 +1129,21 @@ __global__ void __launch_bounds__(256) k_zdft64_fwd(Spec s, const double *__rest
   const int g = lane >> 2, q = lane & 3;
   double re[2][4][2] = {}, im[2][4][2] = {};
   // table fragments of the next K step fetched one step ahead
-  const double *tcr = tc + (r0 + g) * Kp + q, *tsr = ts + (r0 + g) * Kp + q;
-  double nc[2] = {__ldg(tcr), __ldg(tcr + 8 * Kp)}, ns[2] = {__ldg(tsr), __ldg(tsr + 8 * Kp)};
+  const double2 *tf = zd64_frag(tab, warp, Kp / 4, lane);
+  double2 nc = __ldg(tf), ns = __ldg(tf + 1);
   for (int k0 = 1; k0 <= Kp; k0 += 4) {
-    const int k = k0 + q;  // 1 .. Kp: S_k at zf[x][k], D_k at zf[x][M-k] (table zero for k > H)
-    double ac[2] = {nc[0], nc[1]}, as[2] = {ns[0], ns[1]}, bs[4], bd[4];
+    const int k = k0 + q;  // 1 .. Kp: S_k in row k, D_k in row M-k (table zero for k > H)
+    const double ac[2] = {nc.x, nc.y}, as[2] = {ns.x, ns.y};
+    double bs[4], bd[4];
     if (k0 + 4 <= Kp) {
-      nc[0] = __ldg(tcr + k0 + 3);
-      nc[1] = __ldg(tcr + 8 * Kp + k0 + 3);
-      ns[0] = __ldg(tsr + k0 + 3);
-      ns[1] = __ldg(tsr + 8 * Kp + k0 + 3);
+      tf += 64;
+      nc = __ldg(tf);
+      ns = __ldg(tf + 1);
     }
 #pragma unroll
     for (int ct = 0; ct < 4; ++ct) {
-      bs[ct] = zf[(8 * ct + g) * PZ + k];
-      bd[ct] = zf[(8 * ct + g) * PZ + M - k];
+      bs[ct] = zf[k * ZP + 8 * ct + g];
+      bd[ct] = zf[(M - k) * ZP + 8 * ct + g];
     }
 #pragma unroll
     for (int rt = 0; rt < 2; ++rt)
@@ -1131,7 +1153,6 @@ __global__ void __launch_bounds__(256) k_zdft64_fwd(Spec s, const double *__rest
         dmma(im[rt][ct], as[rt], bd[ct]);
       }
   }
-  const bool even = (M & 1) == 0;
 #pragma unroll
   for (int rt = 0; rt < 2; ++rt) {
     const int r = r0 + 8 * rt + g;
@@ -1142,22 +1163,23 @@ __global__ void __launch_bounds__(256) k_zdft64_fwd(Spec s, const double *__rest
       for (int i = 0; i < 2; ++i) {
         const int x = 8 * ct + 2 * q + i;
         if (x0 + x >= s.N) continue;
-        double a = zf[x * PZ] + re[rt][ct][i];
-        if (even) a += (r & 1) ? -zf[x * PZ + M / 2] : zf[x * PZ + M / 2];
+        double a = zf[x] + re[rt][ct][i];
+        if (even) a += (r & 1) ? -zf[M / 2 * ZP + x] : zf[M / 2 * ZP + x];
         C[((long long)b * MH + r) * s.rx + x0 + x] = make_double2(a, -im[rt][ct][i]);
       }
   }
 }
 
-__global__ void __launch_bounds__(256) k_zdft64_inv(Spec s, const double2 *__restrict__ C, double *__restrict__ R,
-                                                    const double *__restrict__ tc, const double *__restrict__ ts) {
-  extern __shared__ double zf[];  // Re [32][PZ], then Im [32][PZ]
-  const int M = s.M, MH = s.MH, Kp = zd64_kp(M), PZ = zd64_pitch(Kp + 1 > MH ? Kp + 1 : MH);
-  double *zr = zf, *zi = zf + 32 * PZ;
+__global__ void ZD64_REGS k_zdft64_inv(Spec s, const double2 *__restrict__ C,
+                                                              double *__restrict__ R,
+                                                              const double *__restrict__ tab) {
+  extern __shared__ __align__(16) double zf[];  // Re [rows][ZP], then Im [rows][ZP]
+  const int M = s.M, MH = s.MH, Kp = zd64_kp(M), rows = zd64_crows(M);
+  double *zr = zf, *zi = zf + rows * ZP;
   const int b = blockIdx.y, x0 = blockIdx.x * 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const bool xin = x0 + lane < s.N;
-  for (int k8 = warp * 8; k8 < PZ; k8 += nw * 8) {
+  for (int k8 = warp * 8; k8 < rows; k8 += nw * 8) {
     double2 v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
@@ -1166,9 +1188,9 @@ __global__ void __launch_bounds__(256) k_zdft64_inv(Spec s, const double2 *__res
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u)
-      if (k8 + u < PZ) {
-        zr[lane * PZ + k8 + u] = v[u].x;
-        zi[lane * PZ + k8 + u] = v[u].y;
+      if (k8 + u < rows) {
+        zr[(k8 + u) * ZP + lane] = v[u].x;
+        zi[(k8 + u) * ZP + lane] = v[u].y;
       }
   }
   __syncthreads();
@@ -1177,21 +1199,21 @@ __global__ void __launch_bounds__(256) k_zdft64_inv(Spec s, const double2 *__res
   if (p0 >= npairs) return;
   const int g = lane >> 2, q = lane & 3;
   double P[2][4][2] = {}, Q[2][4][2] = {};
-  const double *tcr = tc + (p0 + g) * Kp + q, *tsr = ts + (p0 + g) * Kp + q;
-  double nc[2] = {__ldg(tcr), __ldg(tcr + 8 * Kp)}, ns[2] = {__ldg(tsr), __ldg(tsr + 8 * Kp)};
+  const double2 *tf = zd64_frag(tab, warp, Kp / 4, lane);
+  double2 nc = __ldg(tf), ns = __ldg(tf + 1);
   for (int k0 = 1; k0 <= Kp; k0 += 4) {
     const int k = k0 + q;
-    double ac[2] = {nc[0], nc[1]}, as[2] = {ns[0], ns[1]}, br[4], bi[4];
+    const double ac[2] = {nc.x, nc.y}, as[2] = {ns.x, ns.y};
+    double br[4], bi[4];
     if (k0 + 4 <= Kp) {
-      nc[0] = __ldg(tcr + k0 + 3);
-      nc[1] = __ldg(tcr + 8 * Kp + k0 + 3);
-      ns[0] = __ldg(tsr + k0 + 3);
-      ns[1] = __ldg(tsr + 8 * Kp + k0 + 3);
+      tf += 64;
+      nc = __ldg(tf);
+      ns = __ldg(tf + 1);
     }
 #pragma unroll
     for (int ct = 0; ct < 4; ++ct) {
-      br[ct] = zr[(8 * ct + g) * PZ + k];
-      bi[ct] = zi[(8 * ct + g) * PZ + k];
+      br[ct] = zr[k * ZP + 8 * ct + g];
+      bi[ct] = zi[k * ZP + 8 * ct + g];
     }
 #pragma unroll
     for (int rt = 0; rt < 2; ++rt)
@@ -1214,8 +1236,8 @@ __global__ void __launch_bounds__(256) k_zdft64_inv(Spec s, const double2 *__res
       for (int i = 0; i < 2; ++i) {
         const int x = 8 * ct + 2 * q + i;
         if (x0 + x >= s.N) continue;
-        const double c0 = zr[x * PZ];
-        const double ny = even ? zr[x * PZ + M / 2] : 0.0;
+        const double c0 = zr[x];
+        const double ny = even ? zr[M / 2 * ZP + x] : 0.0;
         const double y = (pp & 1) ? -ny : ny;
         const double pv = P[rt][ct][i], qv = Q[rt][ct][i];
         R[((long long)b * M + pp) * s.rx + x0 + x] = (c0 + 2.0 * (pv - qv) + y) * invM;
@@ -1224,32 +1246,32 @@ __global__ void __launch_bounds__(256) k_zdft64_inv(Spec s, const double2 *__res
   }
 }
 
-// tables tc, ts ([MHp][Kp] each, in that order) of the FP64 z transforms
+// tables of the FP64 z transforms in the lanes' order: [row tile][K step][lane][4]
 void zdft64_tables(const Spec &s, std::vector<double> &t) {
   const int M = s.M, H = (M - 1) / 2, rows = zd64_rows(M), Kp = zd64_kp(M), MH = s.MH;
   t.assign(2 * (size_t)rows * Kp, 0.0);
   for (int r = 0; r < MH && r < rows; ++r)
     for (int k = 1; k <= H; ++k) {
       const double a = 2.0 * M_PI * (double)(((long long)r * k) % M) / (double)M;
-      t[(size_t)r * Kp + (k - 1)] = cos(a);
-      t[(size_t)rows * Kp + (size_t)r * Kp + (k - 1)] = sin(a);
+      const int rt = r / 16, g = r % 8, hi = (r % 16) / 8, ks = (k - 1) / 4, q = (k - 1) % 4;
+      const size_t at = (((size_t)rt * (Kp / 4) + ks) * 32 + 4 * g + q) * 4 + hi;
+      t[at] = cos(a);
+      t[at + 2] = sin(a);
     }
 }
 
 void launch_zdft64(const Spec &s, double *R, double2 *C, const double *tab, int inverse, cudaStream_t st) {
-  const int rows = zd64_rows(s.M), Kp = zd64_kp(s.M);
-  const double *tc = tab, *ts = tab + (size_t)rows * Kp;
+  const int rows = zd64_rows(s.M);
   const dim3 grid((s.N + 31) / 32, s.NM);
   const int threads = 32 * (rows / 16);
   if (!inverse) {
-    const size_t sm = (size_t)32 * zd64_pitch(s.M) * sizeof(double);
+    const size_t sm = (size_t)s.M * ZP * sizeof(double);
     cudaFuncSetAttribute(k_zdft64_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_zdft64_fwd<<<grid, threads, sm, st>>>(s, R, C, tc, ts);
+    k_zdft64_fwd<<<grid, threads, sm, st>>>(s, R, C, tab);
   } else {
-    const int len = Kp + 1 > s.MH ? Kp + 1 : s.MH;
-    const size_t sm = (size_t)2 * 32 * zd64_pitch(len) * sizeof(double);
+    const size_t sm = (size_t)2 * zd64_crows(s.M) * ZP * sizeof(double);
     cudaFuncSetAttribute(k_zdft64_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_zdft64_inv<<<grid, threads, sm, st>>>(s, C, R, tc, ts);
+    k_zdft64_inv<<<grid, threads, sm, st>>>(s, C, R, tab);
   }
 }
 

@@ -110,6 +110,28 @@ def test_projection(gpu, grid):
     s.close()
 
 
+@pytest.mark.parametrize("nx,nz", [(34, 10), (35, 11), (7, 12), (66, 13), (37, 33), (34, 34), (40, 35), (5, 64),
+                                   (67, 65), (34, 96), (36, 193), (35, 194), (34, 255), (69, 256)])
+def test_fp64_z_products(gpu, nx, nz):
+    """FP64 z transforms as MMA products, M = nz-2 = 8 .. 254, odd and even:
+    K ranges that end inside a step of 4 and at its edge (H = 3, 4, 5, 15,
+    16, 31, 47, 95, 126), rows that fill a tile of 16 and one more (M/2+1 =
+    16, 17, 32, 128), columns that end inside a CTA's 32 (N = 3, 5, 33, 67)."""
+    c = noisy_laminar(nx, 6, nz, seed=nz)
+    s = cases.solver_for(c)
+    o = oracle.oracle_for(c)
+    for x in (s, o):
+        x.set_dt(0.02)
+    s.apply_boundary_conditions(1)
+    o.apply_bc(1)
+    s.compute_projection_step(1)
+    o.projection(1)
+    for a, b in zip(s.download_state()[:3], o.state()[:3]):
+        assert rel(a, b) < 1e-12
+    assert rel(s.rhs_p()[:, :, :-1], o.rhs_p()[:, :, :-1]) < 1e-11
+    s.close()
+
+
 @pytest.mark.parametrize("rk", [3, 2, 1])
 def test_steps_small(gpu, rk):
     """5 steps at a fixed dt (CFL < 0) on a grid with nzp = 13 (prime) and
