@@ -646,6 +646,31 @@ __device__ __forceinline__ void dct_pair_out(const T2<T> *res, const T2<T> *post
   }
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// The rows of U, V and W that lines q and q+1 are the first to read, into L2
+// while the CTA fills its tables (the rows at j-1 and k-1 are there from
+// earlier lines).  FP64 only (814 x 257 x 193: 485 -> 445 us per launch, at one
+// CTA of four lines per SM); the FP32 kernels keep enough loads in flight, and
+// there the prefetches cost more than they save (218 -> 246 us).
+template <typename T, bool GROUP>
+__device__ __forceinline__ void prefetch_pair(const Geo &g, const Spec &s, const T *U, const T *V, const T *W, int q,
+                                              const LineGroup<GROUP> &lg) {
+  const int nlines = s.NM * s.M;
+  constexpr int STEP = 128 / (int)sizeof(T);
+  for (int l = 0; l < 2 && q + l < nlines; ++l) {
+    const int b = (q + l) / s.M, k = q + l - b * s.M;
+    const long long c = bidx(g, 2, b + 2, k + 2);
+    for (int i = lg.lane * STEP; i < s.N; i += lg.nl() * STEP) {
+      prefetch_l2(U + c + i);
+      prefetch_l2(V + c + i);
+      prefetch_l2(W + c + i);
+    }
+  }
+}
+
 // FP32 CTAs take up to 16 lines (one CTA fills an SM's shared memory); the
 // FP64 kernels need more registers per thread and stop at 8
 template <typename T> struct DctCta { static constexpr int max_threads = sizeof(T) == 4 ? 512 : 256; };
@@ -665,6 +690,7 @@ __global__ void __launch_bounds__(E::max_threads, E::min_blocks) k_div_dct(Geo g
   // FP32: the reciprocal x spacings of the points, N rounded up to 4
   const int N4 = (N + 3) & ~3;
   float *rfx = reinterpret_cast<float *>(post + N + (size_t)nw * E::dline(N));
+  if (sizeof(T) == 8) prefetch_pair<T>(g, s, U, V, W, (blockIdx.x * nw + line) * 2, lg);
   E::fill(tw, pl, threadIdx.x, blockDim.x);
   for (int t = threadIdx.x; t < N; t += blockDim.x) post[t] = pl.post[t];
   if (sizeof(T) == 4)
@@ -793,8 +819,6 @@ __global__ void __launch_bounds__(TwoPassX<A, B, T>::max_threads, TwoPassX<A, B,
   T2<T> *buf = post + N + (size_t)warp * LINE;
   uint64_t *bar = reinterpret_cast<uint64_t *>(
       reinterpret_cast<unsigned char *>(post + N + (size_t)nw * LINE) + 4 * ((N + 3) / 4 * 4)) + warp;
-  E::fill(tw, pl, threadIdx.x, blockDim.x);
-  for (int t = threadIdx.x; t < N; t += blockDim.x) post[t] = pl.post[t];
   const int nlines = s.NM * s.M;
   const int q = (blockIdx.x * nw + warp) * 2;
   const bool hb = q + 1 < nlines;
@@ -806,6 +830,10 @@ __global__ void __launch_bounds__(TwoPassX<A, B, T>::max_threads, TwoPassX<A, B,
     mbar_expect_tx(bar, bytes);
     bulk_load(buf, R + (long long)q * s.rx, bytes, bar);
   }
+  // the tables while the rows are on their way (114 -> 108 us per launch,
+  // mixed, at 814 x 257 x 193)
+  E::fill(tw, pl, threadIdx.x, blockDim.x);
+  for (int t = threadIdx.x; t < N; t += blockDim.x) post[t] = pl.post[t];
   __syncthreads();
   if (q >= nlines) return;
   if (!__all_sync(0xffffffffu, mbar_wait(bar, 0))) {
