@@ -226,9 +226,70 @@ template <bool GROUP> struct LineGroup {
   }
 };
 
+// The outputs of a prime stage from its folded inputs: a lane takes the
+// outputs k = kg + KG u, u = 0..KB-1, of one butterfly, so each s_q, d_q it
+// reads serves KB table values and the KB chains of sums are independent
+template <typename T, bool INV, int KB, bool GROUP>
+__device__ __forceinline__ void prime_outputs(const T2<T> *a, T2<T> *b, const T2<T> *tw, int n, int R, int nb, int Ns,
+                                              const LineGroup<GROUP> &lg) {
+  static_assert(KB > 0, "outputs per lane");
+  constexpr int UN = KB == 1 ? 4 : 2;
+  const int H = (R - 1) / 2;
+  const int KG = (H + KB) / KB;  // groups covering k = 0..H
+  for (int t = lg.lane; t < nb * KG; t += lg.nl()) {
+    const int jj = t % nb, kg = t / nb;
+    const int jm = jj % Ns;
+    const int idxD = (jj - jm) * R + jm;
+    const T2<T> y0 = a[jj];
+    T ax[KB], ay[KB], bx[KB], by[KB];  // bx, by: sums of d_q times the table's imaginary part (-sin)
+    int m[KB], dk[KB];                 // n (q k mod R) / R, and its increment
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      const int k = kg + KG * u;
+      ax[u] = y0.x;
+      ay[u] = y0.y;
+      bx[u] = by[u] = 0;
+      m[u] = 0;
+      dk[u] = (k <= H ? k : 0) * nb;
+    }
+    const T2<T> *as = a + jj, *ad = a + jj + (R - 1) * nb;
+#pragma unroll UN
+    for (int q = 1; q <= H; ++q) {
+      as += nb;
+      const T2<T> sq = *as, dq = *ad;
+      ad -= nb;
+#pragma unroll
+      for (int u = 0; u < KB; ++u) {
+        m[u] += dk[u];
+        if (m[u] >= n) m[u] -= n;
+        const T2<T> w = tw[m[u]];  // (cos, -sin)(2 pi q k / R)
+        ax[u] += sq.x * w.x;
+        ay[u] += sq.y * w.x;
+        bx[u] += dq.x * w.y;
+        by[u] += dq.y * w.y;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      const int k = kg + KG * u;
+      if (k > H) continue;
+      if (k == 0) {
+        b[idxD] = mk<T>(ax[u], ay[u]);
+      } else if (!INV) {
+        b[idxD + k * Ns] = mk<T>(ax[u] - by[u], ay[u] + bx[u]);
+        b[idxD + (R - k) * Ns] = mk<T>(ax[u] + by[u], ay[u] - bx[u]);
+      } else {
+        b[idxD + k * Ns] = mk<T>(ax[u] + by[u], ay[u] - bx[u]);
+        b[idxD + (R - k) * Ns] = mk<T>(ax[u] - by[u], ay[u] + bx[u]);
+      }
+    }
+  }
+}
+
 // Stockham FFT of one complex line in shared memory by its lane group (no
-// block barriers: stages are separated by the group's)
-template <typename T, bool INV, int MAXR, bool GROUP>
+// block barriers: stages are separated by the group's); KB: outputs per lane
+// of a prime stage above the register butterflies, 0 where N has none
+template <typename T, bool INV, int MAXR, int KB, bool GROUP>
 __device__ __forceinline__ T2<T> *fft_line(T2<T> *a, T2<T> *b, const FftPlan<T> &pl, const T2<T> *tw,
                                            const LineGroup<GROUP> &lg) {
   const int n = pl.n, lane = lg.lane, nl = lg.nl();
@@ -237,7 +298,7 @@ __device__ __forceinline__ T2<T> *fft_line(T2<T> *a, T2<T> *b, const FftPlan<T> 
     const int R = pl.rad[s];
     const int nb = n / R;
     const int tsc = n / (Ns * R);
-    if (!reg_radix<MAXR>(R)) {
+    if constexpr (KB > 0) if (!reg_radix<MAXR>(R)) {
       // a large prime R has few butterflies (nb = n/R), so the lanes take
       // (butterfly, term pair) and (butterfly, output pair) items.  First the
       // inputs of butterfly jj are twiddled (y_q = in_q W_n^{q tstep}) and
@@ -260,59 +321,7 @@ __device__ __forceinline__ T2<T> *fft_line(T2<T> *a, T2<T> *b, const FftPlan<T> 
         a[jj + (R - q) * nb] = sub<T>(y1, y2);
       }
       lg.sync();
-      // a lane takes the outputs k = kg + KG u, u = 0..KB-1, of one butterfly:
-      // each s_q, d_q it reads serves KB table values, and the KB chains of
-      // sums are independent
-      constexpr int KB = 4;
-      const int KG = (H + KB) / KB;  // groups covering k = 0..H
-      for (int t = lane; t < nb * KG; t += nl) {
-        const int jj = t % nb, kg = t / nb;
-        const int jm = jj % Ns;
-        const int idxD = (jj - jm) * R + jm;
-        const T2<T> y0 = a[jj];
-        T ax[KB], ay[KB], bx[KB], by[KB];  // bx, by: sums of d_q times the table's imaginary part (-sin)
-        int m[KB], dk[KB];                 // n (q k mod R) / R, and its increment
-#pragma unroll
-        for (int u = 0; u < KB; ++u) {
-          const int k = kg + KG * u;
-          ax[u] = y0.x;
-          ay[u] = y0.y;
-          bx[u] = by[u] = 0;
-          m[u] = 0;
-          dk[u] = (k <= H ? k : 0) * nb;
-        }
-        const T2<T> *as = a + jj, *ad = a + jj + (R - 1) * nb;
-#pragma unroll 2
-        for (int q = 1; q <= H; ++q) {
-          as += nb;
-          const T2<T> sq = *as, dq = *ad;
-          ad -= nb;
-#pragma unroll
-          for (int u = 0; u < KB; ++u) {
-            m[u] += dk[u];
-            if (m[u] >= n) m[u] -= n;
-            const T2<T> w = tw[m[u]];  // (cos, -sin)(2 pi q k / R)
-            ax[u] += sq.x * w.x;
-            ay[u] += sq.y * w.x;
-            bx[u] += dq.x * w.y;
-            by[u] += dq.y * w.y;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < KB; ++u) {
-          const int k = kg + KG * u;
-          if (k > H) continue;
-          if (k == 0) {
-            b[idxD] = mk<T>(ax[u], ay[u]);
-          } else if (!INV) {
-            b[idxD + k * Ns] = mk<T>(ax[u] - by[u], ay[u] + bx[u]);
-            b[idxD + (R - k) * Ns] = mk<T>(ax[u] + by[u], ay[u] - bx[u]);
-          } else {
-            b[idxD + k * Ns] = mk<T>(ax[u] + by[u], ay[u] - bx[u]);
-            b[idxD + (R - k) * Ns] = mk<T>(ax[u] - by[u], ay[u] + bx[u]);
-          }
-        }
-      }
+      prime_outputs<T, INV, KB, GROUP>(a, b, tw, n, R, nb, Ns, lg);
       lg.sync();
       T2<T> *t = a;
       a = b;
@@ -475,7 +484,7 @@ __device__ __forceinline__ void dft_reg(V (&x)[R]) {
 // FFT engines of the x transforms: the shared-memory twiddle table, the
 // per-line buffer and the transform of one line by one warp (result in
 // natural order).  Stockham: any N, ping-pong buffers of N values.
-template <typename T, int MAXR, bool GROUP = false> struct StockhamX {
+template <typename T, int MAXR, int KB, bool GROUP = false> struct StockhamX {
   static constexpr bool grouped = GROUP;  // several warps per line
   static constexpr int max_threads = sizeof(T) == 4 ? 512 : 256, min_blocks = 0;  // 16 or 8 lines, no bound
   static size_t line(int N) { return 2 * (size_t)N; }
@@ -485,7 +494,7 @@ template <typename T, int MAXR, bool GROUP = false> struct StockhamX {
   }
   template <bool INV>
   __device__ static T2<T> *run(T2<T> *buf, const FftPlan<T> &pl, const T2<T> *tw, const LineGroup<GROUP> &lg) {
-    return fft_line<T, INV, MAXR, GROUP>(buf, buf + pl.n, pl, tw, lg);
+    return fft_line<T, INV, MAXR, KB, GROUP>(buf, buf + pl.n, pl, tw, lg);
   }
 };
 
@@ -1632,9 +1641,35 @@ static int radix_class(const int *rad, int nst) {
 // shared memory and grid
 struct XShape {
   int nw, wpl;
+  int kb;  // outputs per lane of a prime stage above the register butterflies, 0 without one
   size_t sm;
   int grid;
 };
+
+// Outputs per lane of a prime stage (radix R, nb butterflies) that one warp
+// works: of 1, 2 and 4 the fewest rounds of 32 items, weighted by what a round
+// costs (a round of 4 outputs about three of one).  us per launch, forward +
+// inverse, 1 / 2 / 4 outputs:
+//   N =  37 (1 1 1 rounds)  FP64 129x130 53.6 56.9 78.9   mixed 41.6 45.4 53.7
+//   N = 127 (2 1 1)         FP64 129x130  152  142  168   mixed 93.2 87.6  104
+//   N = 254 (4 2 1)         FP64 129x130  262  263  244   mixed  147  137  130
+//   N = 298 (5 3 2)         FP64 129x130  337  340  360   mixed  189  190  218
+//   N = 358 (6 3 2)         FP64 129x130  498  438  438   mixed  251  227  256
+//   N = 397 (7 4 2)         FP64 129x130 1234 1148 1001   mixed  624  598  561
+// (ny x nz after the precision.)  Lines of several warps keep 4.
+static int prime_outputs_per_lane(int R, int nb) {
+  const int H = (R - 1) / 2;
+  int best = 1;
+  double least = 0.0;
+  for (int kb = 1; kb <= 4; kb *= 2) {
+    const double cost = ((nb * ((H + kb) / kb) + 31) / 32) * (kb == 1 ? 1.0 : kb == 2 ? 1.6 : 3.0);
+    if (kb == 1 || cost < least) {
+      best = kb;
+      least = cost;
+    }
+  }
+  return best;
+}
 
 // Lines per CTA and warps per line.  Several warps share a line of the
 // Stockham kernels where a prime stage above the register butterflies makes
@@ -1667,6 +1702,7 @@ static XShape x_shape(const Spec &s, const FftPlan<T> &pl, int nw_req, int split
       x.wpl = 2;
     }
   }
+  x.kb = rmax > 31 ? prime_outputs_per_lane(rmax, s.N / rmax) : 0;
   x.sm = dct_smem_bytes(s.N, sizeof(T), x.nw, split);
   x.grid = ((s.NM * s.M + 1) / 2 + x.nw - 1) / x.nw;
   return x;
@@ -1688,25 +1724,31 @@ static void launch_idct_e(const Geo &g, const Spec &s, const FftPlan<T> &pl, con
   k_idct<T, E><<<x.grid, 32 * x.nw * x.wpl, x.sm, st>>>(g, s, pl, R, p, x.wpl);
 }
 
-// the Stockham kernel of the plan's radix class, several warps per line or one
-#define BLGPU_STOCKHAM(CALL)                                                         \
-  do {                                                                               \
-    if (x.wpl > 1) switch (radix_class(pl.rad, pl.nst)) {                            \
-        case 7: CALL(StockhamX<T BLGPU_C 7 BLGPU_C true>); break;                    \
-        case 13: CALL(StockhamX<T BLGPU_C 13 BLGPU_C true>); break;                  \
-        case 19: CALL(StockhamX<T BLGPU_C 19 BLGPU_C true>); break;                  \
-        case 29: CALL(StockhamX<T BLGPU_C 29 BLGPU_C true>); break;                  \
-        default: CALL(StockhamX<T BLGPU_C 31 BLGPU_C true>); break;                  \
-      }                                                                              \
-    else switch (radix_class(pl.rad, pl.nst)) {                                      \
-        case 7: CALL(StockhamX<T BLGPU_C 7>); break;                                 \
-        case 13: CALL(StockhamX<T BLGPU_C 13>); break;                               \
-        case 19: CALL(StockhamX<T BLGPU_C 19>); break;                               \
-        case 29: CALL(StockhamX<T BLGPU_C 29>); break;                               \
-        default: CALL(StockhamX<T BLGPU_C 31>); break;                               \
-      }                                                                              \
-  } while (0)
-#define BLGPU_C ,
+// calls f with the Stockham engine of the plan's radix class and line shape.
+// One warp per line: the instances of the first class differ in their prime
+// stage (none, or 1, 2 or 4 outputs per lane), which sets their registers
+// (FP64 forward 76, 78, 98 with none, 1 and 4: at N = 126 and 128 a CTA per SM
+// less with it); the other classes hold more for their butterflies, and N with
+// a factor above 7 and a prime above 31 are past 400.
+template <class E> struct XEngine { typedef E type; };
+template <typename T, int MAXR, class F> static void stockham_shape(const XShape &x, F f) {
+  if (x.wpl > 1) return f(XEngine<StockhamX<T, MAXR, 4, true>>());
+  if constexpr (MAXR == 7) {
+    if (x.kb == 0) return f(XEngine<StockhamX<T, MAXR, 0>>());
+    if (x.kb == 1) return f(XEngine<StockhamX<T, MAXR, 1>>());
+    if (x.kb == 2) return f(XEngine<StockhamX<T, MAXR, 2>>());
+  }
+  f(XEngine<StockhamX<T, MAXR, 4>>());
+}
+template <typename T, class F> static void with_stockham(const FftPlan<T> &pl, const XShape &x, F f) {
+  switch (radix_class(pl.rad, pl.nst)) {
+    case 7: return stockham_shape<T, 7>(x, f);
+    case 13: return stockham_shape<T, 13>(x, f);
+    case 19: return stockham_shape<T, 19>(x, f);
+    case 29: return stockham_shape<T, 29>(x, f);
+    default: return stockham_shape<T, 31>(x, f);
+  }
+}
 
 template <typename T>
 void launch_div_dct(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *U, const T *V, const T *W, T *R,
@@ -1723,9 +1765,9 @@ void launch_div_dct(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *
     if (split == 19) return launch_div_dct_e<T, TwoPassX<19, 10>>(g, s, pl, U, V, W, R, x, st);
     if (split == 14) return launch_div_dct_e<T, TwoPassX<14, 9>>(g, s, pl, U, V, W, R, x, st);
   }
-#define BLGPU_FWD(...) launch_div_dct_e<T, __VA_ARGS__>(g, s, pl, U, V, W, R, x, st)
-  BLGPU_STOCKHAM(BLGPU_FWD);
-#undef BLGPU_FWD
+  with_stockham<T>(pl, x, [&](auto e) {
+    launch_div_dct_e<T, typename decltype(e)::type>(g, s, pl, U, V, W, R, x, st);
+  });
 }
 
 template <int A, int B, typename T>
@@ -1762,12 +1804,8 @@ void launch_idct(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *R, 
     if (split == 19) return launch_idct_e<T, TwoPassX<19, 10>>(g, s, pl, R, p, x, st);
     if (split == 14) return launch_idct_e<T, TwoPassX<14, 9>>(g, s, pl, R, p, x, st);
   }
-#define BLGPU_INVT(...) launch_idct_e<T, __VA_ARGS__>(g, s, pl, R, p, x, st)
-  BLGPU_STOCKHAM(BLGPU_INVT);
-#undef BLGPU_INVT
+  with_stockham<T>(pl, x, [&](auto e) { launch_idct_e<T, typename decltype(e)::type>(g, s, pl, R, p, x, st); });
 }
-#undef BLGPU_STOCKHAM
-#undef BLGPU_C
 
 template <typename T, int RK>
 static void launch_dft_z_rk(const Spec &s, const T *R, T2<T> *C, const T2<T> *tz, int inverse, cudaStream_t st) {
