@@ -831,6 +831,15 @@ __global__ void __launch_bounds__(TwoPassX<A, B, T>::max_threads, TwoPassX<A, B,
   const int nlines = s.NM * s.M;
   const int q = (blockIdx.x * nw + warp) * 2;
   const bool hb = q + 1 < nlines;
+  // The tables are filled while the rows are on their way in FP32 and before
+  // the copies start in FP64, whose one CTA of four warps per SM reads them
+  // and the rows faster one after the other (814 x 257 x 193, the other order
+  // first: mixed 114 -> 108, FP64 214 -> 207 us per launch).
+  auto tables = [&] {
+    E::fill(tw, pl, threadIdx.x, blockDim.x);
+    for (int t = threadIdx.x; t < N; t += blockDim.x) post[t] = pl.post[t];
+  };
+  if (sizeof(T) == 8) tables();
   if (lane == 0 && q < nlines) {
     mbar_init(bar, 1);
     mbar_init_fence();
@@ -839,10 +848,7 @@ __global__ void __launch_bounds__(TwoPassX<A, B, T>::max_threads, TwoPassX<A, B,
     mbar_expect_tx(bar, bytes);
     bulk_load(buf, R + (long long)q * s.rx, bytes, bar);
   }
-  // the tables while the rows are on their way (114 -> 108 us per launch,
-  // mixed, at 814 x 257 x 193)
-  E::fill(tw, pl, threadIdx.x, blockDim.x);
-  for (int t = threadIdx.x; t < N; t += blockDim.x) post[t] = pl.post[t];
+  if (sizeof(T) == 4) tables();
   __syncthreads();
   if (q >= nlines) return;
   if (!__all_sync(0xffffffffu, mbar_wait(bar, 0))) {
