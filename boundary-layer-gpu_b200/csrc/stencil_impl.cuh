@@ -1159,17 +1159,18 @@ drain:
 // A thread updates VN = 16/sizeof(T) consecutive
 // points i0..i0+VN-1 (i0 = 2 + VN*q, a 16-byte aligned box position) with
 // 16-byte loads and stores; points outside the update ranges keep their
-// loaded value.
+// loaded value.  SAVE: the first substep's instance, which also writes the
+// pressure and its ghosts; the others do without its code.
 template <typename T> struct V16;
 template <> struct V16<float> { typedef float4 t; };
 template <> struct V16<double> { typedef double2 t; };
 
-template <typename T>
+template <typename T, bool SAVE>
 __global__ void __launch_bounds__(256) k_project_v(Geo g, MetT<T> m, const T *__restrict__ p,
                                                    const double *__restrict__ p0, const float *__restrict__ p0g,
                                                    T *__restrict__ U,
                                                    T *__restrict__ V, T *__restrict__ W, T *__restrict__ P,
-                                                   const Scalars *__restrict__ sc, int save_p) {
+                                                   const Scalars *__restrict__ sc) {
   typedef typename V16<T>::t VT;
   constexpr int VN = 16 / sizeof(T);
   const int i0 = 2 + VN * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -1216,14 +1217,15 @@ __global__ void __launch_bounds__(256) k_project_v(Geo g, MetT<T> m, const T *__
   *reinterpret_cast<VT *>(U + c) = u.v;
   *reinterpret_cast<VT *>(V + c) = v.v;
   *reinterpret_cast<VT *>(W + c) = w.v;
-  if (save_p) {
+  if constexpr (SAVE) {
     const double den = sc->dt * 0.5;  // dt*rk2_coef(1,1)
     Vec q;
+    T px = pc.e[0];  // past the interior: the ghost nxg takes the value at nx
 #pragma unroll
     for (int e = 0; e < VN; ++e) {
-      const int i = min(i0 + e, g.nx);  // past the interior: the ghost nxg takes the value at nx
-      double pv = (double)pc.e[i - i0];
-      if (p0) pv += p0r[min(i - 2, N - 1)];
+      if (i0 + e <= g.nx) px = pc.e[e];
+      double pv = (double)px;
+      if (p0) pv += p0r[min(i0 + e - 2, N - 1)];
       q.e[e] = (i0 + e <= g.nxg) ? (T)(pv / den) : (T)0;
     }
     // The ghosts of projection.f90:78-83: the source copies the x ghosts, then
@@ -2141,7 +2143,8 @@ void launch_project(const Geo &g, const MetT<T> &m, const T *p, const double *p0
   const int ngrp = (g.nx - 1 + VN - 1) / VN;  // i = 2..nx in groups of VN
   const int by = tl.proj_by > 0 ? tl.proj_by : 4;  // 4 rows: the autotuner's choice at 814 x 257 x 193 in both precisions
   dim3 block(32, by), grid((ngrp + 31) / 32, (g.ny - 1 + by - 1) / by, g.nz - 1);
-  k_project_v<T><<<grid, block, 0, st>>>(g, m, p, p0, p0g, U, V, W, P, sc, save_p);
+  if (save_p) k_project_v<T, true><<<grid, block, 0, st>>>(g, m, p, p0, p0g, U, V, W, P, sc);
+  else k_project_v<T, false><<<grid, block, 0, st>>>(g, m, p, p0, p0g, U, V, W, P, sc);
 }
 
 #ifdef BLGPU_STENCIL_PRIMARY
