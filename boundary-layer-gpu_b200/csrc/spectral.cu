@@ -1708,9 +1708,15 @@ static XShape x_shape(const Spec &s, const FftPlan<T> &pl, int nw_req, int split
       x.wpl = 2;
     }
   }
-  x.kb = rmax > 31 ? prime_outputs_per_lane(rmax, s.N / rmax) : 0;
   x.sm = dct_smem_bytes(s.N, sizeof(T), x.nw, split);
   x.grid = ((s.NM * s.M + 1) / 2 + x.nw - 1) / x.nw;
+  x.kb = rmax > 31 ? prime_outputs_per_lane(rmax, s.N / rmax) : 0;
+  // A grid of up to two CTAs per SM has the registers to spare: there the FP64
+  // forward kernel takes the instance with more of them (98 against 76), which
+  // keeps more of its divergence loads in flight (N = 126, 33 x 66: 16.7 ->
+  // 15.1 us per launch; two CTAs of six such warps are what an SM holds, and a
+  // 65 x 64 box, 331 CTAs, takes 25.0 us with it, 17.5 without).
+  if (sizeof(T) == 8 && !inverse && !x.kb && x.grid <= 2 * 148) x.kb = 4;
   return x;
 }
 
