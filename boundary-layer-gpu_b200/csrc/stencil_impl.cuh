@@ -1160,13 +1160,16 @@ drain:
 // points i0..i0+VN-1 (i0 = 2 + VN*q, a 16-byte aligned box position) with
 // 16-byte loads and stores; points outside the update ranges keep their
 // loaded value.  SAVE: the first substep's instance, which also writes the
-// pressure and its ghosts; the others do without its code.
+// pressure and its ghosts; the others do without its code.  The FP64 one is
+// held to 64 registers, an eighth warp per scheduler (71 without: 420 -> 398 us
+// per launch at 814 x 257 x 193, of 338 without the pressure; FP32 takes 54
+// and 259 of 196 us, and loses 8 us by a bound).
 template <typename T> struct V16;
 template <> struct V16<float> { typedef float4 t; };
 template <> struct V16<double> { typedef double2 t; };
 
 template <typename T, bool SAVE>
-__global__ void __launch_bounds__(256) k_project_v(Geo g, MetT<T> m, const T *__restrict__ p,
+__global__ void __launch_bounds__(256, SAVE && sizeof(T) == 8 ? 4 : 0) k_project_v(Geo g, MetT<T> m, const T *__restrict__ p,
                                                    const double *__restrict__ p0, const float *__restrict__ p0g,
                                                    T *__restrict__ U,
                                                    T *__restrict__ V, T *__restrict__ W, T *__restrict__ P,
