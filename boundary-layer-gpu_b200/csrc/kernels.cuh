@@ -18,7 +18,7 @@ template <typename T> struct MetT {
 // Launch shapes of the main kernels.  0 selects the built-in choice; the
 // autotuner (blgpu_autotune) searches these per box.
 struct Tiles {
-  int rhs_kc;   // k-planes walked by one CTA of the RHS kernel (0: 8 to 32 by kernel, fewer in small boxes, rhs_chunk)
+  int rhs_kc;   // k-planes walked by one CTA of the RHS kernel (0: 8 to 32 by kernel, fewer in small boxes, z_chunk)
   int rhs_by;   // RHS block is 32 x rhs_by threads (0: 8)
   int dct_nw;   // complex lines (warps) per CTA of the forward DCT, up to 16 in FP32 (8 two-pass) and 8 in FP64 (0: built-in)
   int dftz_rk;  // z wavenumbers per warp in the z-DFT, 4 or 8 (0: 8)

@@ -1957,13 +1957,19 @@ __global__ void __launch_bounds__(256) k_law_of_wall(Geo g, const T *__restrict_
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-// Built-in chunk of k-planes of an RHS kernel whose CTAs cover `tiles` x-y
-// tiles: kc, halved while the grid would hold fewer than 200 CTAs.  A chunk's
-// two extra planes cost little next to SMs without a CTA: per launch at
-// 128 x 64 x 32 (16 x-y tiles) 20.8 us with 16 planes, 10.6 with 2 (mixed),
-// 31.7 and 14.7 (FP64); at 256 x 65 x 96 (32 tiles, 192 CTAs) 8 and 16 planes
-// tie (26.9, 26.7), and at 301 x 98 x 75 (65 tiles) shorter chunks lose.
-static inline int rhs_chunk(int kc, int tiles, int nk) {
+// Built-in chunk of k-planes of a kernel whose CTAs cover `tiles` x-y tiles
+// and walk up in z: kc, halved while the grid would hold fewer than 200 CTAs.
+// A chunk's two extra planes cost little next to SMs without a CTA.  RHS, us
+// per launch by planes per CTA (2 4 8 16), the rule's choice first:
+//   128 x 64 x 32   FP64  2: 14.6 14.3 19.9 30.8   mixed  2: 10.4 11.2 14.6 21.3
+//   128 x 65 x 64   FP64  4: 22.9 21.1 20.7 32.4   mixed  4: 14.0 12.6 14.6 20.9
+//   256 x 65 x 96   FP64  8: 57.5 53.0 52.4 62.6   mixed  8: 30.2 26.8 26.3 26.8
+//   301 x 98 x 75   FP64 16: 82.2 73.8 71.0 77.2   mixed 16: 40.4 35.0 31.4 33.4
+//   512 x 128 x 128 FP64 16:  252  224  211  215   mixed 16:  115 96.4 88.5 87.1
+// Smagorinsky viscosity, us per launch with 16 planes -> the rule's (one a
+// thread at 64 x 32 x 32, four at 128 x 65 x 64): FP64 14.9 -> 3.5 and
+// 16.1 -> 11.5, mixed 10.9 -> 2.9 and 11.6 -> 8.4.
+static inline int z_chunk(int kc, int tiles, int nk) {
   while (kc > 1 && tiles * ((nk + kc - 1) / kc) < 200) kc /= 2;
   return kc;
 }
@@ -2046,7 +2052,7 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
   // chunk for kernels of 32 threads x rows with pts points per thread
   auto chunk = [&](int kc, int pts, int rows) {
     const int nx = pts == 2 ? g.nx / 2 : g.nx - 1;
-    return tl.rhs_kc > 0 ? tl.rhs_kc : rhs_chunk(kc, (nx + 31) / 32 * ((g.ny - 1 + rows - 1) / rows), g.nz - 1);
+    return tl.rhs_kc > 0 ? tl.rhs_kc : z_chunk(kc, (nx + 31) / 32 * ((g.ny - 1 + rows - 1) / rows), g.nz - 1);
   };
   const int kchunk = chunk(8, 1, by);
   dim3 grid = vol_grid(g.nx - 1, g.ny - 1, g.nz - 1, kchunk, by), block(32, by);
@@ -2203,7 +2209,7 @@ void launch_maxdiv(const Geo &g, const T *U, const T *V, const T *W, unsigned lo
 template <typename T>
 void launch_smagorinsky(const Geo &g, const MetT<T> &m, const T *U, const T *V, const T *W, const double *cs2, T *nut,
                         cudaStream_t st) {
-  const int kchunk = 16;
+  const int kchunk = z_chunk(16, (g.nxg - 2 + 31) / 32 * ((g.nyg - 2 + 7) / 8), g.nzg - 2);
   k_smagorinsky<T><<<vol_grid(g.nxg - 2, g.nyg - 2, g.nzg - 2, kchunk), dim3(32, 8), 0, st>>>(g, m, U, V, W, cs2, nut,
                                                                                            kchunk);
 }
