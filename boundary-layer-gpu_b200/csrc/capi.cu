@@ -67,6 +67,7 @@ struct blgpu_ctx {
   ThomasMaps tmaps{};         // TMA maps of C and the pivots for the tiled y-solve
   RhsMaps rmaps[5]{};         // TMA maps of U, V, W of each state buffer, of F1 and of nu_t (TMA-fed RHS)
   bool have_rmaps = false;
+  int boxes = 1;              // boxes whose steps the graph being captured runs side by side (ensembles)
   CufftPath *cf = nullptr;    // poisson = BLGPU_POISSON_CUFFT: plans and work arrays
   int cf_status = 0;          // first failing cufftExec status of an enqueued step (0: none)
   int wait_limit = -1;        // mbarrier polls of the tiled y-solve and the TMA-fed RHS (< 0: built-in), a test hook
@@ -1136,7 +1137,9 @@ static void enq_rhs(blgpu_ctx *ctx, int mode, int in, int o, int outb, double c1
   launch_rhs_rk<T>(ctx->geo, m, mode, ctx->cfg.les_model != 0, Si[0], Si[1], Si[2], (const T *)ctx->nut, So[0], So[1],
                    So[2], F[0], F[1], F[2], Sn[0], Sn[1], Sn[2], ctx->sc, c1, c2, ctx->tiles,
                    ctx->have_rmaps ? &ctx->rmaps[in] : nullptr, ctx->have_rmaps ? &ctx->rmaps[o] : nullptr,
-                   ctx->have_rmaps ? &ctx->rmaps[3] : nullptr, ctx->have_rmaps && ctx->nut ? &ctx->rmaps[4] : nullptr, &ctx->sc->err, ctx->wait_limit, ctx->st);
+                   ctx->have_rmaps ? &ctx->rmaps[3] : nullptr,
+                   ctx->have_rmaps && ctx->nut ? &ctx->rmaps[4] : nullptr, ctx->boxes, &ctx->sc->err, ctx->wait_limit,
+                   ctx->st);
   ph_end(ctx, 1);
 }
 
@@ -1176,7 +1179,8 @@ static int enq_step(blgpu_ctx *ctx, int a, bool with_dt) {
     if (ctx->cfg.les_model == 1) {  // Smagorinsky from the substep's state (time_integration.f90:341-346)
       T **Si = reinterpret_cast<T **>(ctx->S[in]);
       ph_begin(ctx, PH_MISC);
-      launch_smagorinsky<T>(ctx->geo, met<T>(ctx), Si[0], Si[1], Si[2], ctx->d_cs2, (T *)ctx->nut, ctx->st);
+      launch_smagorinsky<T>(ctx->geo, met<T>(ctx), Si[0], Si[1], Si[2], ctx->d_cs2, (T *)ctx->nut, ctx->boxes,
+                            ctx->st);
       ph_end(ctx, 1);
     } else if (ctx->dyn) {  // dynamic Smagorinsky, same place (LES = 2, 3)
       T **Si = reinterpret_cast<T **>(ctx->S[in]);
@@ -1494,14 +1498,14 @@ int blgpu_eddy_viscosity(blgpu_ctx *ctx) {
       ctx->launches += launch_dyn_smagorinsky<double>(ctx->geo, S[0], S[1], S[2], ctx->dyn, ctx->cfg.les_model,
                                                       (double *)ctx->nut, ctx->st);
     else
-      launch_smagorinsky<double>(ctx->geo, ctx->m64, S[0], S[1], S[2], ctx->d_cs2, (double *)ctx->nut, ctx->st);
+      launch_smagorinsky<double>(ctx->geo, ctx->m64, S[0], S[1], S[2], ctx->d_cs2, (double *)ctx->nut, 1, ctx->st);
   } else {
     float **S = reinterpret_cast<float **>(ctx->S[ctx->cur]);
     if (ctx->dyn)
       ctx->launches += launch_dyn_smagorinsky<float>(ctx->geo, S[0], S[1], S[2], ctx->dyn, ctx->cfg.les_model,
                                                      (float *)ctx->nut, ctx->st);
     else
-      launch_smagorinsky<float>(ctx->geo, ctx->m32, S[0], S[1], S[2], ctx->d_cs2, (float *)ctx->nut, ctx->st);
+      launch_smagorinsky<float>(ctx->geo, ctx->m32, S[0], S[1], S[2], ctx->d_cs2, (float *)ctx->nut, 1, ctx->st);
   }
   if (!ctx->dyn) ctx->launches += 1;
   CK(cudaGetLastError());
@@ -1948,7 +1952,9 @@ static int ens_capture(blgpu_ensemble *e, int a) {
     blgpu_ctx *ctx = e->box[b];
     cudaStreamWaitEvent(ctx->st, e->fork, 0);
     const long long l0 = ctx->launches;
+    ctx->boxes = (int)e->box.size();
     e->next[a][b] = ctx->fp64 ? enq_step<double>(ctx, a, true) : enq_step<float>(ctx, a, true);
+    ctx->boxes = 1;
     nl += ctx->launches - l0;
     ctx->launches = l0;
     cudaEventRecord(e->join[b], ctx->st);

@@ -75,12 +75,13 @@ template <typename T> bool rhs_maps(const Geo &g, bool one_point, const T *const
 // mi, mo, mf, mn: tensor maps of the buffers of U V W, Uo Vo Wo, F1 and nu_t (the
 // TMA-fed DNS kernels: FP32 with rhs_pts 0 or 4, FP64 with rhs_pts 4; the LES kernel unless rhs_pts 1), or null; err: device flag, bit 64 set when a plane
 // copy missed its wait limit; wait_limit: mbarrier polls before giving up
-// (< 0: the built-in limit)
+// (< 0: the built-in limit); boxes: boxes whose steps run side by side
+// (launch shape only)
 template <typename T>
 void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *U, const T *V, const T *W,
                    const T *nut, const T *Uo, const T *Vo, const T *Wo, T *F1u, T *F1v, T *F1w, T *Un, T *Vn, T *Wn,
                    const Scalars *sc, double c1, double c2, const Tiles &tl, const RhsMaps *mi, const RhsMaps *mo,
-                   const RhsMaps *mf, const RhsMaps *mn, int *err, int wait_limit, cudaStream_t st);
+                   const RhsMaps *mf, const RhsMaps *mn, int boxes, int *err, int wait_limit, cudaStream_t st);
 template <typename T>
 void launch_project(const Geo &g, const MetT<T> &m, const T *p, const double *p0, const float *p0g, T *U, T *V,
                     T *W, T *P,
@@ -99,7 +100,7 @@ void launch_maxdiv(const Geo &g, const T *U, const T *V, const T *W, unsigned lo
 
 template <typename T>
 void launch_smagorinsky(const Geo &g, const MetT<T> &m, const T *U, const T *V, const T *W, const double *cs2, T *nut,
-                        cudaStream_t st);
+                        int boxes, cudaStream_t st);
 // dynamic Smagorinsky (LES = 2 z-averaged, 3 pointwise), FP64 on dense work arrays;
 // returns the number of kernels launched
 size_t dyn_smagorinsky_work_bytes(int nxg, int nyg, int nzg);

@@ -1958,8 +1958,11 @@ __global__ void __launch_bounds__(256) k_law_of_wall(Geo g, const T *__restrict_
 // launchers
 // ---------------------------------------------------------------------------
 // Built-in chunk of k-planes of a kernel whose CTAs cover `tiles` x-y tiles
-// and walk up in z: kc, halved while the grid would hold fewer than 200 CTAs.
-// A chunk's two extra planes cost little next to SMs without a CTA.  RHS, us
+// and walk up in z: kc, halved while the grids of the boxes that run side by
+// side (an ensemble's) would hold fewer than 200 CTAs.  A chunk's two extra
+// planes cost little next to SMs without a CTA, and are lost where other boxes
+// fill them: with each box counted alone 16 boxes of 128..256 x 65 x 64..96
+// took 4.18 ms per step (now 4.13), 64 boxes 16.26 (15.85), mixed.  RHS of a box alone, us
 // per launch by planes per CTA (2 4 8 16), the rule's choice first:
 //   128 x 64 x 32   FP64  2: 14.6 14.3 19.9 30.8   mixed  2: 10.4 11.2 14.6 21.3
 //   128 x 65 x 64   FP64  4: 22.9 21.1 20.7 32.4   mixed  4: 14.0 12.6 14.6 20.9
@@ -1967,10 +1970,10 @@ __global__ void __launch_bounds__(256) k_law_of_wall(Geo g, const T *__restrict_
 //   301 x 98 x 75   FP64 16: 82.2 73.8 71.0 77.2   mixed 16: 40.4 35.0 31.4 33.4
 //   512 x 128 x 128 FP64 16:  252  224  211  215   mixed 16:  115 96.4 88.5 87.1
 // Smagorinsky viscosity, us per launch with 16 planes -> the rule's (one a
-// thread at 64 x 32 x 32, four at 128 x 65 x 64): FP64 14.9 -> 3.5 and
+// thread at 64 x 32 x 32, eight at 128 x 65 x 64): FP64 14.9 -> 3.5 and
 // 16.1 -> 11.5, mixed 10.9 -> 2.9 and 11.6 -> 8.4.
-static inline int z_chunk(int kc, int tiles, int nk) {
-  while (kc > 1 && tiles * ((nk + kc - 1) / kc) < 200) kc /= 2;
+static inline int z_chunk(int kc, int tiles, int nk, int boxes) {
+  while (kc > 1 && (long long)boxes * tiles * ((nk + kc - 1) / kc) < 200) kc /= 2;
   return kc;
 }
 
@@ -2047,12 +2050,13 @@ template <typename T>
 void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *U, const T *V, const T *W,
                    const T *nut, const T *Uo, const T *Vo, const T *Wo, T *F1u, T *F1v, T *F1w, T *Un, T *Vn, T *Wn,
                    const Scalars *sc, double c1, double c2, const Tiles &tl, const RhsMaps *mi, const RhsMaps *mo,
-                   const RhsMaps *mf, const RhsMaps *mn, int *err, int wait_limit, cudaStream_t st) {
+                   const RhsMaps *mf, const RhsMaps *mn, int boxes, int *err, int wait_limit, cudaStream_t st) {
   const int by = tl.rhs_by > 0 ? tl.rhs_by : 8;
   // chunk for kernels of 32 threads x rows with pts points per thread
   auto chunk = [&](int kc, int pts, int rows) {
     const int nx = pts == 2 ? g.nx / 2 : g.nx - 1;
-    return tl.rhs_kc > 0 ? tl.rhs_kc : z_chunk(kc, (nx + 31) / 32 * ((g.ny - 1 + rows - 1) / rows), g.nz - 1);
+    return tl.rhs_kc > 0 ? tl.rhs_kc
+                         : z_chunk(kc, (nx + 31) / 32 * ((g.ny - 1 + rows - 1) / rows), g.nz - 1, boxes);
   };
   const int kchunk = chunk(8, 1, by);
   dim3 grid = vol_grid(g.nx - 1, g.ny - 1, g.nz - 1, kchunk, by), block(32, by);
@@ -2208,8 +2212,8 @@ void launch_maxdiv(const Geo &g, const T *U, const T *V, const T *W, unsigned lo
 
 template <typename T>
 void launch_smagorinsky(const Geo &g, const MetT<T> &m, const T *U, const T *V, const T *W, const double *cs2, T *nut,
-                        cudaStream_t st) {
-  const int kchunk = z_chunk(16, (g.nxg - 2 + 31) / 32 * ((g.nyg - 2 + 7) / 8), g.nzg - 2);
+                        int boxes, cudaStream_t st) {
+  const int kchunk = z_chunk(16, (g.nxg - 2 + 31) / 32 * ((g.nyg - 2 + 7) / 8), g.nzg - 2, boxes);
   k_smagorinsky<T><<<vol_grid(g.nxg - 2, g.nyg - 2, g.nzg - 2, kchunk), dim3(32, 8), 0, st>>>(g, m, U, V, W, cs2, nut,
                                                                                            kchunk);
 }
@@ -2230,7 +2234,7 @@ void launch_law_of_wall(const Geo &g, const T *U, double *utau, int *iters, int 
   template void launch_rhs_rk<T>(const Geo &, const MetT<T> &, int, bool, const T *, const T *, const T *,          \
                                  const T *, const T *, const T *, const T *, T *, T *, T *, T *, T *, T *,          \
                                  const Scalars *, double, double, const Tiles &, const RhsMaps *, const RhsMaps *,  \
-                                 const RhsMaps *, const RhsMaps *, int *, int, cudaStream_t);                        \
+                                 const RhsMaps *, const RhsMaps *, int, int *, int, cudaStream_t);                   \
   template void launch_project<T>(const Geo &, const MetT<T> &, const T *, const double *, const float *, T *,    \
                                   T *, T *, T *,                                                                    \
                                   const Scalars *, int, const Tiles &, cudaStream_t);                               \
@@ -2240,7 +2244,7 @@ void launch_law_of_wall(const Geo &g, const T *U, double *utau, int *iters, int 
                              cudaStream_t);                                                                         \
   template void launch_maxdiv<T>(const Geo &, const T *, const T *, const T *, unsigned long long *, cudaStream_t); \
   template void launch_smagorinsky<T>(const Geo &, const MetT<T> &, const T *, const T *, const T *, const double *, T *, \
-                                      cudaStream_t);                                                                \
+                                      int, cudaStream_t);                                                           \
   template void launch_stats<T>(const Geo &, const T *, const T *, const T *, const T *, const T *, double *,       \
                                 cudaStream_t);                                                                      \
   template void launch_law_of_wall<T>(const Geo &, const T *, double *, int *, int, cudaStream_t);
