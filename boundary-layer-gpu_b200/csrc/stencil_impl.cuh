@@ -1836,6 +1836,14 @@ template <typename T> struct LdT {
   __device__ __forceinline__ T w(int s, int dj, int k) const { return at(W, s, dj, k); }
 };
 
+// The NaN of a column o[k plane] formed again by divisions (strain_divided)
+template <typename T>
+__device__ __noinline__ void smagorinsky_nan(LdT<T> ld, const T *xF, const T *xC, const T *yF, const T *yC,
+                                             const T *zF, const T *zC, int i, int j, int k0, int k1, T c2, T *o) {
+  for (int k = k0; k <= k1; ++k)
+    if (o[k * ld.pl] != o[k * ld.pl]) o[k * ld.pl] = c2 * strain_divided<T>(ld, xF, xC, yF, yC, zF, zC, i, j, k);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_smagorinsky(Geo g, MetT<T> m, const T *__restrict__ U,
                                                      const T *__restrict__ V, const T *__restrict__ W,
@@ -1847,12 +1855,15 @@ __global__ void __launch_bounds__(256) k_smagorinsky(Geo g, MetT<T> m, const T *
   const LdT<T> ld{U, V, W, bidx(g, i - 1, j, 0), g.px, g.plane, g.nz};
   StrainColumn<T, LdT<T>> col(ld, m.xF, m.xrF, m.xC, m.xrC, m.yF, m.yrF, m.yC, m.yrC, m.zF, m.zrF, m.zC, m.zrC, i, j);
   const T c2 = (T)cs2[j];
+  bool nan = false;
   col.start(k0);
   for (int k = k0; k <= k1; ++k) {
     T s[6];
     const T n = col.cell(k, s);
     nut[bidx(g, i, j, k)] = c2 * n;
+    nan |= n != n;
   }
+  if (nan) smagorinsky_nan<T>(ld, m.xF, m.xC, m.yF, m.yC, m.zF, m.zC, i, j, k0, k1, c2, nut + bidx(g, i, j, 0));
 }
 
 // ---------------------------------------------------------------------------

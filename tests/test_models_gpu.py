@@ -62,6 +62,36 @@ def test_smagorinsky_tile_edges(gpu, grid):
         s.close()
 
 
+def test_smagorinsky_of_infinite_quotients(gpu):
+    """A state near overflow, as a run leaves it that has blown up: where the
+    source's quotient (u_a - u_b)/dx is an infinity the viscosity is one too,
+    not a NaN, and the cells whose corner averages add infinities of both signs
+    hold NaN as the source's do.  The large velocities overflow over every
+    spacing (all below 0.8) in the precision at hand: 1.7e308 in FP64 and 3e38
+    in FP32, whose other cells match to FP32's range."""
+    grid = (12, 9, 14)
+    c = cases.laminar_case(nx=grid[0], ny=grid[1], nz=grid[2], lx=5.0, ly=3.0, lz=5.0)
+    assert max(np.diff(a).max() for a in (c.x, c.y, c.z)) < 0.8
+
+    def state(big):
+        d = cases.laminar_case(nx=grid[0], ny=grid[1], nz=grid[2], lx=5.0, ly=3.0, lz=5.0)
+        d.U[4, 4, 4] = big
+        d.V[8, 3, 9] = -big
+        d.W[3, 6, 10] = big
+        return d
+
+    inner = (slice(1, -1), slice(1, -1), slice(1, -1))
+    ref = oracle.oracle_for(state(1.7e308)).smagorinsky()[inner]
+    assert np.isinf(ref).sum() > 10 and np.isnan(ref).any() and np.isfinite(ref).sum() > 500
+    for prec, big in ((FP64, 1.7e308), (MIXED, 3e38)):
+        s = cases.solver_for(state(big), precision=prec, les_model=1)
+        nut = s.compute_eddy_viscosity()[inner]
+        assert np.array_equal(np.isinf(nut), np.isinf(ref)) and np.array_equal(np.isnan(nut), np.isnan(ref))
+        ok = np.isfinite(ref)
+        assert np.abs(nut[ok] - ref[ok]).max() <= (1e-14 if prec == FP64 else 1e-5) * np.abs(ref[ok]).max()
+        s.close()
+
+
 def test_les_steps_match_oracle(gpu):
     c = noisy(40, 13, 18, seed=22, amp=2e-3, cfl=-2e-3)
     s = cases.solver_for(c, les_model=1)
