@@ -8,7 +8,8 @@
 // and so are the velocities of plane k+1, so a cell costs 17 loads and 19
 // quotients where its 12 edges taken one by one cost 48 and 24.
 // Every quotient is the source's a/b formed by Markstein's correction from
-// the tabulated reciprocal (mdiv, common.cuh).
+// the tabulated reciprocal (mdiv, common.cuh): RN(a/b) in FP64, within
+// (1/2 + 2^-20) ulp of a/b in FP32.
 //
 // LD supplies the velocities as R: u(s, dj, k) is U(i-1+s, j+dj, k), s = 0, 1;
 // v(s, dj, k) is V(i-1+s, j+dj, k), s = 0..2; w(s, dj, k) is W(i-1+s, j+dj, k),
@@ -20,7 +21,9 @@
 
 namespace blgpu {
 
-// the FP32 form of mdiv: RN(a/b) from rb = RN(1/b), three instructions
+// the FP32 form of mdiv, three instructions.  b and rb are the FP64 spacing
+// and its reciprocal, each rounded to FP32, so rb is within 2^-23 of 1/b but
+// not its rounding: the result is RN(a/b + e), |e| < 2^-20 ulp
 __device__ __forceinline__ float mdiv(float a, float b, float rb) {
   const float q = __fmul_rn(a, rb);
   return __fmaf_rn(__fmaf_rn(-q, b, a), rb, q);
