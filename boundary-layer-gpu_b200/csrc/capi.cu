@@ -1035,6 +1035,34 @@ template <typename T> static const MetT<T> &met(const blgpu_ctx *ctx) {
   return *reinterpret_cast<const MetT<T> *>(ctx->fp64 ? (const void *)&ctx->m64 : (const void *)&ctx->m32);
 }
 
+// The z transforms that launch shapes t select: tcgen05 (zdft 0 or 3),
+// mma.sync TF32 (0 without tcgen05, or 2), FP64 MMA products, FP32 products
+// (M/2+1 > 96; zdft 1 selects the direct sums as far as their columns fit
+// shared memory), direct sums.
+enum ZForm { Z_UMMA, Z_MMA, Z_DMMA, Z_PRODUCTS, Z_SUMS };
+static ZForm z_form(const blgpu_ctx *ctx, const Tiles &t) {
+  if (ctx->utab && (t.zdft == 0 || t.zdft == 3)) return Z_UMMA;
+  if (ctx->zfrag && (t.zdft == 0 || t.zdft == 2)) return Z_MMA;
+  if (ctx->ztab64) return Z_DMMA;
+  if (ctx->ztab32 && !(t.zdft == 1 && dft_z_serves(ctx->spec))) return Z_PRODUCTS;
+  return Z_SUMS;
+}
+
+template <typename T> static void enq_dft_z(blgpu_ctx *ctx, int inverse) {
+  typedef typename vec2<T>::type T2;
+  const Spec &s = ctx->spec;
+  float *R = (float *)ctx->R;
+  float2 *C = (float2 *)ctx->C;
+  switch (z_form(ctx, ctx->tiles)) {
+    case Z_UMMA: launch_zdft_umma(s, ctx->umaps, R, C, ctx->utab, inverse, ctx->nsm, &ctx->sc->err, ctx->st); break;
+    case Z_MMA: launch_zdft_tc(s, ctx->zmaps, R, C, ctx->zfrag, inverse, ctx->nsm, &ctx->sc->err, ctx->st); break;
+    case Z_DMMA: launch_zdft64(s, (double *)ctx->R, (double2 *)ctx->C, (const double *)ctx->ztab64, inverse, ctx->st); break;
+    case Z_PRODUCTS: launch_zsum(s, R, C, ctx->ztab32, inverse, ctx->st); break;
+    default:
+      launch_dft_z<T>(s, (T *)ctx->R, (T2 *)ctx->C, (const T2 *)ctx->ztab, inverse, ctx->tiles.dftz_rk, ctx->st);
+  }
+}
+
 template <typename T>
 static void enq_bc(blgpu_ctx *ctx, int b, int o, int rk_step, double tc = -1.0, bool save_to = false) {
   T **S = reinterpret_cast<T **>(ctx->S[b]);
@@ -1081,17 +1109,8 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
   ph_begin(ctx, PH_DIVDCT);
   launch_div_dct<T>(ctx->geo, s, pl, S[0], S[1], S[2], (T *)ctx->R, ctx->tiles.dct_nw, ctx->tiles.xfft, ctx->st);
   ph_end(ctx, 1);
-  // z transforms: tcgen05 (zdft 0 or 3), mma.sync TF32 (0 without tcgen05, or 2), FP32 products
-  // (M/2+1 > 96), FP32/FP64 sums (1)
-  const int zd = ctx->tiles.zdft;
-  const bool um = mixed && ctx->utab && (zd == 0 || zd == 3);
-  const bool tc = mixed && !um && ctx->zfrag && (zd == 0 || zd == 2);
   ph_begin(ctx, PH_DFTZ);
-  if (um) launch_zdft_umma(s, ctx->umaps, (float *)ctx->R, (float2 *)ctx->C, ctx->utab, 0, ctx->nsm, &ctx->sc->err, ctx->st);
-  else if (tc) launch_zdft_tc(s, ctx->zmaps, (float *)ctx->R, (float2 *)ctx->C, ctx->zfrag, 0, ctx->nsm, &ctx->sc->err, ctx->st);
-  else if (ctx->ztab64) launch_zdft64(s, (double *)ctx->R, (double2 *)ctx->C, (const double *)ctx->ztab64, 0, ctx->st);
-  else if (ctx->ztab32) launch_zsum(s, (float *)ctx->R, (float2 *)ctx->C, ctx->ztab32, 0, ctx->st);
-  else launch_dft_z<T>(s, (T *)ctx->R, (T2 *)ctx->C, (const T2 *)ctx->ztab, 0, ctx->tiles.dftz_rk, ctx->st);
+  enq_dft_z<T>(ctx, 0);
   ph_end(ctx, 1);
   const double *sp = ctx->d_spec;
   ph_begin(ctx, PH_THOMAS);
@@ -1108,11 +1127,7 @@ static void enq_projection(blgpu_ctx *ctx, int b, int rk_step) {
     launch_kz0_idct(s, ctx->kz0h, ctx->klow, ctx->cmat, ctx->kz0, ctx->kz0g, ctx->st);
   ph_end(ctx, mixed ? 2 : 1);
   ph_begin(ctx, PH_IDFTZ);
-  if (um) launch_zdft_umma(s, ctx->umaps, (float *)ctx->R, (float2 *)ctx->C, ctx->utab, 1, ctx->nsm, &ctx->sc->err, ctx->st);
-  else if (tc) launch_zdft_tc(s, ctx->zmaps, (float *)ctx->R, (float2 *)ctx->C, ctx->zfrag, 1, ctx->nsm, &ctx->sc->err, ctx->st);
-  else if (ctx->ztab64) launch_zdft64(s, (double *)ctx->R, (double2 *)ctx->C, (const double *)ctx->ztab64, 1, ctx->st);
-  else if (ctx->ztab32) launch_zsum(s, (float *)ctx->R, (float2 *)ctx->C, ctx->ztab32, 1, ctx->st);
-  else launch_dft_z<T>(s, (T *)ctx->R, (T2 *)ctx->C, (const T2 *)ctx->ztab, 1, ctx->tiles.dftz_rk, ctx->st);
+  enq_dft_z<T>(ctx, 1);
   ph_end(ctx, 1);
   ph_begin(ctx, PH_IDCT);
   launch_idct<T>(ctx->geo, s, pl, (const T *)ctx->R, (T *)ctx->rhs_p, ctx->tiles.idct_nw, ctx->tiles.xfft,

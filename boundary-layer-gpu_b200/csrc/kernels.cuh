@@ -144,6 +144,7 @@ void launch_div_dct(const Geo &g, const Spec &s, const FftPlan<T> &pl, const T *
 template <typename T>
 void launch_dft_z(const Spec &s, const T *R, typename vec2<T>::type *C, const typename vec2<T>::type *ztab, int inverse,
                   int rk, cudaStream_t st);
+bool dft_z_serves(const Spec &s);  // the columns of the direct sums fit shared memory (M <= 453, either precision)
 // FP64 z transforms on the FP64 tensor-core MMA (8 <= M <= 254): the host
 // tables (cos, then sin, [rows][Kp] each) and the forward / inverse launch
 void zdft64_tables(const Spec &s, std::vector<double> &t);
@@ -184,7 +185,7 @@ bool zdft_tc_maps(const Spec &s, float *R, float2 *C, ZdftMaps *out);
 void launch_zdft_tc(const Spec &s, const ZdftMaps &maps, float *R, float2 *C, const uint32_t *frag, int inverse,
                     int nsm, int *err, cudaStream_t st);
 // ---- zsum.cu: the mixed form's z transforms as FP32 products, M/2+1 > 96 ----
-bool zsum_serves(const Spec &s);  // M/2+1 > 96 and its columns fit shared memory (M up to about 770)
+bool zsum_serves(const Spec &s);  // M/2+1 > 96 and its columns fit shared memory (M <= 767)
 void zsum_tables(const Spec &s, std::vector<float> &t);
 void launch_zsum(const Spec &s, float *R, float2 *C, const float *tab, int inverse, cudaStream_t st);
 // ---- cufft_path.cu: the cuFFT comparison path (solve_poisson_gpu with cuFFT plans) ----

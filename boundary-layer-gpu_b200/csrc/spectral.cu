@@ -1838,6 +1838,9 @@ static void launch_dft_z_rk(const Spec &s, const T *R, T2<T> *C, const T2<T> *tz
   }
 }
 
+// the forward holds M x 512 bytes of columns, the inverse (M/2+1) x 1024
+bool dft_z_serves(const Spec &s) { return s.M * 512 <= 227 * 1024 && s.MH * 1024 <= 227 * 1024; }
+
 template <typename T>
 void launch_dft_z(const Spec &s, const T *R, T2<T> *C, const T2<T> *tz, int inverse, int rk, cudaStream_t st) {
   if (rk == 4) launch_dft_z_rk<T, 4>(s, R, C, tz, inverse, st);

@@ -250,9 +250,10 @@ int blgpu_check_divergence_noalloc(const double *U, const double *V, const doubl
  * block 32 x rhs_by), dct_nw (complex lines per CTA of the forward DCT, up
  * to 16 in the mixed form (8 with the two-pass x transforms) and 8 in FP64),
  * dftz_rk (z wavenumbers per warp of the z-DFT, 4 or 8), proj_by (projection
- * block 32 x proj_by), zdft (mixed form, where M/2+1 <= 96: 1 = FP32 direct
- * sums, 2 = mma.sync TF32 tensor cores, 3 = tcgen05 tensor cores with the
- * accumulators in tensor memory), rhs_pts (mixed-form DNS RHS: 1 = one
+ * block 32 x proj_by), zdft (mixed form: 1 = FP32 direct sums, M = nz-2 up
+ * to 453; where M/2+1 <= 96 2 = mma.sync TF32 tensor cores, 3 = tcgen05 tensor
+ * cores with the accumulators in tensor memory; at greater M, up to 767, every
+ * value but 1 gives FP32 products), rhs_pts (mixed-form DNS RHS: 1 = one
  * x-point per thread, 2 = two, 3 = two in packed FP32x2 instructions, 4 = as
  * 3 with every plane staged in shared memory by TMA, rhs_by then fixed at
  * 8; FP64 DNS, all bit-identical: 1 = one point, global loads, 4 = one point,

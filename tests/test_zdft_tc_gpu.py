@@ -93,6 +93,53 @@ def test_long_z_transform_products_close_to_fp64(gpu, nx, nz):
         assert rel(a, b) < 1e-5
 
 
+@pytest.mark.parametrize("nz", [194, 258, 402, 455])
+def test_long_z_transform_products_match_direct_sums(gpu, nz):
+    """zdft 1 selects the direct sums beyond the tensor-core lengths as well,
+    to M = 453 (nz = 455), with 4 or 8 wavenumbers per warp: the same FP32
+    transform as the products, for odd M to the bit (the same terms in the same
+    order), for even M to the rounding of sums of M/2 terms (the term M/2 is
+    added first in one form and last in the other)."""
+    c = noisy(nz, nz)
+    out = []
+    for tiles in ({}, {"zdft": 1}, {"zdft": 1, "dftz_rk": 4}, {"zdft": 1, "dftz_rk": 8}):
+        s = cases.solver_for(c, precision=MIXED)
+        s.set_tiles(**tiles)
+        s.apply_boundary_conditions(1)
+        s.compute_projection_step(1)
+        out.append(s.rhs_p())
+        s.close()
+    assert rel(out[0], out[1]) < 1e-5
+    assert np.array_equal(out[0], out[1]) == (nz % 2 == 1)
+    assert np.array_equal(out[1], out[2]) and np.array_equal(out[1], out[3])
+
+
+@pytest.mark.parametrize("nx,nz", [(34, 456), (21, 514), (34, 641), (34, 768), (40, 769)])
+def test_longest_z_transform_products_match_oracle(gpu, nx, nz):
+    """Beyond the direct sums' shared memory (M > 453) up to the products'
+    limit M = 767, the largest columns (M/2+1 = 384) and row tiles of 128 that
+    end full and not (257 and 321 rows, 384): the projection against the FP64
+    oracle at the bars of the shorter lengths."""
+    import oracle
+    c = cases.laminar_case(nx=nx, ny=6, nz=nz, lx=10.0, ly=5.0, lz=16.0)
+    rng = np.random.default_rng(nz)
+    for q in "UVW":
+        a = getattr(c, q)
+        setattr(c, q, np.asfortranarray(a + 0.05 * rng.standard_normal(a.shape)))
+    o = oracle.oracle_for(c)
+    s = cases.solver_for(c, precision=MIXED)
+    o.set_dt(0.01)
+    s.set_dt(0.01)
+    o.apply_bc(1)
+    s.apply_boundary_conditions(1)
+    o.projection(1)
+    s.compute_projection_step(1)
+    assert rel(s.rhs_p()[:, :, :-1], o.rhs_p()[:, :, :-1]) < 3e-5
+    for a, b in zip(s.download_state()[:3], o.state()[:3]):
+        assert rel(a, b) < 1e-5
+    s.close()
+
+
 @pytest.mark.parametrize("nx,ny", [(5, 4), (64, 5), (65, 6), (66, 9), (128, 8), (129, 17), (200, 10)])
 def test_box_scale_pressure_tiles(gpu, nx, ny):
     """The mixed form's FP64 box-scale pressure and its differences at the
