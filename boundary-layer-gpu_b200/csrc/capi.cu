@@ -1048,6 +1048,14 @@ static ZForm z_form(const blgpu_ctx *ctx, const Tiles &t) {
   return Z_SUMS;
 }
 
+// A box whose z columns no form holds: the launch would be refused, and the
+// launches after it would go on with what the spectral arrays hold.
+static int z_check(blgpu_ctx *ctx) {
+  if (ctx->cf || z_form(ctx, ctx->tiles) != Z_SUMS || dft_z_serves(ctx->spec)) return BLGPU_OK;
+  return set_err(ctx, BLGPU_EINVAL, "nz = %d: the z transforms hold up to nz-2 = 453 in shared memory, 767 in the mixed form",
+                 ctx->nz);
+}
+
 template <typename T> static void enq_dft_z(blgpu_ctx *ctx, int inverse) {
   typedef typename vec2<T>::type T2;
   const Spec &s = ctx->spec;
@@ -1250,8 +1258,10 @@ int blgpu_time_step(blgpu_ctx *ctx) {
   if (!ctx) return set_err(ctx, BLGPU_EINVAL, "null ctx");
   if (!ctx->have_grid || !ctx->have_bc || !ctx->have_state)
     return set_err(ctx, BLGPU_ESTATE, "blgpu_time_step: grid, boundary and state must be set first");
+  int rc = z_check(ctx);
+  if (rc) return rc;
   CK(cudaSetDevice(ctx->cfg.device));
-  int rc = step_once(ctx, false);
+  rc = step_once(ctx, false);
   if (rc) return rc;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));
@@ -1263,6 +1273,7 @@ int blgpu_advance(blgpu_ctx *ctx, int nsteps) {
   if (nsteps < 0) return set_err(ctx, BLGPU_EINVAL, "blgpu_advance: nsteps < 0");
   if (!ctx->have_grid || !ctx->have_bc || !ctx->have_state)
     return set_err(ctx, BLGPU_ESTATE, "blgpu_advance: grid, boundary and state must be set first");
+  if (int rc = z_check(ctx)) return rc;
   CK(cudaSetDevice(ctx->cfg.device));
   for (int n = 0; n < (nsteps > 0 ? nsteps : 1); ++n) {
     const int a = ctx->cur;
@@ -1381,10 +1392,12 @@ int blgpu_apply_bc(blgpu_ctx *ctx, int rk_step) {
 int blgpu_projection(blgpu_ctx *ctx, int rk_step) {
   if (!ctx) return set_err(ctx, BLGPU_EINVAL, "null ctx");
   if (!ctx->have_grid || !ctx->have_state) return set_err(ctx, BLGPU_ESTATE, "blgpu_projection: no grid/state");
+  int rc = z_check(ctx);
+  if (rc) return rc;
   CK(cudaSetDevice(ctx->cfg.device));
   if (ctx->fp64) enq_projection<double>(ctx, ctx->cur, rk_step);
   else enq_projection<float>(ctx, ctx->cur, rk_step);
-  int rc = cf_check(ctx);
+  rc = cf_check(ctx);
   if (rc) return rc;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));
@@ -1450,6 +1463,8 @@ int blgpu_phase_times(blgpu_ctx *ctx, int nsteps, double *ms, long long *kernels
   if (!ctx || !ms || nphase < PH_N || nsteps < 1) return set_err(ctx, BLGPU_EINVAL, "blgpu_phase_times: bad argument");
   if (!ctx->have_grid || !ctx->have_bc || !ctx->have_state)
     return set_err(ctx, BLGPU_ESTATE, "blgpu_phase_times: grid, boundary and state must be set first");
+  int rc = z_check(ctx);
+  if (rc) return rc;
   CK(cudaSetDevice(ctx->cfg.device));
   CK(cudaStreamSynchronize(ctx->st));
   for (int p = 0; p < nphase; ++p) {
@@ -1458,7 +1473,6 @@ int blgpu_phase_times(blgpu_ctx *ctx, int nsteps, double *ms, long long *kernels
   }
   ctx->prof_on = true;
   ctx->marks.clear();
-  int rc = 0;
   for (int n = 0; n < nsteps && !rc; ++n) rc = step_once(ctx, true);
   ctx->prof_on = false;
   cudaError_t e = cudaStreamSynchronize(ctx->st);
@@ -2038,6 +2052,7 @@ int blgpu_ensemble_advance(blgpu_ensemble *e, int nsteps) {
   for (blgpu_ctx *c : e->box) {
     if (!c->have_grid || !c->have_bc || !c->have_state)
       return ens_err(e, BLGPU_ESTATE, "blgpu_ensemble_advance: every box needs grid, boundary and state");
+    if (int rc = z_check(c)) return ens_err(e, rc, "%s", c->err.c_str());
     ECK(cudaStreamSynchronize(c->st));  // earlier work of a box on its own stream comes first
   }
   for (int n = 0; n < (nsteps > 0 ? nsteps : 1); ++n) {

@@ -45,7 +45,8 @@ typedef struct blgpu_ctx blgpu_ctx;
 
 /* Run parameters: the .turbb keys of the path (params.f90:119-207). */
 typedef struct blgpu_config {
-  int nx, ny, nz;     /* nxyz: face points (params.f90:131) */
+  int nx, ny, nz;     /* nxyz: face points (params.f90:131); nz-2 up to 453 (mixed: 767) for the
+                         projection's own z transforms, which refuse more */
   double nu;          /* nu (params.f90:119) */
   double cfl;         /* CFL; < 0 means fixed dt = -CFL (time_integration.f90:539) */
   double dpdx, dpdz;  /* dPdx, dPdz (params.f90:152-153) */

@@ -140,6 +140,28 @@ def test_longest_z_transform_products_match_oracle(gpu, nx, nz):
     s.close()
 
 
+@pytest.mark.parametrize("prec,nz", [(MIXED, 770), (FP64, 456)])
+def test_z_lengths_past_shared_memory_are_refused(gpu, prec, nz):
+    """No z transform holds M = 768 columns in the mixed form, or 454 in FP64:
+    projections and steps say so instead of going on without the transform, and
+    neither the context nor the next one is left with an error."""
+    from blgpu import BlgpuError, Ensemble
+    c = cases.laminar_case(nx=10, ny=6, nz=nz, lx=10.0, ly=5.0, lz=16.0)
+    s = cases.solver_for(c, precision=prec)
+    s.set_dt(0.01)
+    s.apply_boundary_conditions(1)
+    ens = Ensemble([s])
+    for call in (lambda: s.compute_projection_step(1), s.time_step, lambda: s.advance(1), lambda: s.phase_times(1),
+                 lambda: ens.advance(1)):
+        with pytest.raises(BlgpuError, match="z transforms hold"):
+            call()
+    ens.close()
+    s.sync()
+    assert np.isfinite(s.compute_rhs(c.U, c.V, c.W)[0]).all()
+    s.close()
+    cases.solver_for(c, precision=prec).close()
+
+
 @pytest.mark.parametrize("nx,ny", [(5, 4), (64, 5), (65, 6), (66, 9), (128, 8), (129, 17), (200, 10)])
 def test_box_scale_pressure_tiles(gpu, nx, ny):
     """The mixed form's FP64 box-scale pressure and its differences at the
