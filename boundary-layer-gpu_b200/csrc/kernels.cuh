@@ -19,14 +19,17 @@ template <typename T> struct MetT {
 // autotuner (blgpu_autotune) searches these per box.
 struct Tiles {
   int rhs_kc;   // k-planes walked by one CTA of the RHS kernel (0: 8 to 32 by kernel, fewer in small boxes, z_chunk)
-  int rhs_by;   // RHS block is 32 x rhs_by threads (0: 8)
-  int dct_nw;   // complex lines (warps) per CTA of the forward DCT, up to 16 in FP32 (8 two-pass) and 8 in FP64 (0: built-in)
-  int dftz_rk;  // z wavenumbers per warp in the z-DFT, 4 or 8 (0: 8)
+  int rhs_by;   // RHS block is 32 x rhs_by threads (0: 8); read by the forms with global loads (rhs_pts 1; FP32 DNS 2, 3)
+  int dct_nw;   // complex lines per CTA of the forward DCT, one warp each, up to 16 in FP32 (8 two-pass) and 8 in FP64
+                // (0: built-in, where a line may have several warps)
+  int dftz_rk;  // z wavenumbers per warp in the direct sums of the z transform, 4 or 8 (0: 8)
   int proj_by;  // projection block is 32 x proj_by threads (0: 4)
-  int zdft;     // mixed-form z transforms: 1 FP32 sums, 2 mma.sync TF32, 3 tcgen05 (0: tcgen05, else mma.sync, else sums)
+  int zdft;     // mixed-form z transforms: 1 FP32 sums, 2 mma.sync TF32, 3 tcgen05 (0: tcgen05, else mma.sync, else
+                // FP32 products beyond M/2+1 = 96)
   int rhs_pts;  // FP32 DNS RHS: 1 one point per thread, 2 two points, 3 two points packed in FP32x2
                 // instructions, 4 the same fed by TMA (0: 4 where its tensor maps exist, else 2);
-                // FP64 DNS: 1 one point with global loads, 4 one point TMA-fed, 0 or 2 two points
+                // FP64 DNS: 1 one point with global loads, 4 one point TMA-fed, 0 or 2 two points;
+                // LES: 1 one point with global loads, else one point TMA-fed
   int thomas;   // y-solve: 1 register ring, 2 TMA tiles where the box allows (one thread per mode), 3 the
                 // tiles with each mode's rows split over 16 threads (0: 3 where the tiles exist, else 1)
   int idct_nw;  // complex lines (warps) per CTA of the inverse DCT, as dct_nw (0: built-in)

@@ -248,9 +248,12 @@ int blgpu_check_divergence_noalloc(const double *U, const double *V, const doubl
 
 /* ---- launch shapes and the autotuner ----
  * tiles[5 to 10] = rhs_kc (k-planes per CTA of the RHS kernel), rhs_by (RHS
- * block 32 x rhs_by), dct_nw (complex lines per CTA of the forward DCT, up
- * to 16 in the mixed form (8 with the two-pass x transforms) and 8 in FP64),
- * dftz_rk (z wavenumbers per warp of the z-DFT, 4 or 8), proj_by (projection
+ * block 32 x rhs_by, in the forms with global loads: rhs_pts 1 and the mixed
+ * DNS forms 2 and 3), dct_nw (complex lines per CTA of the forward DCT, up
+ * to 16 in the mixed form (8 with the two-pass x transforms) and 8 in FP64; an
+ * explicit count gives each line one warp, where the built-in choice gives
+ * long lines with a prime factor above 31 two or four), dftz_rk (z wavenumbers
+ * per warp of the direct sums of the z transform, 4 or 8), proj_by (projection
  * block 32 x proj_by), zdft (mixed form: 1 = FP32 direct sums, M = nz-2 up
  * to 453; where M/2+1 <= 96 2 = mma.sync TF32 tensor cores, 3 = tcgen05 tensor
  * cores with the accumulators in tensor memory; at greater M, up to 767, every
@@ -258,7 +261,9 @@ int blgpu_check_divergence_noalloc(const double *U, const double *V, const doubl
  * x-point per thread, 2 = two, 3 = two in packed FP32x2 instructions, 4 = as
  * 3 with every plane staged in shared memory by TMA, rhs_by then fixed at
  * 8; FP64 DNS, all bit-identical: 1 = one point, global loads, 4 = one point,
- * TMA-fed planes, 2 = two points in a register window),
+ * TMA-fed planes, 2 = two points in a register window; LES: 1 = one point,
+ * global loads, every other value = one point, TMA-fed planes, bit-identical in
+ * FP64),
  * thomas (y-solve: 1 = register ring,
  * 2 = TMA-fed tiles where ny-1 <= 256, one thread per mode, 3 = the same
  * tiles with each mode's rows split over 16 threads; the built-in choice

@@ -94,6 +94,26 @@ def test_autotune_restores_state_and_keeps_results(gpu):
     assert same(states([ref]), states([s]))
 
 
+@pytest.mark.parametrize("kind", ["les fp64", "les mixed", "long z", "fp64", "mixed"])
+def test_autotune_leaves_knobs_without_effect(gpu, kind):
+    """A knob that the chosen kernels do not read keeps its value: rhs_by where
+    the RHS stages its planes (LES and the mixed DNS default) or takes fixed
+    rows (FP64 DNS), dftz_rk where the z transform is a product."""
+    nz = 200 if kind == "long z" else 66  # products of every kind; shorter mixed boxes take the direct sums
+    c = cases.turbulent_case(nx=40, ny=9, nz=nz, lx=5.0, ly=4.0, lz=nz * 0.04, retheta=900.0, seed=5)
+    s = cases.solver_for(c, precision=FP64 if "fp64" in kind else MIXED, les_model=1 if "les" in kind else 0,
+                         inflow=False)
+    s.autotune(steps=1)
+    t = s.tiles()
+    if "les" in kind or t["rhs_pts"] in (0, 4):
+        assert t["rhs_by"] == 0
+    if "les" in kind:
+        assert t["rhs_pts"] == 0
+    if "fp64" in kind or t["zdft"] != 1:
+        assert t["dftz_rk"] == 0
+    s.close()
+
+
 def test_ensemble_autotune_shares_tiles_by_shape(gpu):
     cs = small_boxes(4, seed=15) + small_boxes(2, seed=16)
     box = [cases.solver_for(c, precision=MIXED) for c in cs]
