@@ -342,7 +342,7 @@ int blgpu_create(const blgpu_config *cfg, blgpu_ctx **out) {
   if (!ctx->fp64) {
     // the modes kx < klow of kz = 0 carry the box-scale pressure of a step's
     // flux change; above them the modes are small enough for FP32
-    ctx->klow = std::min(128, s.N);
+    ctx->klow = std::min(KLOW_MAX, s.N);
     TRY(dalloc(ctx, (void **)&ctx->kz0, (size_t)s.NM * s.N * sizeof(double)));
     TRY(dalloc(ctx, (void **)&ctx->kz0h, (size_t)s.NM * ctx->klow * sizeof(double)));
     TRY(dalloc(ctx, (void **)&ctx->kz0g, 2 * (size_t)s.NM * s.N * sizeof(float)));

@@ -157,6 +157,7 @@ void launch_zdft64(const Spec &s, double *R, double2 *C, const double *tab, int 
 template <typename T>
 void launch_thomas(const Spec &s, typename vec2<T>::type *C, const double *piv, const double *dl, const double *du,
                    double *H0, int klow, cudaStream_t st);
+constexpr int KLOW_MAX = 128;  // most modes of the box-scale pressure (klow <= KLOW_MAX: k_kz0 holds that many)
 // p0[NM][N] = inverse cosine sum of H0 (cm[kx][i] = w_kx cos(pi kx (2i+1)/2N)/(N M))
 // and grad = FP32 x and y differences of p0 ([2][NM][N])
 void launch_kz0_idct(const Spec &s, const double *H0, int klow, const double *cm, double *p0, float *grad,

@@ -18,7 +18,6 @@
 //               z-periodic copies of apply_periodic_z_pressure
 //               (projection.f90:295-303).
 #include <algorithm>
-#include <cstdlib>
 
 #include "kernels.cuh"
 #include "divergence.cuh"
@@ -1536,13 +1535,14 @@ constexpr int KZ_R = 4, KZ_C = 63, KZ_G = 4;
 __global__ void __launch_bounds__(64 * KZ_G) k_kz0(Spec s, const double *__restrict__ H, int K,
                                                    const double *__restrict__ cm, double *__restrict__ p0,
                                                    float *__restrict__ gx, float *__restrict__ gy) {
-  __shared__ double Hs[KZ_R + 1][128];
+  static_assert((KLOW_MAX & (KLOW_MAX - 1)) == 0, "mode index by mask");
+  __shared__ double Hs[KZ_R + 1][KLOW_MAX];
   __shared__ double ps[KZ_G][KZ_R + 1][64];
   const int N = s.N, NM = s.NM;
   const int b0 = blockIdx.y * KZ_R, i0 = blockIdx.x * KZ_C;
   const int c = threadIdx.x, grp = threadIdx.y, t = grp * 64 + c;
-  for (int q = t; q < (KZ_R + 1) * 128; q += 64 * KZ_G) {
-    const int r = q >> 7, k = q & 127;
+  for (int q = t; q < (KZ_R + 1) * KLOW_MAX; q += 64 * KZ_G) {
+    const int r = q / KLOW_MAX, k = q & (KLOW_MAX - 1);
     Hs[r][k] = (b0 + r < NM && k < K) ? __ldg(H + (long long)(b0 + r) * K + k) : 0.0;
   }
   __syncthreads();
