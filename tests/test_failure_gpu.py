@@ -80,15 +80,17 @@ def test_y_solve_wait_limit_reports_and_recovers(gpu, thomas):
     r.close()
 
 
-def test_rhs_plane_wait_limit_reports_and_recovers(gpu):
-    """The TMA-fed RHS (mixed form, rhs_pts 4) given zero polls: every CTA's
-    first plane wait gives up, the CTA drains the copies it issued and
-    leaves, the step reports BLGPU_EDEVICE; with the limit restored and the
+@pytest.mark.parametrize("precision,les,pts", [(MIXED, 0, 4), (FP64, 0, 4), (MIXED, 1, 0), (FP64, 1, 0)])
+def test_rhs_plane_wait_limit_reports_and_recovers(gpu, precision, les, pts):
+    """The TMA-fed RHS (the packed mixed form and the one-point form, rhs_pts
+    4, and the LES default with its four fields per stage) given zero polls:
+    every CTA's first plane wait gives up, the CTA drains the copies it issued
+    and leaves, the step reports BLGPU_EDEVICE; with the limit restored and the
     state uploaded again the context steps exactly as a fresh one."""
     c = _case()
     c.cfl = -1e-3
-    s = cases.solver_for(c, precision=MIXED)
-    s.set_tiles(rhs_pts=4, thomas=1)  # the register-ring y-solve waits on no mbarrier
+    s = cases.solver_for(c, precision=precision, les_model=les)
+    s.set_tiles(rhs_pts=pts, thomas=1)  # the register-ring y-solve waits on no mbarrier
     s.set_wait_limit(0)
     s.time_step()
     with pytest.raises(BlgpuError, match="RHS"):
@@ -98,8 +100,8 @@ def test_rhs_plane_wait_limit_reports_and_recovers(gpu):
     s.upload_state(c.U, c.V, c.W)
     s.set_dt(1e-3)
     s.advance(2)
-    r = cases.solver_for(c, precision=MIXED)
-    r.set_tiles(rhs_pts=4, thomas=1)
+    r = cases.solver_for(c, precision=precision, les_model=les)
+    r.set_tiles(rhs_pts=pts, thomas=1)
     r.advance(2)
     for a, b in zip(s.download_state()[:3], r.download_state()[:3]):
         assert np.array_equal(a, b)
