@@ -15,7 +15,7 @@
 // Ghost entries (apply_Neumann_bc_x / apply_periodic_bc_x,
 // boundary_conditions.f90:295-344; apply_periodic_bc_z, :732-760; one process)
 // are never stored: a reader takes the interior entry that the source's copies
-// would have left there, by index (XMap, zmap).
+// would have left there, by index (xmap, zmap, zmap_w).
 // The filter of filter_xzy (subgrid.f90:140-184, fil_size = 2) is the product
 // of (1,4,1)/6 along x, y and z (one-sided 2/3, 1/3 at the first and last row
 // of its y section), applied as three sums.

@@ -1122,7 +1122,10 @@ __host__ __device__ inline int zd64_kp(int M) { return ((M - 1) / 2 + 3) / 4 * 4
 __host__ __device__ inline int zd64_rows(int M) { return (M / 2 + 1 + 15) / 16 * 16; }
 // rows of the inverse's column data: kz = 0 .. M/2 and the products' K range 1 .. Kp
 __host__ __device__ inline int zd64_crows(int M) { return zd64_kp(M) + 1 > M / 2 + 1 ? zd64_kp(M) + 1 : M / 2 + 1; }
-// 112 registers: three CTAs of six warps per SM (M = 191), two at the 126 and 118 taken otherwise
+// 112 registers: three CTAs of six warps per SM (M = 191), two at the 126 and
+// 118 taken otherwise.  Other lengths keep the bound: every one gained with the
+// layout above (130 x 65 x nz, us per launch of both directions, before -> now:
+// nz = 34 21.1 -> 18.6, 66 24.9 -> 21.2, 130 38.6 -> 33.5, 256 69.0 -> 60.4)
 #define ZD64_REGS __maxnreg__(112)
 constexpr int ZP = 36;  // pitch of the [k][x] column data, 32 columns
 

@@ -1028,10 +1028,10 @@ __global__ void __launch_bounds__(32 * R64_BY, sizeof(T) == 8 ? 2 : 3)
                    const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mou,
                    const __grid_constant__ CUtensorMap mov, const __grid_constant__ CUtensorMap mow,
                    const __grid_constant__ CUtensorMap mfu, const __grid_constant__ CUtensorMap mfv,
-                   const __grid_constant__ CUtensorMap mfw, const __grid_constant__ CUtensorMap mn, Geo g, MetT<T> m, T *__restrict__ F1u,
-                   T *__restrict__ F1v, T *__restrict__ F1w, T *__restrict__ Un,
-                   T *__restrict__ Vn, T *__restrict__ Wn, const Scalars *__restrict__ sc, double c1,
-                   double c2, int kchunk, int *err, int wait_limit) {
+                   const __grid_constant__ CUtensorMap mfw, const __grid_constant__ CUtensorMap mn, Geo g, MetT<T> m,
+                   T *__restrict__ F1u, T *__restrict__ F1v, T *__restrict__ F1w, T *__restrict__ Un,
+                   T *__restrict__ Vn, T *__restrict__ Wn, const Scalars *__restrict__ sc, double c1, double c2,
+                   int kchunk, int *err, int wait_limit) {
   constexpr int NS = R1_NS<LES>, TW = R1_TW<T>, FS = R1_FS<T>, NF = LES ? 4 : 3, NPW = rt_npw(MODE),
                 SS = R1_STAGE<T, MODE, LES>;
   constexpr uint32_t ES = sizeof(T);
@@ -1133,7 +1133,7 @@ __global__ void __launch_bounds__(32 * R64_BY, sizeof(T) == 8 ? 2 : 3)
         }
       }
       if (k == k1) goto drain;
-      __syncthreads();  // plane k-1 read by all: its stage takes plane k+4
+      __syncthreads();  // plane k-1 read by all: its stage takes plane k+NS-1
       if (*bad) goto drain;
       if (tid == 0 && k + NS - 1 <= k1 + 1) {
         issue(k + NS - 1);
@@ -1259,7 +1259,8 @@ __global__ void __launch_bounds__(256, SAVE && sizeof(T) == 8 ? 4 : 0) k_project
 // threads take longer over the plane than the launch: 0.094 -> 0.200 ms per
 // step at 256 x 65 x 96.)  The first call of a substep also moves the time
 // (tc >= 0: t = to + tc dt, time_integration.f90:349,383,417), the last one
-// of a step saves it as the next step's start time.
+// of a step saves it as the next step's start time (save_to).  The two are not
+// for the same call: block 0 would write to while other blocks read it.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double mode_sum(const double2 *__restrict__ q, int ld, int j, int nm, int mm,
                                            const double *__restrict__ zmode, const double *__restrict__ tmode,
@@ -1781,9 +1782,6 @@ __global__ void __launch_bounds__(256) k_dt_reduce4(Geo g, const T *__restrict__
   }
 }
 
-// time_integration.f90:560-575 (dt = min(dt_conv, dt_vis)); also arms the
-// accumulators for the next call and records to = t for the RK substeps.
-
 // check_divergence (projection.f90:399-408): max |div| over i=2..nxg-2
 template <typename T>
 __global__ void __launch_bounds__(256) k_maxdiv(Geo g, const T *__restrict__ U, const T *__restrict__ V,
@@ -1973,8 +1971,8 @@ __global__ void __launch_bounds__(256) k_law_of_wall(Geo g, const T *__restrict_
 // side (an ensemble's) would hold fewer than 200 CTAs.  A chunk's two extra
 // planes cost little next to SMs without a CTA, and are lost where other boxes
 // fill them: with each box counted alone 16 boxes of 128..256 x 65 x 64..96
-// took 4.18 ms per step (now 4.13), 64 boxes 16.26 (15.85), mixed.  RHS of a box alone, us
-// per launch by planes per CTA (2 4 8 16), the rule's choice first:
+// took 4.18 ms per step (now 4.13), 64 boxes 16.26 (15.85), mixed.  RHS of a
+// box alone, us per launch by planes per CTA (2 4 8 16), the rule's choice first:
 //   128 x 64 x 32   FP64  2: 14.6 14.3 19.9 30.8   mixed  2: 10.4 11.2 14.6 21.3
 //   128 x 65 x 64   FP64  4: 22.9 21.1 20.7 32.4   mixed  4: 14.0 12.6 14.6 20.9
 //   256 x 65 x 96   FP64  8: 57.5 53.0 52.4 62.6   mixed  8: 30.2 26.8 26.3 26.8
@@ -2115,8 +2113,6 @@ void launch_rhs_rk(const Geo &g, const MetT<T> &m, int mode, bool les, const T *
 #undef BLGPU_DNS_CASE
   } else if (!les) {
     if constexpr (sizeof(T) == 8) {
-      // FP64 DNS: the TMA-fed kernel (results bit-identical to k_rhs_rk) where
-      // its maps exist, unless rhs_pts = 1 asks for the global-load kernel
       // FP64 DNS: the two-point register window (rhs_pts 0 or 2, bit-identical to
       // k_rhs_rk: its shared and carried terms are the same expressions), the
       // TMA-fed one-point kernel (rhs_pts 4) or the global-load kernel (1)

@@ -14,8 +14,12 @@
 // pairs in FP32x2 multiply-adds: per k six 16-byte shared loads for 64
 // multiply-adds.  Bounded by FP32 arithmetic (Q^2 multiply-adds per column
 // and product): 1.6e9 at 512 x 96 x 256, 44 us at one per lane and clock.
-// With one column pair per lane and the table read through L1 (k_dft_z_*):
-// 0.203 / 0.213 ms per launch there.
+// The direct sums (k_dft_z_*: one column group per lane, the table through L1)
+// lose at every length they hold; us per launch at 258 x 65 x nz, forward /
+// inverse, sums -> products: nz = 195 68 / 54 -> 33 / 31, 226 79 / 62 ->
+// 37 / 35, 258 106 / 103 -> 68 / 66, 322 154 / 140 -> 99 / 94, 402 237 / 236 ->
+// 118 / 109 (from Q = 145 on one CTA fits an SM); 514 and 769, which the sums
+// do not hold: 217 / 202 and 311 / 290.
 #include <cmath>
 #include <vector>
 
@@ -177,6 +181,7 @@ size_t zsum_smem(const Spec &s) { return ((size_t)2 * kpad_of(s) * ZC + 2 * ZK *
 
 }  // namespace
 
+// M = 192 .. 767: above the tensor-core lengths, to the columns that fit a CTA
 bool zsum_serves(const Spec &s) { return s.MH > 96 && zsum_smem(s) <= 227 * 1024; }
 
 void zsum_tables(const Spec &s, std::vector<float> &t) {

@@ -28,17 +28,18 @@ def noisy(nx, ny, nz, seed, amp, **kw):
 @pytest.mark.parametrize("model", [2, 3])
 @pytest.mark.parametrize("grid", [(26, 14, 11), (61, 17, 16), (300, 9, 40)])
 def test_dynamic_nu_t_matches_oracle(gpu, model, grid):
-    """300 x 9 x 40: several 128-point x blocks of the filter kernel (the
-    halo at ib-1 and ib+128 and the guard at the last block) and three
-    16-plane k blocks, against the oracle."""
+    """300 x 9 x 40: ten 32-column blocks of the strain and filter kernels and
+    ten 30-output warps of the contraction, three z chunks of 16 planes and two
+    of 32, against the oracle."""
     c = noisy(*grid, seed=31, amp=0.05)
     s = cases.solver_for(c, les_model=model)
     o = oracle.oracle_for(c)
     nut = s.compute_eddy_viscosity()
     ref = o.dynamic_smagorinsky(model)
     assert ref.max() > 0 and (ref > 0).mean() > 0.1
-    # FP64 in the oracle's evaluation order; sqrt against pow(x, 0.5) and the
-    # Mij Lij / Mij Mij quotient leave a few ulps
+    # FP64; the filters as three sums of (1,4,1)/6 against the oracle's 27-point
+    # one, sqrt against pow(x, 0.5) and the Mij Lij / Mij Mij quotient leave some
+    # ulps of Lij's operands
     assert np.abs(nut - ref).max() <= 1e-12 * np.abs(ref).max()
     s.close()
 
