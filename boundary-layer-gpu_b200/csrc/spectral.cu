@@ -1650,34 +1650,41 @@ static int radix_class(const int *rad, int nst) {
 // shared memory and grid
 struct XShape {
   int nw, wpl;
-  int kb;  // outputs per lane of a prime stage above the register butterflies, 0 without one
+  int kb;  // outputs per lane of a prime stage above the register butterflies, 0: the kernel has none
   size_t sm;
   int grid;
 };
 
+// Cost of a grid of x-transform CTAs against another shape of the kernel:
+// waves of the CTAs that `warps` of registers and the shared memory let an SM
+// hold, a wave of c of them taken as c + 3 (they share the SM, and part of
+// their time is latency)
+static double x_wave_cost(const XShape &x, int warps) {
+  const int fit = std::max(1, std::min(warps / x.nw, (int)(228 * 1024 / (x.sm + 1024))));
+  return (double)((x.grid + 148 * fit - 1) / (148 * fit)) * (std::min(fit, (x.grid + 147) / 148) + 3);
+}
+
 // Outputs per lane of a prime stage (radix R, nb butterflies) that one warp
 // works: of 1, 2 and 4 the fewest rounds of 32 items, weighted by what a round
-// costs (a round of 4 outputs about three of one).  us per launch, forward +
-// inverse, 1 / 2 / 4 outputs:
-//   N =  37 (1 1 1 rounds)  FP64 129x130 53.6 56.9 78.9   mixed 41.6 45.4 53.7
-//   N = 127 (2 1 1)         FP64 129x130  152  142  168   mixed 93.2 87.6  104
-//   N = 254 (4 2 1)         FP64 129x130  262  263  244   mixed  147  137  130
-//   N = 298 (5 3 2)         FP64 129x130  337  340  360   mixed  189  190  218
-//   N = 358 (6 3 2)         FP64 129x130  498  438  438   mixed  251  227  256
-//   N = 397 (7 4 2)         FP64 129x130 1234 1148 1001   mixed  624  598  561
-// (ny x nz after the precision.)  Lines of several warps keep 4.
-static int prime_outputs_per_lane(int R, int nb) {
+// costs; `four`: the cost of the kernel's grid with 4 outputs, whose registers
+// let fewer warps stay on an SM in FP64, over that with 1 or 2.  A round of 4 is
+// cheaper with more butterflies in FP64, whose lanes then read the same table
+// values (16 bytes each bound it; FP32 is bound by its instructions).  us per
+// launch, forward + inverse, 1 / 2 / 4 outputs, 129 x 130 (ny x nz):
+//   N =  37 (1 1 1 rounds)  FP64 53.6 56.9 78.9   mixed 41.6 45.4 53.7
+//   N = 127 (2 1 1)         FP64  152  142  168   mixed 93.2 87.6  104
+//   N = 254 (4 2 1)         FP64  262  263  244   mixed  147  137  130
+//   N = 298 (5 3 2)         FP64  337  340  360   mixed  189  190  218
+//   N = 358 (6 3 2)         FP64  498  438  438   mixed  251  227  256
+//   N = 370 (6 4 2)         FP64  293    -  236
+//   N = 397 (7 4 2)         FP64 1234 1148 1001   mixed  624  598  561
+// Lines of several warps and N >= 400 keep 4.
+static int prime_outputs_per_lane(bool fp64, int R, int nb, double four) {
   const int H = (R - 1) / 2;
-  int best = 1;
-  double least = 0.0;
-  for (int kb = 1; kb <= 4; kb *= 2) {
-    const double cost = ((nb * ((H + kb) / kb) + 31) / 32) * (kb == 1 ? 1.0 : kb == 2 ? 1.6 : 3.0);
-    if (kb == 1 || cost < least) {
-      best = kb;
-      least = cost;
-    }
-  }
-  return best;
+  auto rounds = [&](int kb) { return (double)((nb * ((H + kb) / kb) + 31) / 32); };
+  const double c1 = rounds(1), c2 = rounds(2) * (fp64 ? 1.5 : 1.6);
+  const double c4 = rounds(4) * (!fp64 ? 2.9 : nb <= 2 ? 2.6 : nb <= 6 ? 2.2 : 1.9) * four;
+  return c4 < c1 && c4 < c2 ? 4 : c2 < c1 ? 2 : 1;
 }
 
 // Lines per CTA and warps per line.  Several warps share a line of the
@@ -1713,13 +1720,17 @@ static XShape x_shape(const Spec &s, const FftPlan<T> &pl, int nw_req, int split
   }
   x.sm = dct_smem_bytes(s.N, sizeof(T), x.nw, split);
   x.grid = ((s.NM * s.M + 1) / 2 + x.nw - 1) / x.nw;
-  x.kb = rmax > 31 ? prime_outputs_per_lane(rmax, s.N / rmax) : 0;
-  // A grid of up to two CTAs per SM has the registers to spare: there the FP64
-  // forward kernel takes the instance with more of them (98 against 76), which
-  // keeps more of its divergence loads in flight (N = 126, 33 x 66: 16.7 ->
-  // 15.1 us per launch; two CTAs of six such warps are what an SM holds, and a
-  // 65 x 64 box, 331 CTAs, takes 25.0 us with it, 17.5 without).
-  if (sizeof(T) == 8 && !inverse && !x.kb && x.grid <= 2 * 148) x.kb = 4;
+  // FP64, one warp per line: an SM holds the registers of 24 warps with 1 or 2
+  // outputs per lane or no prime stage, of 16 (inverse 20) with 4
+  const double four = sizeof(T) == 8 ? x_wave_cost(x, inverse ? 20 : 16) / x_wave_cost(x, 24) : 1.0;
+  x.kb = rmax > 31 && s.N < 400 ? prime_outputs_per_lane(sizeof(T) == 8, rmax, s.N / rmax, four) : 4;
+  // Without a prime stage the FP64 instance that has none leaves room for more
+  // CTAs (N = 126 in a 65 x 64 box, 331 CTAs: 25.0 -> 17.5 us forward per
+  // launch); the forward transform takes the one with more registers (98
+  // against 76), which keeps more of its divergence loads in flight, where its
+  // waves cost no more (33 x 66, 171 CTAs: 16.7 -> 15.1; N = 256 in 65 x 100,
+  // 523 CTAs: 45.1 -> 38.9).
+  if (sizeof(T) == 8 && rmax <= 31 && (inverse || four > 1.0)) x.kb = 0;
   return x;
 }
 
@@ -1741,15 +1752,15 @@ static void launch_idct_e(const Geo &g, const Spec &s, const FftPlan<T> &pl, con
 
 // calls f with the Stockham engine of the plan's radix class and line shape.
 // One warp per line: the instances of the first class differ in their prime
-// stage (none, or 1, 2 or 4 outputs per lane), which sets their registers
-// (FP64 forward 76, 78, 98 with none, 1 and 4: at N = 126 and 128 a CTA per SM
-// less with it); the other classes hold more for their butterflies, and N with
-// a factor above 7 and a prime above 31 are past 400.
+// stage (1, 2 or 4 outputs per lane, none in FP64), which sets their registers
+// (FP64 forward 78, 78, 98, 76); the other classes hold more for their
+// butterflies, and N with a factor above 7 and a prime above 31 are past 400.
 template <class E> struct XEngine { typedef E type; };
 template <typename T, int MAXR, class F> static void stockham_shape(const XShape &x, F f) {
   if (x.wpl > 1) return f(XEngine<StockhamX<T, MAXR, 4, true>>());
   if constexpr (MAXR == 7) {
-    if (x.kb == 0) return f(XEngine<StockhamX<T, MAXR, 0>>());
+    if constexpr (sizeof(T) == 8)
+      if (x.kb == 0) return f(XEngine<StockhamX<T, MAXR, 0>>());
     if (x.kb == 1) return f(XEngine<StockhamX<T, MAXR, 1>>());
     if (x.kb == 2) return f(XEngine<StockhamX<T, MAXR, 2>>());
   }

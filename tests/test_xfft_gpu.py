@@ -124,7 +124,7 @@ def test_fp64_two_pass_matches_stockham(gpu, nx, ny, nz):
 def test_prime_stage_outputs(gpu, n):
     """x lengths with a prime stage above the register butterflies (37, 41,
     43, 2 37, 3 37, 4 37, 2 103, 2 127, 7 37, 331, 397, 509), where a lane
-    takes one output (37, 41, 43, 148), two (74, 111, 259, 331) or four and
+    takes one output (37, 41, 43), two (74, 111, 331; 259 mixed) or four and
     the number of outputs per butterfly, (R+1)/2 = 19, 21, 22, 52, 64, 166,
     199, 255, is or is not a multiple of that; FP64 against the oracle (the
     projection's bar), mixed against FP64 at the Stockham transform's FP32
