@@ -14,8 +14,9 @@
 // LD supplies the velocities as R: u(s, dj, k) is U(i-1+s, j+dj, k), s = 0, 1;
 // v(s, dj, k) is V(i-1+s, j+dj, k), s = 0..2; w(s, dj, k) is W(i-1+s, j+dj, k),
 // s = 0..2 (Fortran indices; LD may map ghost columns and planes); pre(k) starts
-// the three fields' lines of plane k on their way (the kernels wait on loads:
-// 5 to 7 of 10 stall cycles per instruction).
+// the three fields' lines of plane k on their way.  Loads are what the kernels
+// wait for most: 4.4 cycles of the 8.7 between a warp's instructions in the
+// FP64 Smagorinsky kernel, 3.4 and 3.8 of about 8 in the dynamic model's.
 #pragma once
 #include "common.cuh"
 
