@@ -1122,10 +1122,13 @@ __host__ __device__ inline int zd64_kp(int M) { return ((M - 1) / 2 + 3) / 4 * 4
 __host__ __device__ inline int zd64_rows(int M) { return (M / 2 + 1 + 15) / 16 * 16; }
 // rows of the inverse's column data: kz = 0 .. M/2 and the products' K range 1 .. Kp
 __host__ __device__ inline int zd64_crows(int M) { return zd64_kp(M) + 1 > M / 2 + 1 ? zd64_kp(M) + 1 : M / 2 + 1; }
-// 112 registers: three CTAs of six warps per SM (M = 191), two at the 126 and
-// 118 taken otherwise.  Other lengths keep the bound: every one gained with the
-// layout above (130 x 65 x nz, us per launch of both directions, before -> now:
-// nz = 34 21.1 -> 18.6, 66 24.9 -> 21.2, 130 38.6 -> 33.5, 256 69.0 -> 60.4)
+// 112 registers, 16 warps per SM: two CTAs at M = 191 (six warps).  Bounds of 256
+// threads give 96 and 102 (20 and 16 warps), no better over the lengths: us per
+// launch, forward / inverse, 112 against those, 814 x 257 x 193 332 / 349 against
+// 336 / 331, 512 x 129 x 193 113 / 114 against 113 / 115, x 256 167 / 161
+// against 166 / 166, x 66 33.2 / 31.2 against 32.6 / 33.1.  Every length gained
+// with the layout above (130 x 65 x nz, us per launch of both directions, before
+// -> now: nz = 34 21.1 -> 18.6, 66 24.9 -> 21.2, 130 38.6 -> 33.5, 256 69.0 -> 60.4).
 #define ZD64_REGS __maxnreg__(112)
 constexpr int ZP = 36;  // pitch of the [k][x] column data, 32 columns
 
