@@ -70,6 +70,7 @@ struct blgpu_ctx {
   int boxes = 1;              // boxes whose steps the graph being captured runs side by side (ensembles)
   CufftPath *cf = nullptr;    // poisson = BLGPU_POISSON_CUFFT: plans and work arrays
   int cf_status = 0;          // first failing cufftExec status of an enqueued step (0: none)
+  cudaError_t launch_err = cudaSuccess;  // first launch error of an enqueued step
   int wait_limit = -1;        // mbarrier polls of the tiled y-solve and the TMA-fed RHS (< 0: built-in), a test hook
   bool have_tmaps = false;
   int nsm = 148;
@@ -128,8 +129,11 @@ static void ph_begin(blgpu_ctx *ctx, int phase) {
   }
 }
 
+// Also keeps the first launch error: the runtime's last error is cleared by the
+// next successful cudaFuncSetAttribute, which most launchers call.
 static void ph_end(blgpu_ctx *ctx, int nk) {
   ctx->launches += nk;
+  if (ctx->launch_err == cudaSuccess) ctx->launch_err = cudaPeekAtLastError();
   if (ctx->prof_on) {
     cudaEvent_t b;
     cudaEventCreate(&b);
@@ -1238,18 +1242,25 @@ static int enq_step(blgpu_ctx *ctx, int a, bool with_dt) {
 }
 
 // a cufftExec of the cuFFT comparison path refused work that was enqueued
-static int cf_check(blgpu_ctx *ctx) {
-  if (!ctx->cf_status) return BLGPU_OK;
+// reports, once, what failed while work was enqueued
+static int enq_check(blgpu_ctx *ctx) {
+  const cudaError_t e = ctx->launch_err;
   const int r = ctx->cf_status;
+  ctx->launch_err = cudaSuccess;
   ctx->cf_status = 0;
-  return set_err(ctx, BLGPU_ECUDA, "cuFFT comparison path: cufftExec failed (cufftResult %d)", r);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return check_cuda(ctx, e, "a kernel launch");
+  }
+  if (r) return set_err(ctx, BLGPU_ECUDA, "cuFFT comparison path: cufftExec failed (cufftResult %d)", r);
+  return BLGPU_OK;
 }
 
 static int step_once(blgpu_ctx *ctx, bool with_dt) {
   int nb = ctx->fp64 ? enq_step<double>(ctx, ctx->cur, with_dt) : enq_step<float>(ctx, ctx->cur, with_dt);
   ctx->old = ctx->cur;
   ctx->cur = nb;
-  return cf_check(ctx);
+  return enq_check(ctx);
 }
 
 extern "C" {
@@ -1285,11 +1296,11 @@ int blgpu_advance(blgpu_ctx *ctx, int nsteps) {
       ctx->graph_launches[a] = ctx->launches - l0;
       ctx->launches = l0;
       cudaError_t e = cudaStreamEndCapture(ctx->st, &gr);
-      if (e != cudaSuccess) return check_cuda(ctx, e, "cudaStreamEndCapture");
-      if (ctx->cf_status) {
-        cudaGraphDestroy(gr);
-        return cf_check(ctx);
+      if (int rc = enq_check(ctx)) {
+        if (gr) cudaGraphDestroy(gr);
+        return rc;
       }
+      if (e != cudaSuccess) return check_cuda(ctx, e, "cudaStreamEndCapture");
       e = cudaGraphInstantiate(&ctx->graph[a], gr, 0);
       cudaGraphDestroy(gr);
       if (e != cudaSuccess) return check_cuda(ctx, e, "cudaGraphInstantiate");
@@ -1352,6 +1363,7 @@ int blgpu_compute_rhs(blgpu_ctx *ctx, const double *U, const double *V, const do
   if (rc) return rc;
   if (ctx->fp64) enq_rhs<double>(ctx, 0, sb, sb, sb, 0.0, 0.0);
   else enq_rhs<float>(ctx, 0, sb, sb, sb, 0.0, 0.0);
+  if ((rc = enq_check(ctx))) return rc;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));
   const int nx = ctx->nx, ny = ctx->ny, nz = ctx->nz, nxg = ctx->nxg, nyg = ctx->nyg, nzg = ctx->nzg;
@@ -1384,6 +1396,7 @@ int blgpu_apply_bc(blgpu_ctx *ctx, int rk_step) {
   CK(cudaSetDevice(ctx->cfg.device));
   if (ctx->fp64) enq_bc<double>(ctx, ctx->cur, ctx->old, rk_step);
   else enq_bc<float>(ctx, ctx->cur, ctx->old, rk_step);
+  if (int rc = enq_check(ctx)) return rc;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));
   return BLGPU_OK;
@@ -1397,7 +1410,7 @@ int blgpu_projection(blgpu_ctx *ctx, int rk_step) {
   CK(cudaSetDevice(ctx->cfg.device));
   if (ctx->fp64) enq_projection<double>(ctx, ctx->cur, rk_step);
   else enq_projection<float>(ctx, ctx->cur, rk_step);
-  rc = cf_check(ctx);
+  rc = enq_check(ctx);
   if (rc) return rc;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));
@@ -2007,6 +2020,14 @@ static int ens_capture(blgpu_ensemble *e, int a) {
     e->gens[a][b] = ctx->gen;
   }
   cudaError_t ce = cudaStreamEndCapture(e->st, &gr);
+  int rc = BLGPU_OK;
+  for (blgpu_ctx *ctx : e->box)
+    if (int r = enq_check(ctx))
+      if (!rc) rc = ens_err(e, r, "%s", ctx->err.c_str());
+  if (rc) {
+    if (gr) cudaGraphDestroy(gr);
+    return rc;
+  }
   if (ce != cudaSuccess) return ens_err(e, BLGPU_ECUDA, "ensemble capture failed: %s", cudaGetErrorString(ce));
   ce = cudaGraphInstantiate(&e->graph[a], gr, 0);
   cudaGraphDestroy(gr);

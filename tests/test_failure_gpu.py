@@ -107,3 +107,25 @@ def test_rhs_plane_wait_limit_reports_and_recovers(gpu, precision, les, pts):
         assert np.array_equal(a, b)
     s.close()
     r.close()
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+def test_refused_launch_is_reported(gpu, precision):
+    """65537 y rows of modes are one grid dimension too many for the direct sums
+    of the z transform: the launch is refused, and the launches after it (whose
+    attribute calls clear the runtime's last error) do not hide that from the
+    projection, a step or a captured step.  The next context starts clean."""
+    c = cases.laminar_case(nx=5, ny=65538, nz=5, lx=2.0, ly=400.0, lz=2.0)
+    s = cases.solver_for(c, precision=precision)
+    s.set_dt(1e-6)
+    s.apply_boundary_conditions(1)
+    for call in (lambda: s.compute_projection_step(1), s.time_step, lambda: s.advance(1)):
+        with pytest.raises(BlgpuError, match="kernel launch"):
+            call()
+    s.apply_boundary_conditions(1)  # reported once
+    s.close()
+    d = _case()
+    r = cases.solver_for(d, precision=precision)
+    r.advance(1)
+    r.sync()
+    r.close()
