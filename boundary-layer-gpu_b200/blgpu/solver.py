@@ -271,8 +271,8 @@ class Solver:
 
     # -- wall model ----------------------------------------------------------
     def set_wait_limit(self, polls):
-        """Test hook: mbarrier polls of the tiled y-solve before a copy counts
-        as lost (< 0: the built-in limit)."""
+        """Test hook: mbarrier polls of the tiled y-solve and the TMA-fed
+        right-hand sides before a copy counts as lost (< 0: the built-in limit)."""
         self._ck(self.lib.blgpu_set_wait_limit(self.ctx, int(polls)))
 
     def set_wall_model(self, mode, jh=3, net=None):

@@ -221,9 +221,10 @@ int blgpu_law_of_wall(blgpu_ctx *ctx, double *utau, int *iters_max);
 int blgpu_advance_timed(blgpu_ctx *ctx, int nsteps, double *ms);
 
 /* Test hook of the failure path, no counterpart in the reference: the
- * number of mbarrier polls the tiled y-solve's CTAs make before a tile copy
- * counts as lost (polls < 0 restores the built-in limit of 2^24).  A wait
- * that gives up sets bit 4 of the device flag; the CTA still waits, with the
+ * number of mbarrier polls the CTAs of the tiled y-solve and of the TMA-fed
+ * right-hand sides make before a copy counts as lost (polls < 0 restores the
+ * built-in limit of 2^24).  A wait that gives up sets bit 4 (y-solve) or 64
+ * (right-hand side) of the device flag; the CTA still waits, with the
  * built-in limit, for its copy to land before it leaves, and the next
  * blgpu_sync / blgpu_advance_timed reports BLGPU_EDEVICE (once; the flag is
  * cleared when reported).  The state of such a step is not valid. */
